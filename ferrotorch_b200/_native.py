@@ -143,7 +143,7 @@ _KERNEL_PROTOS = {
     "ft_swiglu_fwd": (_i, [_vp, _vp, _ll, _i, _ll, _i, _i, _vp]),
     "ft_swiglu_bwd": (_i, [_vp, _vp, _vp, _ll, _i, _ll, _i, _i, _vp]),
     "ft_embedding_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp]),
-    "ft_embedding_bwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp]),
+    "ft_embedding_bwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "ft_adamw_flat": (_i, [_vp, _vp, _vp, _vp, _vp, _ll, _i, _vp, _f, _f, _f, _f, _f, _i, _i, _i, _vp]),
     "ft_sgd_flat": (_i, [_vp, _vp, _vp, _vp, _ll, _i, _vp, _f, _f, _f, _f, _i, _i, _i, _vp]),
     "ft_grad_norm_scratch": (_i, [_i]),

@@ -589,13 +589,14 @@ class _EmbeddingFn(torch.autograd.Function):
         dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
         mg = getattr(w, "main_grad", None)
         dw = None
-        if mg is None or mg.dtype != torch.bfloat16:
+        if mg is not None and (mg.dtype == torch.bfloat16 or (mg.dtype == torch.float32 and mg.is_contiguous() and H % 4 == 0
+                                                              and mg.data_ptr() % 16 == 0 and dy2.data_ptr() % 8 == 0)):
+            target = mg
+        else:
             dw = torch.zeros_like(w)
             target = dw
-        else:
-            target = mg
         rc = _native.kernels().ft_embedding_bwd(flat.data_ptr(), dy2.data_ptr(), target.data_ptr(),
-                                                flat.numel(), H, V, _dev(w), _stream())
+                                                flat.numel(), H, V, int(target.dtype == torch.float32), _dev(w), _stream())
         _native.check(rc, "ft_embedding_bwd")
         if dw is None:
             hook = getattr(w, "grad_ready_hook", None)

@@ -119,6 +119,20 @@ def test_gemm_small_m(M, N, K, ksplit):
     assert (F.stats["gemm_small_m"] > n0) == (N >= 1024 and K >= 512)
 
 
+def test_embedding_gradient_into_an_fp32_arena():
+    # repeated and out-of-order ids; sums of bf16 rows in fp32, against 64 bits
+    torch.manual_seed(5)
+    V, H, T = 97, 520, 700
+    w = _rand(V, H).requires_grad_()
+    w.main_grad = torch.randn(V, H, device=DEV)
+    ids, dy, before = torch.randint(0, V, (T,), device=DEV), _rand(T, H), w.main_grad.double().clone()
+    F.embedding(ids, w).backward(dy)
+    want = before.index_add(0, ids, dy.double())
+    assert w.grad is None
+    # at most 30 additions of magnitude 4 to a value: 30 roundings of 2^-24 relative to 30
+    assert float((w.main_grad.double() - want).abs().max()) < 30 * 30 * 2.0 ** -24
+
+
 def test_gemm_epilogues():
     torch.manual_seed(0)
     M, N, K = 520, 776, 392
