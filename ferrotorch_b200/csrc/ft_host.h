@@ -51,6 +51,19 @@ int sm_count(int device);
 // CUDA context bound, and driver entry points such as the tensor-map encoder require one.
 int ensure_device(int device);
 
+// Launch a kernel that may start while the one before it in the stream still runs (it calls grid_dependency_wait, ft_ptx.cuh, before it
+// touches memory).  Behind anything but such a kernel it is an ordinary launch.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 #define FT_CUDA_CHECK(expr)                                                        \
   do {                                                                             \
     cudaError_t _e = (expr);                                                       \

@@ -124,6 +124,10 @@ __device__ __forceinline__ void tma_gather4_2d(uint32_t dst, const CUtensorMap* 
       : "r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
       : "memory");
 }
+// Bring a box of a 2D tensor into L2.  A hint: nothing is read, so nothing goes stale if the tensor is being written.
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int x,
                                             int y, int z) {
   asm volatile(
@@ -159,6 +163,16 @@ template <int N>
 __device__ __forceinline__ void tma_store_wait() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
+
+// ----------------------------------------------------------------------------- overlapped launches
+// For kernels launched with launch_dependent (ft_host.h), which may start while the kernel before them in the stream still runs.
+// grid_dependency_launch lets the next such kernel start as soon as every CTA of this one has; grid_dependency_wait returns once the
+// kernel before this one has completed and its writes are visible.  Rules: every thread that reads or writes global memory waits first
+// (hints such as an L2 prefetch excepted), data of earlier kernels is not read through the non-coherent path (no __ldg, no const
+// __restrict__), and a kernel that lets the next one start always waits itself, so that the completion of a
+// kernel implies that of all before it.  Both do nothing in a plain launch.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ----------------------------------------------------------------------------- tcgen05
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_result, uint32_t ncols) {

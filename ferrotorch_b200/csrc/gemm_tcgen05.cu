@@ -27,7 +27,7 @@
 // Every wait is bounded; a wait that runs out aborts the CTA cleanly and reports
 // through the device status word.
 #include "ft_host.h"
-#include "ft_ptx.cuh"
+#include "gemm_flags.cuh"
 
 namespace ft {
 
@@ -35,20 +35,6 @@ constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;
 constexpr int GEMM_THREADS = 256;
 constexpr int GEMM_GROUP_M = 16;
-
-enum GemmFlags : int {
-  GEMM_OUT_F32 = 1,     // C is fp32 (default bf16)
-  GEMM_ACCUMULATE = 2,  // C += A B^T
-  GEMM_BIAS = 4,        // + bias[N] (bf16)
-  GEMM_BIAS_F32 = 8,    // bias is fp32
-  GEMM_RELU = 16,       // activation fused in the epilogue (after bias)
-  GEMM_GELU = 32,
-  GEMM_SILU = 64,
-  GEMM_RELU2 = 128,     // max(v, 0)^2
-  GEMM_ACT_MASK = GEMM_RELU | GEMM_GELU | GEMM_SILU | GEMM_RELU2,
-  GEMM_EPI_DIRECT = 1 << 16,  // internal: per-lane read-modify-write epilogue
-  GEMM_EPI_TRANSPOSED = 1 << 17,  // internal: the tile holds C^T; lane = column of C, register = row of C
-};
 
 template <int BN>
 struct GemmCfg {
@@ -81,9 +67,6 @@ struct GemmParams {
   // (n * cHo + i - c_oh) * cWo + j - c_ow of C when (i - c_oh, j - c_ow) lies inside the
   // cHo x cWo window, and dropped otherwise (cHo == 0: rows are stored as they are).
   int gHp, gWp, cHo, cWo, c_oh, c_ow;
-  // MODE 2 without accumulation: piece ks of the split contraction stores its tile at row
-  // ks * split_rows + m (one slice of the workspace per piece; summed later in a fixed order).
-  int split_rows;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, int m_blocks, int n_blocks, int& mb, int& nb) {
@@ -95,15 +78,6 @@ __device__ __forceinline__ void tile_coords(int tile, int m_blocks, int n_blocks
   mb = first_m + (r % gm);
   nb = r / gm;
 }
-
-__device__ __forceinline__ float apply_act(float v, int flags) {
-  if (flags & GEMM_RELU) return fmaxf(v, 0.f);
-  if (flags & GEMM_GELU) return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
-  if (flags & GEMM_SILU) return v / (1.f + __expf(-v));
-  if (flags & GEMM_RELU2) return fmaxf(v, 0.f) * fmaxf(v, 0.f);
-  return v;
-}
-
 
 // Bias and activation on 32 accumulator columns.  The kind of both is decided once, outside the unrolled loops: with
 // the choice inside, the epilogue's code no longer fits the instruction cache and outlasts the main loop.
@@ -291,42 +265,6 @@ __device__ __forceinline__ void epilogue_crop(const GemmParams& p, uint32_t t_ro
   }
 }
 
-
-// Epilogue for a tile that holds C^T (small-batch GEMMs are issued with the weight as the
-// 128-row MMA operand): accumulator row = column n of C, accumulator column = row m of C.  For
-// a fixed m the 32 lanes of a warp write 32 consecutive bf16 of row m: 64-byte segments.
-// p.M / p.N are the extents of the *tile space* (rows of W, batch), p.ldc the row stride of C.
-template <int BN>
-__device__ __forceinline__ void epilogue_transposed(const GemmParams& p, uint32_t t_row, int n_idx, int m0) {
-  const bool n_ok = n_idx < p.M;
-  const bool has_bias = (p.flags & (GEMM_BIAS | GEMM_BIAS_F32)) != 0;
-  const bool has_act = (p.flags & GEMM_ACT_MASK) != 0;
-  float bias = 0.f;
-  if (has_bias && n_ok)
-    bias = (p.flags & GEMM_BIAS_F32) ? static_cast<const float*>(p.bias)[n_idx]
-                                     : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n_idx]);
-#pragma unroll 1
-  for (int c = 0; c < BN / 32; ++c) {
-    uint32_t r[32];
-    tmem_ld_32x32(t_row + c * 32, r);
-    tmem_ld_wait();
-    if (!n_ok) continue;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + bias);
-    if (has_act) act32(r, p.flags);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int m = m0 + c * 32 + j;
-      if (m < p.N) {
-        const float v = __uint_as_float(r[j]);
-        if (p.flags & GEMM_OUT_F32)
-          static_cast<float*>(p.C)[static_cast<long long>(m) * p.ldc + n_idx] = v;
-        else
-          static_cast<__nv_bfloat16*>(p.C)[static_cast<long long>(m) * p.ldc + n_idx] = __float2bfloat16(v);
-      }
-    }
-  }
-}
 
 template <int BN, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -554,7 +492,7 @@ __device__ __forceinline__ void pair_tile_coords(int tile, int m_blocks, int n_b
 
 // Work item of a CTA pair: output block, contraction range and (MODE 2) the filter tap.
 struct PairTile {
-  int mb, nb, kb_begin, kb_end, tap, ks;
+  int mb, nb, kb_begin, kb_end, tap;
 };
 
 template <int BN, int MODE>
@@ -571,7 +509,6 @@ __device__ __forceinline__ PairTile pair_tile(const GemmParams& p, int tile, int
     const int mn = m_blocks * n_blocks;
     const int per_ks = mn * p.taps;
     const int ks = tile / per_ks;
-    t.ks = ks;
     const int r = tile - ks * per_ks;
     t.tap = r / mn;
     const int q = r - t.tap * mn;
@@ -585,7 +522,6 @@ __device__ __forceinline__ PairTile pair_tile(const GemmParams& p, int tile, int
     t.kb_begin = 0;
     t.kb_end = k_blocks;
     t.tap = 0;
-    t.ks = 0;
   }
   return t;
 }
@@ -761,18 +697,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const int m0 = t.mb * 2 * GEMM_BM + static_cast<int>(rank) * GEMM_BM + ew * 32;
       const int n0 = t.nb * BN;
       const int c_off = MODE == 2 ? t.tap * p.N : 0;  // dW[co, tap, ci]: tap t starts at column t * Cin
-      const int r_off = MODE == 2 ? t.ks * p.split_rows : 0;
       if (!mbar_wait(tfull_bar(acc), acc_phase, abort_word, FT_ERR_TIMEOUT_EPILOGUE)) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) +
                              static_cast<uint32_t>(acc * BN);
       if (MODE == 1 && p.cHo > 0) {
         epilogue_crop<BN>(p, t_row, m0 + lane, n0);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty_bar(acc), 0));
-      } else if (p.flags & GEMM_EPI_TRANSPOSED) {
-        epilogue_transposed<BN>(p, t_row, m0 + lane, n0);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty_bar(acc), 0));
@@ -839,9 +769,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           __syncwarp();
           if (lane == 0) {
             if (accumulate)
-              tma_reduce_add_2d(&tmC, tile_s, c_off + col0, r_off + m0);
+              tma_reduce_add_2d(&tmC, tile_s, c_off + col0, m0);
             else
-              tma_store_2d(&tmC, tile_s, c_off + col0, r_off + m0);
+              tma_store_2d(&tmC, tile_s, c_off + col0, m0);
             tma_store_commit();
           }
           buf ^= 1;
@@ -965,10 +895,13 @@ FT_API int ft_gemm_bf16(const void* A, const void* B, void* C, const void* bias,
   p.C = C; p.bias = bias; p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.flags = flags;
   p.status = device_status_word(device);
   p.taps = 0; p.cblocks = 0; p.ksplit = 1;
-  p.gHp = p.gWp = p.cHo = p.cWo = p.c_oh = p.c_ow = 0; p.split_rows = 0;
+  p.gHp = p.gWp = p.cHo = p.cWo = p.c_oh = p.c_ow = 0;
 
-  // Problems with at least one full 256-row block and N >= 128 run on the CTA-pair kernel.
-  if (!force_single && M >= 2 * GEMM_BM && N >= 128 && (bn == 0 || bn >= 128)) {
+  // Problems with at least one full 256-row block and N >= 128 run on the CTA-pair kernel, and those with more than half of one that
+  // need more than a wave of the one-CTA kernel's smallest tiles (214 x 3072 x 8192: 43 against 76 us, 214 x 4096 x 4096: 25 against 40;
+  // within a wave the small tiles win, 214 x 2048 x 2048: 13 against 15).
+  const bool tall = M >= 2 * GEMM_BM || (M > GEMM_BM && 2ll * ((N + 31) / 32) > sm_count(device));
+  if (!force_single && tall && N >= 128 && (bn == 0 || bn >= 128)) {
     const int pairs = (max_ctas > 0 && max_ctas < sm_count(device) ? max_ctas : sm_count(device)) / 2;
     const long long mb2 = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
     int pbn = bn ? bn : 256;
@@ -1058,7 +991,7 @@ FT_API int ft_conv_shift_gemm(const void* xp, const void* w, void* y, const void
   p.status = device_status_word(device);
   p.taps = taps; p.cblocks = Cin / GEMM_BK; p.ksplit = 1;
   for (int t = 0; t < GEMM_MAX_TAPS; ++t) p.shift[t] = t < taps ? shift[t] : 0;
-  p.gHp = p.gWp = p.cHo = p.cWo = p.c_oh = p.c_ow = 0; p.split_rows = 0;
+  p.gHp = p.gWp = p.cHo = p.cWo = p.c_oh = p.c_ow = 0;
   long long y_rows = P;
   if (crop) {
     p.gHp = crop[0]; p.gWp = crop[1]; p.cHo = crop[2]; p.cWo = crop[3]; p.c_oh = crop[4]; p.c_ow = crop[5];
@@ -1107,7 +1040,7 @@ FT_API int ft_conv_shift_wgrad(const void* dyp, const void* xp, float* dw, long 
   p.ldc = static_cast<long long>(taps) * Cin;
   p.flags = GEMM_OUT_F32 | GEMM_ACCUMULATE;
   p.status = device_status_word(device);
-  p.gHp = p.gWp = p.cHo = p.cWo = p.c_oh = p.c_ow = 0; p.split_rows = 0;
+  p.gHp = p.gWp = p.cHo = p.cWo = p.c_oh = p.c_ow = 0;
   p.taps = taps; p.cblocks = Cin / GEMM_BK;
   for (int t = 0; t < GEMM_MAX_TAPS; ++t) p.shift[t] = t < taps ? shift[t] : 0;
   const int bn = Cin >= 256 ? 256 : 128;
@@ -1135,227 +1068,4 @@ FT_API int ft_conv_shift_wgrad(const void* dyp, const void* xp, float* dw, long 
   if (rc) return rc;
   if (bn == 256) return launch_pair<256, true, true, 2>(tmA, tmB, tmC, p, device, max_ctas, stream);
   return launch_pair<128, true, true, 2>(tmA, tmB, tmC, p, device, max_ctas, stream);
-}
-
-namespace ft {
-
-// ws holds the pieces of the split contraction: C^T as fp32 [ksplit][slice_rows >= N, ld_ws].  Write
-// C[m, n] = act(sum_ks ws[ks][n, m] (+ bias[n]) (+ residual[m, n])) as bf16; the pieces are summed in
-// index order, so the result does not depend on which CTA finished first.
-__global__ void small_m_finalize_kernel(const float* __restrict__ ws, __nv_bfloat16* __restrict__ C,
-                                        const __nv_bfloat16* __restrict__ residual, const void* __restrict__ bias,
-                                        int flags, int M, int N, int ld_ws, int ksplit, int slice_rows,
-                                        long long ldc, long long ldr) {
-  // block = 32 x 8 threads over a 32 (n) x 32 (m) patch, transposed through shared memory
-  __shared__ float tile[32][33];
-  const int n0 = blockIdx.x * 32, m0 = blockIdx.y * 32;
-  const long long slice = static_cast<long long>(slice_rows) * ld_ws;
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int n = n0 + i, m = m0 + threadIdx.x;
-    float v = 0.f;
-    if (n < N && m < ld_ws) {
-      const float* src = ws + static_cast<long long>(n) * ld_ws + m;
-      for (int ks = 0; ks < ksplit; ++ks) v += src[ks * slice];
-    }
-    tile[i][threadIdx.x] = v;
-  }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int m = m0 + i, n = n0 + threadIdx.x;
-    if (m < M && n < N) {
-      float v = tile[threadIdx.x][i];
-      if (bias) v += (flags & GEMM_BIAS_F32) ? static_cast<const float*>(bias)[n] : __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[n]);
-      if (residual) v += __bfloat162float(residual[static_cast<long long>(m) * ldr + n]);
-      C[static_cast<long long>(m) * ldc + n] = __float2bfloat16(apply_act(v, flags));
-    }
-  }
-}
-
-// The same sum for an fp32 result: C[m, n] (+)= sum_ks ws[ks][n, m], with the next layer's dynamic tanh
-// applied to the new value on its way out: dyt_out = (tanh(alpha C) w + b) as bf16.  Being element by
-// element, that norm needs no pass of its own over the residual stream.
-__global__ void small_m_finalize_f32_kernel(const float* __restrict__ ws, float* __restrict__ C, int accumulate,
-                                            const float* __restrict__ alpha_p, const float* __restrict__ w,
-                                            const float* __restrict__ b, __nv_bfloat16* __restrict__ dyt_out, float dyt_scale,
-                                            int M, int N, int ld_ws, int ksplit, int slice_rows, long long ldc, long long ldd) {
-  __shared__ float tile[32][33];
-  const int n0 = blockIdx.x * 32, m0 = blockIdx.y * 32;
-  const long long slice = static_cast<long long>(slice_rows) * ld_ws;
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int n = n0 + i, m = m0 + threadIdx.x;
-    float v = 0.f;
-    if (n < N && m < M) {
-      const float* src = ws + static_cast<long long>(n) * ld_ws + m;
-      for (int ks = 0; ks < ksplit; ++ks) v += src[ks * slice];
-    }
-    tile[i][threadIdx.x] = v;
-  }
-  __syncthreads();
-  const float alpha = dyt_out ? *alpha_p : 0.f;
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int m = m0 + i, n = n0 + threadIdx.x;
-    if (m < M && n < N) {
-      float v = tile[threadIdx.x][i];
-      float* c = C + static_cast<long long>(m) * ldc + n;
-      if (accumulate) v += *c;
-      *c = v;
-      if (dyt_out) dyt_out[static_cast<long long>(m) * ldd + n] = __float2bfloat16((tanhf(alpha * v) * w[n] + b[n]) * dyt_scale);
-    }
-  }
-}
-
-}  // namespace ft
-
-constexpr int SMALL_M_MAX_SPLIT = 16;
-
-// Floats of workspace ft_gemm_small_m may need for an [M, N] result (its contents do not matter).
-FT_API long long ft_gemm_small_m_workspace(int M, int N) {
-  const int mpad = M <= 64 ? 64 : 128;
-  return static_cast<long long>((N + 255) / 256 * 256) * mpad * SMALL_M_MAX_SPLIT;
-}
-
-namespace ft {
-
-// How many pieces the contraction of a small-batch GEMM is cut into (>= min_split).
-static int small_m_pick_split(int N, int K, int ksplit, int min_split, int device) {
-  const int pairs = sm_count(device) / 2;
-  const int tiles = (N + 255) / 256;
-  const int k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
-  if (ksplit <= 0) {
-    ksplit = 1;
-    if (tiles < pairs) {
-      // one wave: as many pieces per tile as there are CTA pairs to take them, each piece long
-      // enough (>= 4 k-blocks) to be worth a pipeline fill
-      ksplit = pairs / tiles;
-      const int max_split = k_blocks / 4 > 0 ? k_blocks / 4 : 1;
-      if (ksplit > max_split) ksplit = max_split;
-      if (ksplit < 1) ksplit = 1;
-    }
-  }
-  if (ksplit < min_split) ksplit = min_split;
-  if (ksplit > k_blocks) ksplit = k_blocks;
-  return ksplit > SMALL_M_MAX_SPLIT ? SMALL_M_MAX_SPLIT : ksplit;
-}
-
-// The whole contraction in one pass, C written transposed by the epilogue (bf16, or fp32 with GEMM_OUT_F32).
-static int small_m_single(const void* X, const void* W, void* C, const void* bias, int M, int N, int K, long long ldx,
-                          long long ldw, long long ldc, int flags, int device, cudaStream_t stream) {
-  const int bn = M <= 64 ? 64 : 128;
-  GemmParams p;
-  p.bias = bias; p.M = N; p.N = M; p.K = K;   // tile space: rows of W x batch
-  p.status = device_status_word(device);
-  p.taps = 0; p.cblocks = 0; p.ksplit = 1;
-  for (int t = 0; t < GEMM_MAX_TAPS; ++t) p.shift[t] = 0;
-  p.gHp = p.gWp = p.cHo = p.cWo = p.c_oh = p.c_ow = 0; p.split_rows = 0;
-  p.C = C; p.ldc = ldc;
-  p.flags = flags | GEMM_EPI_TRANSPOSED;
-  CUtensorMap tmA, tmB, tmC;
-  int rc = make_tmap_2d(&tmA, W, 2, K, N, ldw * 2, GEMM_BK, GEMM_BM, 3);
-  if (rc) return rc;
-  rc = make_tmap_2d(&tmB, X, 2, K, M, ldx * 2, GEMM_BK, bn / 2, 3);
-  if (rc) return rc;
-  // the store map is not used by the transposed epilogue; point it at W so that it is valid
-  rc = make_tmap_2d(&tmC, W, 2, K, N, ldw * 2, 64, 32, 3);
-  if (rc) return rc;
-  return bn == 64 ? launch_pair<64, false, false, 0>(tmA, tmB, tmC, p, device, 0, stream)
-                  : launch_pair<128, false, false, 0>(tmA, tmB, tmC, p, device, 0, stream);
-}
-
-// Launch the split contraction of a small-batch GEMM into `workspace` (slices of ceil(N / 256) * 256 rows
-// x 64 or 128 columns); *ksplit returns the number of slices.
-static int small_m_split(const void* X, const void* W, float* workspace, int M, int N, int K, long long ldx, long long ldw,
-                         int* ksplit, int min_split, int device, cudaStream_t stream) {
-  const int bn = M <= 64 ? 64 : 128;
-  const int k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
-  const int pieces = small_m_pick_split(N, K, *ksplit, min_split, device);
-  GemmParams p;
-  p.bias = nullptr; p.M = N; p.N = M; p.K = K;   // tile space: rows of W x batch
-  p.status = device_status_word(device);
-  p.taps = 1; p.cblocks = 0;
-  for (int t = 0; t < GEMM_MAX_TAPS; ++t) p.shift[t] = 0;
-  p.gHp = p.gWp = p.cHo = p.cWo = p.c_oh = p.c_ow = 0;
-  const int per = (k_blocks + pieces - 1) / pieces;
-  p.ksplit = *ksplit = (k_blocks + per - 1) / per;
-  p.C = workspace; p.ldc = bn;
-  p.flags = GEMM_OUT_F32;
-  // a slice is a whole number of 256-row tiles, so a tile that hangs over the end of W stays
-  // inside its own slice
-  p.split_rows = (N + 255) / 256 * 256;
-  CUtensorMap tmA, tmB, tmC;
-  int rc = make_tmap_2d(&tmA, W, 2, K, N, ldw * 2, GEMM_BK, GEMM_BM, 3);
-  if (rc) return rc;
-  rc = make_tmap_2d(&tmB, X, 2, K, M, ldx * 2, GEMM_BK, bn / 2, 3);
-  if (rc) return rc;
-  rc = make_tmap_2d(&tmC, workspace, 4, bn, static_cast<uint64_t>(p.ksplit) * p.split_rows,
-                    static_cast<uint64_t>(bn) * 4, 32, 32, 3);
-  if (rc) return rc;
-  return bn == 64 ? launch_pair<64, false, false, 2>(tmA, tmB, tmC, p, device, 0, stream)
-                  : launch_pair<128, false, false, 2>(tmA, tmB, tmC, p, device, 0, stream);
-}
-
-}  // namespace ft
-
-// C[M, N] = X[M, K] W[N, K]^T (+ bias[N]) (+ residual[M, N]) for a small batch M <= 128 (decode):
-// the weight is the 128-row MMA operand, so every byte of W crosses the tensor core once with all
-// 128 rows in use and the batch is only the (64- or 128-wide) N dimension of the instruction.
-// When N / 256 tiles would leave most SMs idle, the contraction is split across CTA pairs; each
-// piece stores its fp32 partial tile into its own slice of `workspace` and a second small kernel
-// sums the slices in index order (deterministic) and writes C.  workspace:
-// ft_gemm_small_m_workspace(M, N) floats, contents irrelevant (may be null when no split is
-// needed; then residual must be null).
-// All of X, W, C bf16; K-major operands; ldx, ldw, ldc, ldr in elements.
-FT_API int ft_gemm_small_m(const void* X, const void* W, void* C, const void* bias, const void* residual,
-                           float* workspace, int M, int N, int K, long long ldx, long long ldw, long long ldc,
-                           long long ldr, int flags, int ksplit, int device, cudaStream_t stream) {
-  if (int _rc = ft::ensure_device(device)) return _rc;
-  using namespace ft;
-  FT_REQUIRE(X && W && C, "ft_gemm_small_m: null operand");
-  FT_REQUIRE(M > 0 && M <= 128 && N > 0 && K > 0, "ft_gemm_small_m: M=%d must be in 1..128 (N=%d K=%d)", M, N, K);
-  FT_REQUIRE(ldx % 8 == 0 && ldw % 8 == 0 && N % 8 == 0, "ft_gemm_small_m: strides and N must be multiples of 8");
-  FT_REQUIRE(!(flags & (GEMM_OUT_F32 | GEMM_ACCUMULATE)), "ft_gemm_small_m: bf16 output, no accumulation");
-  FT_REQUIRE(!(flags & (GEMM_BIAS | GEMM_BIAS_F32)) || bias, "ft_gemm_small_m: bias flag without bias");
-  const int bn = M <= 64 ? 64 : 128;
-  const int k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
-  if (ksplit <= 0) ksplit = workspace ? small_m_pick_split(N, K, 0, 1, device) : 1;
-  // the residual is added by the finalize pass, which only the split path has
-  if (residual && ksplit == 1 && workspace && k_blocks >= 2) ksplit = 2;
-  FT_REQUIRE(ksplit == 1 || workspace, "ft_gemm_small_m: a split contraction needs the workspace");
-  FT_REQUIRE(ksplit > 1 || !residual, "ft_gemm_small_m: the residual is added by the split path only");
-  if (ksplit == 1) return small_m_single(X, W, C, bias, M, N, K, ldx, ldw, ldc, flags & 0xFFFF, device, stream);
-  int rc = small_m_split(X, W, workspace, M, N, K, ldx, ldw, &ksplit, 2, device, stream);
-  if (rc) return rc;
-  dim3 grid((N + 31) / 32, (M + 31) / 32), block(32, 8);
-  small_m_finalize_kernel<<<grid, block, 0, stream>>>(workspace, static_cast<__nv_bfloat16*>(C),
-                                                      static_cast<const __nv_bfloat16*>(residual), bias,
-                                                      flags, M, N, bn, ksplit,
-                                                      (N + 255) / 256 * 256, ldc, ldr);
-  FT_CUDA_CHECK(cudaGetLastError());
-  count_launch();
-  return FT_E_OK;
-}
-
-// C[M, N] (fp32) (+)= X[M, K] W[N, K]^T for a small batch M <= 128: in one pass when W alone fills the GPU and
-// nothing is added, else through the split contraction and its finalize pass (see ft_gemm_small_m), which also writes dyt_out[M, N] = (tanh(alpha C) w + b) * dyt_scale
-// as bf16 when dyt_out is given.  workspace: ft_gemm_small_m_workspace(M, N) floats.
-FT_API int ft_gemm_small_m_f32(const void* X, const void* W, float* C, int accumulate, const float* alpha, const float* dyt_w,
-                               const float* dyt_b, void* dyt_out, float dyt_scale, float* workspace, int M, int N, int K,
-                               long long ldx, long long ldw, long long ldc, long long ldd, int ksplit, int device,
-                               cudaStream_t stream) {
-  if (int _rc = ft::ensure_device(device)) return _rc;
-  using namespace ft;
-  FT_REQUIRE(X && W && C && workspace, "ft_gemm_small_m_f32: null operand");
-  FT_REQUIRE(M > 0 && M <= 128 && N > 0 && K > GEMM_BK, "ft_gemm_small_m_f32: M=%d must be in 1..128, K=%d above %d (N=%d)", M, K, GEMM_BK, N);
-  FT_REQUIRE(ldx % 8 == 0 && ldw % 8 == 0, "ft_gemm_small_m_f32: strides must be multiples of 8");
-  FT_REQUIRE(!dyt_out || (alpha && dyt_w && dyt_b), "ft_gemm_small_m_f32: the fused norm needs its parameters");
-  if (!accumulate && !dyt_out && small_m_pick_split(N, K, ksplit, 1, device) == 1)
-    return small_m_single(X, W, C, nullptr, M, N, K, ldx, ldw, ldc, GEMM_OUT_F32, device, stream);
-  int rc = small_m_split(X, W, workspace, M, N, K, ldx, ldw, &ksplit, 2, device, stream);
-  if (rc) return rc;
-  dim3 grid((N + 31) / 32, (M + 31) / 32), block(32, 8);
-  small_m_finalize_f32_kernel<<<grid, block, 0, stream>>>(workspace, C, accumulate, alpha, dyt_w, dyt_b,
-                                                          static_cast<__nv_bfloat16*>(dyt_out), dyt_scale, M, N, M <= 64 ? 64 : 128,
-                                                          ksplit, (N + 255) / 256 * 256, ldc, ldd);
-  FT_CUDA_CHECK(cudaGetLastError());
-  count_launch();
-  return FT_E_OK;
 }

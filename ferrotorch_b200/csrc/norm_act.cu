@@ -54,10 +54,12 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // y = (x [+ delta]) * rstd * w ; if delta != null also writes res_out = x + delta.
 // One block per row, grid-stride over rows. H % 8 == 0.
 __global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
+rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* delta,
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                    __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int rows, int H,
                    float eps) {
+  grid_dependency_launch();
+  grid_dependency_wait();
   __shared__ float red[32];
   const int nvec = H >> 3;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -253,9 +255,11 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 // 32 contiguous bytes.  cos/sin come as two float4 each.  Needs D % 16 == 0 and 16-byte
 // aligned rows (checked by the launcher).
 __global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cos_t,
-                                const float* __restrict__ sin_t, const int* __restrict__ pos, int T,
+                                const float* __restrict__ sin_t, const int* pos, int T,
                                 int n_rot_heads, int D, long long ld, int seq_len, int pos_offset,
                                 int interleaved, float sign) {
+  grid_dependency_launch();
+  grid_dependency_wait();
   const int half = D >> 1;
   const int groups_per_head = half >> 3;                       // 8 pairs per group
   const int groups_per_tok = n_rot_heads * groups_per_head;
@@ -323,8 +327,10 @@ __device__ __forceinline__ float act_bwd(float g, int act) {
 }
 // Two vectors per thread with all loads issued first and streaming (evict-first) hints on the
 // inputs, which are read exactly once.
-__global__ void swiglu_fwd2_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
+__global__ void swiglu_fwd2_kernel(const __nv_bfloat16* gu, __nv_bfloat16* __restrict__ out,
                                    long long T, int F, long long ld_gu, int act) {
+  grid_dependency_launch();
+  grid_dependency_wait();
   const int fv = F >> 3;
   const long long total = T * fv;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -599,11 +605,9 @@ FT_API int ft_rmsnorm_fwd(const void* x, const void* delta, const void* w, void*
   FT_REQUIRE(H % 8 == 0 && H <= NORM_THREADS * NORM_MAX_VEC * 8, "ft_rmsnorm_fwd: H=%d unsupported", H);
   if (rows <= 0) return FT_E_OK;
   const int grid = rows < sm_count(device) * 8 ? rows : sm_count(device) * 8;
-  rmsnorm_fwd_kernel<<<grid, NORM_THREADS, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(delta),
-      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
-      static_cast<__nv_bfloat16*>(res_out), rstd, rows, H, eps);
-  FT_CUDA_CHECK(cudaGetLastError());
+  FT_CUDA_CHECK(launch_dependent(rmsnorm_fwd_kernel, grid, NORM_THREADS, 0, stream, static_cast<const __nv_bfloat16*>(x),
+                                 static_cast<const __nv_bfloat16*>(delta), static_cast<const __nv_bfloat16*>(w),
+                                 static_cast<__nv_bfloat16*>(y), static_cast<__nv_bfloat16*>(res_out), rstd, rows, H, eps));
   count_launch();
   return FT_E_OK;
 }
@@ -650,9 +654,8 @@ FT_API int ft_rope(void* x, const float* cos_t, const float* sin_t, const int* p
   const long long work = static_cast<long long>(T) * n_rot_heads * (D / 4);
   if (D % 16 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
       (reinterpret_cast<uintptr_t>(cos_t) & 15) == 0 && (reinterpret_cast<uintptr_t>(sin_t) & 15) == 0)
-    rope_vec_kernel<<<blocks_for(work / 4, 256, device), 256, 0, stream>>>(
-        static_cast<__nv_bfloat16*>(x), cos_t, sin_t, pos, T, n_rot_heads, D, ld, seq_len, pos_offset,
-        interleaved, backward ? -1.f : 1.f);
+    FT_CUDA_CHECK(launch_dependent(rope_vec_kernel, blocks_for(work / 4, 256, device), 256, 0, stream, static_cast<__nv_bfloat16*>(x),
+                                   cos_t, sin_t, pos, T, n_rot_heads, D, ld, seq_len, pos_offset, interleaved, backward ? -1.f : 1.f));
   else
     rope_kernel<<<blocks_for(work, 256, device), 256, 0, stream>>>(
         static_cast<__nv_bfloat16*>(x), cos_t, sin_t, pos, T, n_rot_heads, D, ld, seq_len, pos_offset,
@@ -668,9 +671,8 @@ FT_API int ft_swiglu_fwd(const void* gu, void* out, long long T, int F, long lon
   FT_REQUIRE(gu && out, "ft_swiglu_fwd: null pointer");
   FT_REQUIRE(F % 8 == 0 && ld_gu % 8 == 0, "ft_swiglu_fwd: F must be a multiple of 8");
   if (T <= 0) return FT_E_OK;
-  swiglu_fwd2_kernel<<<blocks_for(T * (F / 8) / 2 + 1, 256, device), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), T, F, ld_gu, act);
-  FT_CUDA_CHECK(cudaGetLastError());
+  FT_CUDA_CHECK(launch_dependent(swiglu_fwd2_kernel, blocks_for(T * (F / 8) / 2 + 1, 256, device), 256, 0, stream,
+                                 static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), T, F, ld_gu, act));
   count_launch();
   return FT_E_OK;
 }

@@ -36,11 +36,12 @@ constexpr int PD_WARPS = PD_THREADS / 32;
 
 // k_new / v_new: rows of kv16 / vv16 16-byte units (all KV heads of a token) with token strides ldk16 / ldv16 units.
 // Token i goes to sequence seq_ids[i] (or i / tokens_per_seq when null) at position pos[i].
-__global__ void kv_append_kernel(const uint4* __restrict__ k_new, const uint4* __restrict__ v_new, uint4* __restrict__ k_cache,
-                                 uint4* __restrict__ v_cache, const int* __restrict__ block_table,
-                                 const int* __restrict__ pos, const int* __restrict__ seq_ids, int T, int tokens_per_seq,
+__global__ void kv_append_kernel(const uint4* k_new, const uint4* v_new, uint4* k_cache, uint4* v_cache, const int* block_table,
+                                 const int* pos, const int* seq_ids, int T, int tokens_per_seq,
                                  int kv16, int vv16, long long ldk16, long long ldv16, int block_size, int max_blocks,
                                  int num_blocks) {
+  grid_dependency_launch();
+  grid_dependency_wait();
   for (int t = blockIdx.x; t < T; t += gridDim.x) {
     const int b = seq_ids ? seq_ids[t] : t / tokens_per_seq;
     const int p = pos[t];
@@ -276,9 +277,10 @@ paged_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   }
 }
 
-__global__ void paged_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                            __nv_bfloat16* __restrict__ out, int Hq, int D, long long ldo, int n_splits,
+__global__ void paged_decode_combine_kernel(const float* part_o, const float* part_ml, __nv_bfloat16* __restrict__ out, int Hq, int D, long long ldo, int n_splits,
                                             const float* __restrict__ sink, HeadGate gate, float out_scale) {
+  grid_dependency_launch();
+  grid_dependency_wait();
   const int hq = blockIdx.x, b = blockIdx.y;
   const long long base = (static_cast<long long>(b) * Hq + hq) * n_splits;
   float mm = -INFINITY;
@@ -347,8 +349,8 @@ struct PtCfg {  // HD: width of the K tile (64 or 128)
 template <int HD, int G>
 __global__ void __launch_bounds__(PT_THREADS, 1)
 paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
-                       const __nv_bfloat16* __restrict__ q, const int* __restrict__ block_table,
-                       const int* __restrict__ row_slot, const int* __restrict__ ctx_len, __nv_bfloat16* __restrict__ out,
+                       const __nv_bfloat16* q, const int* block_table,
+                       const int* row_slot, const int* ctx_len, __nv_bfloat16* __restrict__ out,
                        float* __restrict__ part_o, float* __restrict__ part_ml, int Hq, int Hkv, int D, int Dv, int g_real,
                        long long ldq, long long ldo, int block_size, int max_blocks, int num_blocks, float scale_log2,
                        int n_splits, KeyRange range, PooledKeys pooled, const float* __restrict__ slopes, const float* __restrict__ sink,
@@ -369,16 +371,7 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
 
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int len = ctx_len[b];
-  const int first = range.first_visible(len);
-  // tiles of pooled blocks, then tiles of keys from the first visible one's on; tile_lo counts in this order
-  const int n_pool = pooled.count(first), pool_tiles = (n_pool + PT_TILE - 1) / PT_TILE;
-  const int key_tile = first / PT_TILE - pool_tiles;             // tile t holds keys from (key_tile + t) * PT_TILE on
-  const int tiles_all = pool_tiles + max(0, (len + PT_TILE - 1) / PT_TILE - first / PT_TILE);
-  const int tiles_per_split = (tiles_all + n_splits - 1) / n_splits;
-  const int tile_lo = split * tiles_per_split;
-  const int n_tiles = max(0, min(tiles_all, tile_lo + tiles_per_split) - tile_lo);
-
+  grid_dependency_launch();
   if (threadIdx.x == 0) {
     *abort_word = 0;
     for (int s = 0; s < PT_STAGES; ++s) {
@@ -404,6 +397,16 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
   if (D < HD || Dv < PT_VD)
     for (int i = threadIdx.x; i < PT_STAGES * Cfg::STAGE_BYTES / 16; i += blockDim.x)
       reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+  grid_dependency_wait();
+  const int len = ctx_len[b];
+  const int first = range.first_visible(len);
+  // tiles of pooled blocks, then tiles of keys from the first visible one's on; tile_lo counts in this order
+  const int n_pool = pooled.count(first), pool_tiles = (n_pool + PT_TILE - 1) / PT_TILE;
+  const int key_tile = first / PT_TILE - pool_tiles;             // tile t holds keys from (key_tile + t) * PT_TILE on
+  const int tiles_all = pool_tiles + max(0, (len + PT_TILE - 1) / PT_TILE - first / PT_TILE);
+  const int tiles_per_split = (tiles_all + n_splits - 1) / n_splits;
+  const int tile_lo = split * tiles_per_split;
+  const int n_tiles = max(0, min(tiles_all, tile_lo + tiles_per_split) - tile_lo);
   __syncthreads();
   for (int i = threadIdx.x; i < g_real * (D / 8); i += blockDim.x) {
     const int g = i / (D / 8), j = i - g * (D / 8);  // 16-byte chunk j of head g
@@ -472,7 +475,7 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
               const int row = row0 + 8 * i;
               const int key = key0 + row;
               const int page = key / block_size;
-              int blk = (key < len && page < max_blocks) ? __ldg(bt + page) : 0;
+              int blk = (key < len && page < max_blocks) ? bt[page] : 0;
               blk = min(max(blk, 0), num_blocks - 1);
               copy(row, k_cache, v_cache, (static_cast<long long>(blk) * block_size + key % block_size) * Hkv + kvh, key < len);
             }
@@ -811,11 +814,10 @@ FT_API int ft_kv_append(const void* k_new, const void* v_new, void* k_cache, voi
                reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0, "ft_kv_append: pointers must be 16-byte aligned");
   if (T <= 0) return FT_E_OK;
   const int grid = T < sm_count(device) * 8 ? T : sm_count(device) * 8;
-  kv_append_kernel<<<grid, 128, 0, stream>>>(static_cast<const uint4*>(k_new), static_cast<const uint4*>(v_new),
-                                             static_cast<uint4*>(k_cache), static_cast<uint4*>(v_cache), block_table, pos,
-                                             seq_ids, T, tokens_per_seq, Hkv * D / unit, Hkv * Dv / unit, ldk / unit, ldv / unit,
-                                             block_size, max_blocks, num_blocks);
-  FT_CUDA_CHECK(cudaGetLastError());
+  FT_CUDA_CHECK(launch_dependent(kv_append_kernel, grid, 128, 0, stream, static_cast<const uint4*>(k_new),
+                                 static_cast<const uint4*>(v_new), static_cast<uint4*>(k_cache), static_cast<uint4*>(v_cache), block_table,
+                                 pos, seq_ids, T, tokens_per_seq, Hkv * D / unit, Hkv * Dv / unit, ldk / unit, ldv / unit, block_size,
+                                 max_blocks, num_blocks));
   count_launch();
   return FT_E_OK;
 }
@@ -900,10 +902,10 @@ FT_API int ft_paged_decode(const void* q, const void* k_cache, const void* v_cac
       FT_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PtCfg<HH>::SMEM_BYTES)); \
       attr_set[device] = true;                                                                                  \
     }                                                                                                           \
-    kern<<<grid, PT_THREADS, PtCfg<HH>::SMEM_BYTES, stream>>>(                                                  \
+    FT_CUDA_CHECK(launch_dependent(kern, grid, PT_THREADS, PtCfg<HH>::SMEM_BYTES, stream,                       \
         static_cast<const __nv_bfloat16*>(k_cache), static_cast<const __nv_bfloat16*>(v_cache),                \
         static_cast<const __nv_bfloat16*>(q), block_table, row_slot, ctx_len, static_cast<__nv_bfloat16*>(out), \
-        part_o, part_ml, Hq, Hkv, D, Dv, G, ldq, ldo, block_size, max_blocks, num_blocks, sl2, n_splits, range, pooled, slopes, sink, hg, out_scale, status); \
+        part_o, part_ml, Hq, Hkv, D, Dv, G, ldq, ldo, block_size, max_blocks, num_blocks, sl2, n_splits, range, pooled, slopes, sink, hg, out_scale, status)); \
   }
 #define FT_PT_BY_G(HH)                     \
   if (G == 1) FT_PT_LAUNCH(HH, 1)          \
@@ -940,8 +942,8 @@ FT_API int ft_paged_decode(const void* q, const void* k_cache, const void* v_cac
   count_launch();
   if (n_splits > 1) {
     dim3 g2(Hq, B);
-    paged_decode_combine_kernel<<<g2, Dv <= 64 ? 64 : 128, 0, stream>>>(part_o, part_ml, static_cast<__nv_bfloat16*>(out), Hq, Dv, ldo, n_splits, sink, hg, out_scale);
-    FT_CUDA_CHECK(cudaGetLastError());
+    FT_CUDA_CHECK(launch_dependent(paged_decode_combine_kernel, g2, Dv <= 64 ? 64 : 128, 0, stream, part_o, part_ml,
+                                   static_cast<__nv_bfloat16*>(out), Hq, Dv, ldo, n_splits, sink, hg, out_scale));
     count_launch();
   }
   return FT_E_OK;

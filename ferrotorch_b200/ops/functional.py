@@ -26,28 +26,15 @@ stats = {"gemm_native": 0, "gemm_library": 0, "gemm_small_m": 0}
 
 _native.register_protos({
     "ft_gemm_small_m": (_native._i, [_native._vp] * 6 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 3 + [_native._vp]),
-    "ft_gemm_small_m_workspace": (_native._ll, [_native._i, _native._i]),
 })
-_small_m_ws: dict = {}
-
-
-def _small_m_workspace(n_floats: int, device) -> torch.Tensor:
-    """fp32 workspace of the split-K small-batch GEMM for the current stream (one slice per piece
-    of the contraction; contents do not matter between calls)."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
-    buf = _small_m_ws.get(key)
-    if buf is None or buf.numel() < n_floats:
-        buf = torch.empty(n_floats, device=device, dtype=torch.float32)
-        _small_m_ws[key] = buf
-    return buf
 
 
 def gemm_small_m(x: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None = None,
                  residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
                  activation: str | None = None, ksplit: int = 0) -> torch.Tensor:
     """``x @ w.T (+ bias) (+ residual)`` for a small batch ``x [M <= 128, K]`` against ``w [N, K]``
-    (both bf16, row-major): the decode-time GEMM.  The weight is the 128-row operand of the MMA and
-    the contraction is split over the GPU when ``N / 256`` tiles would leave SMs idle."""
+    (both bf16, row-major): the decode-time GEMM.  The weight is the 128-row operand of the MMA, the contraction of a tile is
+    shared by a cluster of CTAs (``ksplit`` is a hint that is not needed any more)."""
     M, K = x.shape
     N = w.shape[0]
     if out is None:
@@ -61,17 +48,14 @@ def gemm_small_m(x: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None 
     lib = _native.kernels()
     if residual is not None and ksplit == 1:
         raise ValueError("gemm_small_m: a residual needs the split path (ksplit != 1)")
-    ws = None
-    if ksplit != 1:
-        ws = _small_m_workspace(int(lib.ft_gemm_small_m_workspace(M, N)), x.device)
     rc = lib.ft_gemm_small_m(x.data_ptr(), w.data_ptr(), out.data_ptr(), bias_ptr,
-                             residual.data_ptr() if residual is not None else None,
-                             ws.data_ptr() if ws is not None else None, M, N, K, x.stride(0), w.stride(0),
+                             residual.data_ptr() if residual is not None else None, None, M, N, K, x.stride(0), w.stride(0),
                              out.stride(0), residual.stride(0) if residual is not None else 0, flags, ksplit,
                              _dev(x), _stream())
     _native.check(rc, "ft_gemm_small_m")
     stats["gemm_small_m"] += 1
     return out
+
 
 _NATIVE = True
 _GEMM_CTA_LIMIT = 0
@@ -433,11 +417,10 @@ def _small_m_shape(a: torch.Tensor, w: torch.Tensor) -> bool:
 def _small_m_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool, norm: tuple | None) -> torch.Tensor | None:
     (M, K), N = a.shape, w.shape[0]
     lib = _native.kernels()
-    ws = _small_m_workspace(int(lib.ft_gemm_small_m_workspace(M, N)), a.device)
     h = torch.empty((M, N), device=a.device, dtype=torch.bfloat16) if norm is not None else None
     alpha, nw, nb, scale = norm if norm is not None else (None, None, None, 1.0)
     rc = lib.ft_gemm_small_m_f32(a.data_ptr(), w.data_ptr(), out.data_ptr(), int(accumulate),
-                                 *(t.data_ptr() if t is not None else None for t in (alpha, nw, nb, h)), float(scale), ws.data_ptr(),
+                                 *(t.data_ptr() if t is not None else None for t in (alpha, nw, nb, h)), float(scale), None,
                                  M, N, K, a.stride(0), w.stride(0), out.stride(0), N, 0, _dev(a), _stream())
     _native.check(rc, "ft_gemm_small_m_f32")
     stats["gemm_small_m"] += 1

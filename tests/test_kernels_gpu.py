@@ -119,6 +119,28 @@ def test_gemm_small_m(M, N, K, ksplit):
     assert (F.stats["gemm_small_m"] > n0) == (N >= 1024 and K >= 512)
 
 
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 127, 128])
+@pytest.mark.parametrize("N,K", [(8, 64), (136, 128), (1000, 200), (3080, 4104), (2048, 8192), (9000, 520)])
+def test_gemm_small_m_tile_edges(M, N, K):
+    # clusters of 1, 2, 4 and 8 CTAs, ragged last tiles of W and of the contraction, rows around the multiples of 16
+    torch.manual_seed(M * 7 + N + K)
+    x, w, res, bias = _rand(M, K), _rand(N, K) * 0.05, _rand(M, N), _rand(N)
+    want = x.double() @ w.double().t()
+    # fp32 sums of K products of magnitude 0.05, then one rounding to bf16 (half of 2^-8 relative)
+    bound = 2.0 ** -8 * want.abs() + 0.05 * K ** 0.5 * 2.0 ** -18
+    y = F.gemm_small_m(x, w)
+    assert bool(((y.double() - want).abs() <= bound).all()) and torch.equal(F.gemm_small_m(x, w), y)
+    want = want + bias.double() + res.double()
+    got = F.gemm_small_m(x, w, bias=bias, residual=res)
+    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 0.05 * K ** 0.5 * 2.0 ** -18 + 2.0 ** -20).all())
+    if K > 64:
+        c0 = torch.randn(M, N, device=DEV)
+        c = c0.clone()
+        F._small_m_f32(x, w, c, True, None)
+        _assert_close(c.double(), c0.double() + x.double() @ w.double().t(), rtol=1e-5, atol=1e-3, what="fp32 accumulate")
+    assert _native.device_status(0) == 0
+
+
 def test_embedding_gradient_into_an_fp32_arena():
     # repeated and out-of-order ids; sums of bf16 rows in fp32, against 64 bits
     torch.manual_seed(5)
