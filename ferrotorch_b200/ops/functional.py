@@ -85,7 +85,30 @@ def native_enabled() -> bool:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle: torch.cuda.current_stream() builds a Stream object and looks its device up in the environment, 3.3 us a launch
+    # against 0.3
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+class _NoContext:
+    """Stands in for an autograd context where nothing is recorded."""
+
+    def save_for_backward(self, *tensors) -> None:
+        pass
+
+    def mark_dirty(self, *tensors) -> None:
+        for t in tensors:
+            if not t.is_inference():
+                torch.autograd.graph.increment_version(t)
+
+
+def _apply(fn, *args):
+    """``fn.apply(*args)``; without gradients, function transforms, forward-mode levels or tracing the forward by itself (a decoder layer's
+    16 us a call for a node that is thrown away)."""
+    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
+            or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling()):
+        return fn.apply(*args)
+    return fn.forward(_NoContext(), *args)
 
 
 def _dev(t: torch.Tensor) -> int:
@@ -216,7 +239,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -
     """``x @ w.T + bias`` with ``w [out, in]`` (ferrotorch-nn/src/linear.rs:166-211)."""
     if not _NATIVE or not x.is_cuda or x.dtype != torch.bfloat16:
         return torch.nn.functional.linear(x, w, bias)
-    return _LinearFn.apply(x, w, bias)
+    return _apply(_LinearFn, x, w, bias)
 
 
 # --------------------------------------------------------------------------- RMSNorm
@@ -225,7 +248,8 @@ _scratch: dict = {}
 
 def _get_scratch(key, numel: int, device, dtype=torch.float32) -> torch.Tensor:
     """Per-(stream, purpose) scratch buffer, grown on demand and reused across calls."""
-    k = (key, device, torch.cuda.current_stream(device).cuda_stream, dtype)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    k = (key, index, torch._C._cuda_getCurrentRawStream(index), dtype)
     buf = _scratch.get(k)
     if buf is None or buf.numel() < numel:
         buf = torch.empty(max(numel, 1), device=device, dtype=dtype)
@@ -310,7 +334,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5,
         return (y, x) if residual is not None else y
     if not _NATIVE or not x.is_cuda or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16:
         return ref.rmsnorm(x, weight, eps, residual)
-    return _RMSNormFn.apply(x, weight, eps, residual)
+    return _apply(_RMSNormFn, x, weight, eps, residual)
 
 
 # --------------------------------------------------------------------------- dynamic tanh and packed decoder rows
@@ -503,7 +527,7 @@ def rope_(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, *, positions: t
         rot = ref.rope(xs[:, :n_rot], cos, sin, positions.long(), interleaved)
         return torch.cat([rot, xs[:, n_rot:]], dim=1).reshape(x.shape)
     assert x.stride(-1) == 1 and x.stride(-2) == x.shape[-1], "rope_: heads must be packed"
-    return _RopeFn.apply(x, cos, sin, positions, n_rot, seq_len, pos_offset, interleaved)
+    return _apply(_RopeFn, x, cos, sin, positions, n_rot, seq_len, pos_offset, interleaved)
 
 
 # --------------------------------------------------------------------------- SwiGLU
@@ -548,7 +572,7 @@ def swiglu(gu: torch.Tensor, activation: str = "silu", param: float | None = Non
     act = _ACT_ID[activation]
     if not _NATIVE or not gu.is_cuda or gu.dtype != torch.bfloat16 or (gu.shape[-1] // 2) % 8:
         return ref.swiglu(gu, act)
-    return _SwiGLUFn.apply(gu, act)
+    return _apply(_SwiGLUFn, gu, act)
 
 
 # --------------------------------------------------------------------------- embedding
@@ -595,7 +619,7 @@ def embedding(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """Row gather ``weight[ids]`` (ferrotorch-gpu/src/bf16.rs:1065); the backward scatter-adds rows."""
     if not _NATIVE or not weight.is_cuda or weight.dtype != torch.bfloat16 or weight.shape[1] % 8:
         return torch.nn.functional.embedding(ids, weight)
-    return _EmbeddingFn.apply(ids, weight)
+    return _apply(_EmbeddingFn, ids, weight)
 
 
 # --------------------------------------------------------------------------- cross entropy

@@ -22,6 +22,7 @@ import torch
 from torch import nn
 
 from .. import _native
+from ..ops import functional as F
 
 
 def _pad(n: int, mult: int = 64) -> int:
@@ -178,7 +179,7 @@ class FlatTrainer:
             rc = lib.ft_grad_norm(a.grads.data_ptr(), a.numel, int(a.grads.dtype == torch.float32),
                                   self._norm_partial.data_ptr(), None, float(self.max_grad_norm or 0.0),
                                   self._norm_out.data_ptr(), a.device.index or 0,
-                                  torch.cuda.current_stream().cuda_stream)
+                                  F._stream())
             _native.check(rc, "ft_grad_norm")
         else:
             n = a.grads.float().norm()
@@ -230,7 +231,7 @@ class FlatTrainer:
         n = e - s
         if self.native:
             lib = _native.kernels()
-            dev, stream = a.device.index or 0, torch.cuda.current_stream().cuda_stream
+            dev, stream = a.device.index or 0, F._stream()
             gf32 = int(grads.dtype == torch.float32)
             gptr = grads.data_ptr() + s * grads.element_size()
             plp = a.params.data_ptr() + s * a.params.element_size() if a.params.dtype == torch.bfloat16 else None

@@ -176,3 +176,47 @@ def test_block_masks_and_einops_helpers():
         C.flex_attention(q[:, :, :4], k, v, block_mask=bm)
     x = torch.arange(12.0).view(3, 4)
     assert C.reduce(x, "a b -> a", "sum").tolist() == [6.0, 22.0, 38.0] and C.repeat(x, "a b -> a b c", c=2).shape == (3, 4, 2)
+
+
+def test_a_forward_runs_alone_only_where_nothing_looks_at_it():
+    from torch.autograd import forward_ad
+
+    from ferrotorch_b200.ops import functional as F
+
+    class Twice(torch.autograd.Function):
+        contexts: list = []
+
+        @staticmethod
+        def forward(ctx, x):
+            ctx.save_for_backward(x)
+            Twice.contexts.append(type(ctx))
+            x.mul_(2)
+            ctx.mark_dirty(x)
+            return x
+
+        @staticmethod
+        def backward(ctx, g):
+            return 2 * g
+
+        @staticmethod
+        def jvp(ctx, t):
+            return t.mul_(2)
+
+    def alone():
+        return Twice.contexts[-1] is F._NoContext
+
+    x = torch.ones(3)
+    with torch.no_grad():
+        before = x._version
+        assert torch.equal(F._apply(Twice, x), torch.full((3,), 2.0)) and alone() and x._version > before
+        with forward_ad.dual_level():
+            out = F._apply(Twice, forward_ad.make_dual(torch.ones(2), torch.ones(2)))
+            assert not alone() and torch.equal(forward_ad.unpack_dual(out).tangent, torch.full((2,), 2.0))
+        with pytest.raises(RuntimeError):                       # a function without a rule for it stays refused
+            torch.func.vmap(lambda t: F._apply(Twice, t))(torch.ones(2, 2))
+    with torch.inference_mode():
+        F._apply(Twice, torch.ones(2))
+        assert alone()
+    w = torch.ones(2, requires_grad=True)
+    F._apply(Twice, w * 1).sum().backward()
+    assert not alone() and torch.equal(w.grad, torch.full((2,), 2.0))
