@@ -89,6 +89,44 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
   }
 }
 
+// The same with 16-byte loads: D / 8 lanes a row, four rows of a head in flight per lane, so that it runs at memory bandwidth (1 x 8192
+// tokens, 32 heads of 128, attention and its backward: 2908 us with four bytes a lane and one row a warp, 2862 now; of it 134 MB, 20 us, are
+// read here).
+template <int D>
+__global__ void __launch_bounds__(256)
+attn_delta_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout, const float* __restrict__ lse,
+                      float* __restrict__ delta, float* __restrict__ lse2, int Sq, int Hq, long long ldo, long long lddo) {
+  constexpr int LANES = D / 8, GROUPS = 256 / LANES, ROWS = 4;
+  const int g = threadIdx.x / LANES, l = threadIdx.x % LANES, h = blockIdx.y, b = blockIdx.z;
+  const int i0 = blockIdx.x * (GROUPS * ROWS) + g;
+  uint4 ov[ROWS], dv[ROWS];
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k) {
+    const long long tok = static_cast<long long>(b) * Sq + min(i0 + k * GROUPS, Sq - 1);
+    ov[k] = __ldg(reinterpret_cast<const uint4*>(o + tok * ldo + static_cast<long long>(h) * D) + l);
+    dv[k] = __ldg(reinterpret_cast<const uint4*>(dout + tok * lddo + static_cast<long long>(h) * D) + l);
+  }
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k) {
+    const uint32_t a[4] = {ov[k].x, ov[k].y, ov[k].z, ov[k].w}, c[4] = {dv[k].x, dv[k].y, dv[k].z, dv[k].w};
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 x = unpack_bf16x2(a[j]), y = unpack_bf16x2(c[j]);
+      s += x.x * y.x + x.y * y.y;
+    }
+#pragma unroll
+    for (int m = LANES / 2; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    const int i = i0 + k * GROUPS;
+    if (l == 0 && i < Sq) {
+      const long long idx = (static_cast<long long>(b) * Hq + h) * Sq + i;
+      delta[idx] = s;
+      const float v = lse[idx];
+      lse2[idx] = (v == -INFINITY) ? INFINITY : v * 1.4426950408889634f;
+    }
+  }
+}
+
 // tmR1/tmR2: resident operands (dK/dV: K, V; dQ: Q, dO); tmC1/tmC2: streamed (dK/dV: Q, dO;
 // dQ: K, V).  All are 3-D maps {heads*D, seq, batch} with 64-element (128-byte) boxes.
 template <int HD, bool IS_DQ>
@@ -879,9 +917,16 @@ FT_API int ft_flash_attn_bwd(const void* q, const void* k, const void* v, const 
     const long long rows = static_cast<long long>(B) * Sq * Hq;
     const int threads = 256;
     const long long blocks = (rows * 32 + threads - 1) / threads;
-    attn_delta_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), lse, delta_scratch,
-        delta_scratch + rows, B, Sq, Hq, D, ldo, static_cast<long long>(Hq) * D);
+    const __nv_bfloat16 *ob = static_cast<const __nv_bfloat16*>(o), *db = static_cast<const __nv_bfloat16*>(dout);
+    const bool vectors = ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 15) == 0 && Hq < 65536 && B < 65536;
+    const long long lddo_ = static_cast<long long>(Hq) * D;
+    if (vectors && D == 128)
+      attn_delta_vec_kernel<128><<<dim3((Sq + 63) / 64, Hq, B), 256, 0, stream>>>(ob, db, lse, delta_scratch, delta_scratch + rows, Sq, Hq, ldo, lddo_);
+    else if (vectors && D == 64)
+      attn_delta_vec_kernel<64><<<dim3((Sq + 127) / 128, Hq, B), 256, 0, stream>>>(ob, db, lse, delta_scratch, delta_scratch + rows, Sq, Hq, ldo, lddo_);
+    else   // an output that a caller cut out at an odd place
+      attn_delta_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(ob, db, lse, delta_scratch, delta_scratch + rows, B, Sq, Hq, D,
+                                                                               ldo, lddo_);
     FT_CUDA_CHECK(cudaGetLastError());
     count_launch();
   }

@@ -130,3 +130,27 @@ def test_flash_bwd_packed_qkv_grad_layout():
     qr, kr, vr = ref_in[:, :, :Hq], ref_in[:, :, Hq:Hq + Hkv], ref_in[:, :, Hq + Hkv:]
     R.attention(qr, kr, vr, True)[0].backward(do.float())
     _close(qkv.grad, ref_in.grad, 3e-2, 3e-2, "packed dqkv")
+
+
+@pytest.mark.parametrize("D,offset", [(128, 0), (128, 4), (64, 0), (64, 4)])
+@pytest.mark.parametrize("Sq", [1, 63, 130])
+def test_flash_bwd_with_an_output_at_any_place(D, offset, Sq):
+    # the row sums of O * dO read 16 bytes at a time where both allow it; an output eight bytes into its buffer takes the narrow loads
+    from ferrotorch_b200.ops.attention import attention_block_backward
+
+    torch.manual_seed(D + Sq)
+    B, H = 2, 3
+    q, k, v, do = _rand(B, Sq, H, D), _rand(B, Sq, H, D), _rand(B, Sq, H, D), _rand(B, Sq, H, D, scale=0.5)
+    out, lse = F.flash_attn_fwd(q, k, v, False)
+    buf = torch.empty(out.numel() + offset, device=DEV, dtype=out.dtype)
+    moved = buf[offset:].view(out.shape)
+    moved.copy_(out)
+    want = attention_block_backward(q, k, v, out, lse, do, False)
+    got = attention_block_backward(q, k, v, moved, lse, do, False)
+    # the sums of D products differ in their order only: 2^-20 of them, then gradients rounded to bf16
+    for g, w, what in zip(got, want, ("dq", "dk", "dv")):
+        _close(g, w, 2.0 ** -8, 2.0 ** -7, what)
+    qr, kr, vr = (t.float().requires_grad_() for t in (q, k, v))
+    R.attention(qr, kr, vr, False)[0].backward(do.float())
+    for g, w, what in zip(got, (qr.grad, kr.grad, vr.grad), ("dq", "dk", "dv")):
+        _close(g, w, 3e-2, 3e-2, what)
