@@ -27,3 +27,16 @@ def test_forward_backward_match_torch(c, k, s, p, hw):
         P.use_native_pool(prev)
     assert torch.equal(y, ref)
     torch.testing.assert_close(x.grad.float(), gref.float(), rtol=2e-2, atol=2e-2)      # sums of up to 4 bf16 terms: order may differ
+
+
+def test_index_widths_agree():
+    # a batch whose vectors are counted in 64 bits (2^31 of them would not fit a test; the pooled rows of a slice have to be the same)
+    from ferrotorch_b200.ops import pool as P
+
+    x = torch.randn(5, 24, 33, 17, device="cuda", dtype=torch.bfloat16).contiguous(memory_format=torch.channels_last)
+    prev = P.use_native_pool(True)
+    try:
+        assert torch.equal(P.max_pool2d(x, 3, 2, 1), tF.max_pool2d(x, 3, 2, 1))
+        assert torch.equal(P.max_pool2d(x[3:], 3, 2, 1), tF.max_pool2d(x, 3, 2, 1)[3:])
+    finally:
+        P.use_native_pool(prev)
