@@ -500,7 +500,11 @@ static int launch_bwd(const CUtensorMap& r1, const CUtensorMap& r2, const CUtens
 //   warp 0 TMA producer, warp 1 MMA issuer, warp 2 TMEM allocator,
 //   warps 4-11 softmax (two per TMEM lane quarter, 32 score columns each), warps 12-15 dQ reduction
 constexpr int AF_THREADS = 512;
-constexpr int AF_STAGES = 2;
+// Three {Q_c, dO_c} stages, so that the load of a tile need not wait until the tile two steps before has been multiplied.  The room comes
+// from one P^T tile instead of two (its MMA is the first of a step) and from adding up dQ sixteen queries at a time.  1 x 8192 tokens, 32 / 8
+// heads of 128, causal, attention and its backward: 2961 us, 2946 now.
+constexpr int AF_STAGES = 3;
+constexpr int AF_DQ_ROWS = 16;   // queries of a dQ tile that are added to the accumulator at a time
 
 struct AttFusedCfg {
   static constexpr int HD = 128;
@@ -509,10 +513,10 @@ struct AttFusedCfg {
   static constexpr int PS_TILE = AB_R * AB_C * 2;       // P^T or dS^T: 128 rows x 128 bytes
   static constexpr int OFF_R = 0;
   static constexpr int OFF_C = 2 * R_TILE;
-  static constexpr int OFF_PS = OFF_C + AF_STAGES * 2 * C_TILE;   // 2 buffers x {P^T, dS^T}
-  static constexpr int DQ_TILE = AB_C * HD * 4;                   // dQ_c as fp32 [64 queries][128 dims]
-  static constexpr int OFF_DQ = OFF_PS + 2 * 2 * PS_TILE;
-  static constexpr int OFF_LD = OFF_DQ + DQ_TILE;                 // lse / delta, 2 buffers
+  static constexpr int OFF_PS = OFF_C + AF_STAGES * 2 * C_TILE;   // P^T, then two dS^T
+  static constexpr int DQ_TILE = AF_DQ_ROWS * HD * 4;             // part of dQ_c as fp32 [16 queries][128 dims], two of them
+  static constexpr int OFF_DQ = OFF_PS + 3 * PS_TILE;
+  static constexpr int OFF_LD = OFF_DQ + 2 * DQ_TILE;                 // lse / delta, 2 buffers
   static constexpr int OFF_BAR = OFF_LD + 2 * 2 * AB_C * 4;
   static constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
   // TMEM columns
@@ -545,9 +549,9 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   const uint32_t sbase = smem_u32(smem);
   const uint32_t sK = sbase + Cfg::OFF_R, sV = sK + Cfg::R_TILE;
   const uint32_t sC = sbase + Cfg::OFF_C;     // stage s: Q_c at sC + s*2*C_TILE, dO_c right after
-  const uint32_t sPS = sbase + Cfg::OFF_PS;   // buffer b: P^T at sPS + b*2*PS_TILE, dS^T right after
+  const uint32_t sP = sbase + Cfg::OFF_PS, sDS = sP + Cfg::PS_TILE;   // dS^T of step t at sDS + (t & 1) * PS_TILE
   enum { R_FULL = 0, C_FULL = 1, C_EMPTY = C_FULL + AF_STAGES, S_FULL = C_EMPTY + AF_STAGES, S_READ = S_FULL + 1,
-         P_FULL = S_READ + 1, PS_EMPTY = P_FULL + 2, DQ_FULL = PS_EMPTY + 2, DQ_EMPTY = DQ_FULL + 2,
+         P_FULL = S_READ + 1, P_EMPTY = P_FULL + 2, DS_EMPTY = P_EMPTY + 1, DQ_FULL = DS_EMPTY + 2, DQ_EMPTY = DQ_FULL + 2,
          ACC_FULL = DQ_EMPTY + 2, NBARS = ACC_FULL + 1 };
   const uint32_t bar0 = sbase + Cfg::OFF_BAR;
   auto bar = [&](int i) { return bar0 + 8u * i; };
@@ -581,10 +585,11 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     mbar_init(bar(S_READ), 4 * AB_SPLIT);      // every softmax warp has its scores in registers
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar(P_FULL + s), 4 * AB_SPLIT);
-      mbar_init(bar(PS_EMPTY + s), 1);
+      mbar_init(bar(DS_EMPTY + s), 1);
       mbar_init(bar(DQ_FULL + s), 1);
       mbar_init(bar(DQ_EMPTY + s), 4);
     }
+    mbar_init(bar(P_EMPTY), 1);
     mbar_init(bar(ACC_FULL), 1);
     fence_mbar_init();
     tma_prefetch_desc(&tmK);
@@ -672,12 +677,15 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
         if (!ok) break;
         tc_fence_after();
         const uint32_t c1 = sC + st * 2 * Cfg::C_TILE, c2 = c1 + Cfg::C_TILE;
-        const uint32_t sPt = sPS + pb * 2 * Cfg::PS_TILE, sDSt = sPt + Cfg::PS_TILE;
+        const uint32_t sDSt = sDS + pb * Cfg::PS_TILE;
+        // dV += P^T dO_c, then dK += dS^T Q_c   (A: 128 keys x 64 queries K-major; B: streamed tile MN-major)
+#pragma unroll
+        for (int kk = 0; kk < AB_C / 16; ++kk)
+          umma_f16_ss(tmem_base + Cfg::COL_DV, make_smem_desc_sw128(sP + kk * 32, 16, 1024),
+                      make_smem_desc_sw128(c2 + kk * 2048, AB_C * 128, 1024), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(bar(P_EMPTY));
 #pragma unroll
         for (int kk = 0; kk < AB_C / 16; ++kk) {
-          // dV += P^T dO_c ; dK += dS^T Q_c   (A: 128 keys x 64 queries K-major; B: streamed tile MN-major)
-          umma_f16_ss(tmem_base + Cfg::COL_DV, make_smem_desc_sw128(sPt + kk * 32, 16, 1024),
-                      make_smem_desc_sw128(c2 + kk * 2048, AB_C * 128, 1024), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
           umma_f16_ss(tmem_base + Cfg::COL_DK, make_smem_desc_sw128(sDSt + kk * 32, 16, 1024),
                       make_smem_desc_sw128(c1 + kk * 2048, AB_C * 128, 1024), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
         }
@@ -690,7 +698,7 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
                       make_smem_desc_sw128(sDSt + kk * 2048, AB_C * 128, 1024), idesc_dq, kk > 0 ? 1u : 0u);
         }
         umma_commit(bar(DQ_FULL + pb));
-        umma_commit(bar(PS_EMPTY + pb));
+        umma_commit(bar(DS_EMPTY + pb));
       }
       if (ok) umma_commit(bar(ACC_FULL));
     }
@@ -755,17 +763,19 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
           dk[c >> 1] = pack_bf16x2(dv[0], dv[1]);
           dk[(c >> 1) + 1] = pack_bf16x2(dv[2], dv[3]);
         }
-        // the P^T / dS^T buffer of this parity was last read by the MMAs of step t - 2
-        if (!mbar_wait(bar(PS_EMPTY + pb), ((t >> 1) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_EPILOGUE)) ok = false;
+        // P^T was last read by step t - 1 (the first MMA behind its P_FULL), the dS^T tile of this parity by step t - 2
+        if (!mbar_wait(bar(DS_EMPTY + pb), ((t >> 1) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_EPILOGUE) ||
+            !mbar_wait(bar(P_EMPTY), (t & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_EPILOGUE))
+          ok = false;
         if (ok) {
-          const uint32_t ps = sPS + pb * 2 * Cfg::PS_TILE;
+          const uint32_t ds = sDS + pb * Cfg::PS_TILE;
 #pragma unroll
           for (int uu = 0; uu < 4; ++uu) {
             const int u = half * 4 + uu;
             const uint32_t off = r * 128 + ((u ^ (r & 7)) << 4);
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ps + off), "r"(pk[uu * 4]),
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sP + off), "r"(pk[uu * 4]),
                          "r"(pk[uu * 4 + 1]), "r"(pk[uu * 4 + 2]), "r"(pk[uu * 4 + 3]) : "memory");
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ps + Cfg::PS_TILE + off), "r"(dk[uu * 4]),
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ds + off), "r"(dk[uu * 4]),
                          "r"(dk[uu * 4 + 1]), "r"(dk[uu * 4 + 2]), "r"(dk[uu * 4 + 3]) : "memory");
           }
           fence_proxy_async_smem();
@@ -838,29 +848,32 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(DQ_EMPTY + pb));
       }
-      // the staging tile is free once the previous step's reduce has read it
-      if (threadIdx.x == 12 * 32) tma_store_wait_read<0>();
-      asm volatile("bar.sync 2, 128;" ::: "memory");
-      if (ok) {
-        // transpose: thread d writes column d of the [64 queries][128 dims] tile (a warp writes
-        // 32 consecutive floats of one row: no bank conflicts)
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(sDQ + static_cast<uint32_t>(j * HD + d) * 4u), "r"(v0[j]) : "memory");
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(sDQ + static_cast<uint32_t>((32 + j) * HD + d) * 4u), "r"(v1[j])
-                       : "memory");
+      for (int part = 0; part < AB_C / AF_DQ_ROWS; ++part) {
+        const uint32_t tile = sDQ + (part & 1) * Cfg::DQ_TILE;
+        // the staging tile is free once the reduce before the previous one has read it
+        if (threadIdx.x == 12 * 32) tma_store_wait_read<1>();
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+        if (ok) {
+          // transpose: thread d writes column d of the [16 queries][128 dims] tile (a warp writes
+          // 32 consecutive floats of one row: no bank conflicts)
+#pragma unroll
+          for (int j = 0; j < AF_DQ_ROWS; ++j)
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + static_cast<uint32_t>(j * HD + d) * 4u),
+                         "r"(part < 2 ? v0[part * AF_DQ_ROWS + j] : v1[(part - 2) * AF_DQ_ROWS + j]) : "memory");
+          fence_proxy_async_smem();
         }
-        fence_proxy_async_smem();
-      }
-      asm volatile("bar.sync 2, 128;" ::: "memory");
-      if (ok && threadIdx.x == 12 * 32) {
-        // dq_acc[batch, q0 .. q0+63, head, :] += tile (queries past Sq are clipped by the tensor map)
-        asm volatile(
-            "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-            :
-            : "l"(reinterpret_cast<uint64_t>(&tmDQ)), "r"(sDQ), "r"(iter_head(t) * HD), "r"(iter_cblk(t) * AB_C), "r"(batch)
-            : "memory");
-        tma_store_commit();
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+        if (ok && threadIdx.x == 12 * 32) {
+          // dq_acc[batch, q0 .. q0 + 15, head, :] += tile (queries past Sq are clipped by the tensor map)
+          if (iter_cblk(t) * AB_C + part * AF_DQ_ROWS < p.Sq) asm volatile(
+              "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+              :
+              : "l"(reinterpret_cast<uint64_t>(&tmDQ)), "r"(tile), "r"(iter_head(t) * HD),
+                "r"(iter_cblk(t) * AB_C + part * AF_DQ_ROWS), "r"(batch)
+              : "memory");
+          tma_store_commit();
+        }
       }
     }
     if (threadIdx.x == 12 * 32) tma_store_wait<0>();   // shared memory must outlive the reduce that reads it
@@ -965,10 +978,10 @@ FT_API int ft_flash_attn_bwd(const void* q, const void* k, const void* v, const 
                                          AttFusedCfg::SMEM_BYTES));
       attr_set[device] = true;
     }
-    // dq_acc as {Hq*D, Sq, B} fp32; one box = 128 dims x 64 queries, unswizzled (512-byte rows)
+    // dq_acc as {Hq*D, Sq, B} fp32; one box = 128 dims x 16 queries, unswizzled (512-byte rows)
     CUtensorMap tdq;
     rc = make_tmap_3d(&tdq, dq_acc, 4, static_cast<uint64_t>(Hq) * D, Sq, B, static_cast<uint64_t>(Hq) * D * 4,
-                      static_cast<uint64_t>(Sq) * Hq * D * 4, 128, AB_C, 1, 0);
+                      static_cast<uint64_t>(Sq) * Hq * D * 4, 128, AF_DQ_ROWS, 1, 0);
     if (rc) return rc;
     dim3 grid((Sk + AB_R - 1) / AB_R, Hkv, B);
     flash_bwd_fused_kernel<<<grid, AF_THREADS, AttFusedCfg::SMEM_BYTES, stream>>>(tk_r, tv_r, tq_c, tdo_c, tdq, f);

@@ -154,3 +154,14 @@ def test_flash_bwd_with_an_output_at_any_place(D, offset, Sq):
     R.attention(qr, kr, vr, False)[0].backward(do.float())
     for g, w, what in zip(got, (qr.grad, kr.grad, vr.grad), ("dq", "dk", "dv")):
         _close(g, w, 3e-2, 3e-2, what)
+
+
+@pytest.mark.parametrize("Sq,Sk,causal", [(1, 128, False), (15, 130, False), (16, 16, True), (17, 200, True), (49, 49, True), (65, 300, False), (128, 129, True),
+                                          (193, 193, True)])
+@pytest.mark.parametrize("Hq,Hkv", [(1, 1), (6, 2)])
+def test_flash_bwd_ragged_parts_of_a_query_tile(Sq, Sk, causal, Hq, Hkv):
+    # one to twelve steps through the three stages; dQ is added sixteen queries at a time, the last of them past Sq or cut by it.
+    # Gradients lie in the middle of a larger buffer's rows' worth of scratch only if nothing is written past Sq: the next batch would show it
+    from ferrotorch_b200.ops.attention import flash_attention
+
+    _flash_bwd_case(flash_attention, 2, Sq, Sk, Hq, Hkv, 128, causal)
