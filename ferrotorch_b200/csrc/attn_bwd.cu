@@ -21,6 +21,7 @@
 // memory.  The softmax scale is applied once, to the accumulators in the epilogue.  In the dK/dV
 // pass the per-query lse / delta of the next block are fetched one step ahead into shared memory.
 // All waits are bounded.
+#include "attn_order.cuh"
 #include "ft_host.h"
 #include "ft_ptx.cuh"
 
@@ -151,22 +152,23 @@ flash_bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_
   float* ld_buf = reinterpret_cast<float*>(smem + Cfg::OFF_LD);  // [2 buffers][lse | delta][AB_C]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int batch = blockIdx.z;
+  const AttnBlock at = attn_block(((IS_DQ ? p.Sq : p.Sk) + AB_R - 1) / AB_R, IS_DQ ? p.Hq : p.Hkv, p.causal);
+  const int batch = at.batch;
   const int group = p.Hq / p.Hkv;
   // resident tile index; heavy tiles first under a causal mask
   int rblk, head_r;  // head_r: kv head (dK/dV) or q head (dQ)
-  head_r = blockIdx.y;
+  head_r = at.head;
   int c_begin, c_end, n_heads_iter;
   if constexpr (IS_DQ) {
     const int nb = (p.Sq + AB_R - 1) / AB_R;
-    rblk = nb - 1 - blockIdx.x;
+    rblk = nb - 1 - at.block;
     c_begin = 0;
     int kv_end = p.Sk;
     if (p.causal) kv_end = min(p.Sk, rblk * AB_R + AB_R + p.causal_offset);
     c_end = kv_end > 0 ? (kv_end + AB_C - 1) / AB_C : 0;
     n_heads_iter = 1;
   } else {
-    rblk = blockIdx.x;
+    rblk = at.block;
     c_end = (p.Sq + AB_C - 1) / AB_C;
     c_begin = 0;
     if (p.causal) {
@@ -473,7 +475,7 @@ static int launch_bwd(const CUtensorMap& r1, const CUtensorMap& r2, const CUtens
     FT_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     attr_set[device] = true;
   }
-  dim3 grid(IS_DQ ? (p.Sq + AB_R - 1) / AB_R : (p.Sk + AB_R - 1) / AB_R, IS_DQ ? p.Hq : p.Hkv, p.B);
+  const dim3 grid = attn_grid(IS_DQ ? (p.Sq + AB_R - 1) / AB_R : (p.Sk + AB_R - 1) / AB_R, IS_DQ ? p.Hq : p.Hkv, p.B);
   kern<<<grid, AB_THREADS, Cfg::SMEM_BYTES, stream>>>(r1, r2, c1, c2, p);
   FT_CUDA_CHECK(cudaGetLastError());
   count_launch();
@@ -560,7 +562,8 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   float* ld_buf = reinterpret_cast<float*>(smem + Cfg::OFF_LD);  // [2 buffers][lse | delta][AB_C]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int batch = blockIdx.z, kvh = blockIdx.y, rblk = blockIdx.x;
+  const AttnBlock at = attn_block((p.Sk + AB_R - 1) / AB_R, p.Hkv, p.causal);   // the first keys are the heaviest
+  const int batch = at.batch, kvh = at.head, rblk = at.block;
   const int group = p.Hq / p.Hkv;
   int c_end = (p.Sq + AB_C - 1) / AB_C, c_begin = 0;
   if (p.causal) {
@@ -983,7 +986,7 @@ FT_API int ft_flash_attn_bwd(const void* q, const void* k, const void* v, const 
     rc = make_tmap_3d(&tdq, dq_acc, 4, static_cast<uint64_t>(Hq) * D, Sq, B, static_cast<uint64_t>(Hq) * D * 4,
                       static_cast<uint64_t>(Sq) * Hq * D * 4, 128, AF_DQ_ROWS, 1, 0);
     if (rc) return rc;
-    dim3 grid((Sk + AB_R - 1) / AB_R, Hkv, B);
+    const dim3 grid = attn_grid((Sk + AB_R - 1) / AB_R, Hkv, B);
     flash_bwd_fused_kernel<<<grid, AF_THREADS, AttFusedCfg::SMEM_BYTES, stream>>>(tk_r, tv_r, tq_c, tdo_c, tdq, f);
     FT_CUDA_CHECK(cudaGetLastError());
     count_launch();

@@ -19,6 +19,7 @@
 //              max/sum need no shuffles; P goes back through shared memory (128B swizzle)
 //              as the A operand of the second MMA; O is rescaled in TMEM when a row max moves
 // All waits are bounded and report through the device status word.
+#include "attn_order.cuh"
 #include "attn_row.cuh"
 #include "ft_host.h"
 
@@ -71,8 +72,9 @@ flash_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qblocks = (p.Sq + ATT_BM - 1) / ATT_BM;
-  const int qb = n_qblocks - 1 - blockIdx.x;  // heaviest (latest) query blocks first
-  const int head = blockIdx.y, batch = blockIdx.z;
+  const AttnBlock at = attn_block(n_qblocks, p.Hq, p.causal);
+  const int qb = n_qblocks - 1 - at.block;  // heaviest (latest) query blocks first
+  const int head = at.head, batch = at.batch;
   const int kv_head = head / (p.Hq / p.Hkv);
   const int q0 = qb * ATT_BM;
   int kv_end = p.Sk;
@@ -315,7 +317,7 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     FT_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     attr_set[device] = true;
   }
-  dim3 grid((p.Sq + ATT_BM - 1) / ATT_BM, p.Hq, p.B);
+  const dim3 grid = attn_grid((p.Sq + ATT_BM - 1) / ATT_BM, p.Hq, p.B);
   kern<<<grid, ATT_THREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   FT_CUDA_CHECK(cudaGetLastError());
   count_launch();
@@ -370,8 +372,9 @@ flash_fwd2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qpairs = (p.Sq + 2 * ATT_BM - 1) / (2 * ATT_BM);
-  const int qp = n_qpairs - 1 - blockIdx.x;  // heaviest (latest) query blocks first
-  const int head = blockIdx.y, batch = blockIdx.z;
+  const AttnBlock at = attn_block(n_qpairs, p.Hq, p.causal);
+  const int qp = n_qpairs - 1 - at.block;  // heaviest (latest) query blocks first
+  const int head = at.head, batch = at.batch;
   const int kv_head = head / (p.Hq / p.Hkv);
   const int q0 = qp * 2 * ATT_BM;
   // number of key blocks each tile needs
@@ -631,7 +634,7 @@ static int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     FT_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     attr_set[device] = true;
   }
-  dim3 grid((p.Sq + 2 * ATT_BM - 1) / (2 * ATT_BM), p.Hq, p.B);
+  const dim3 grid = attn_grid((p.Sq + 2 * ATT_BM - 1) / (2 * ATT_BM), p.Hq, p.B);
   kern<<<grid, ATT2_THREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   FT_CUDA_CHECK(cudaGetLastError());
   count_launch();

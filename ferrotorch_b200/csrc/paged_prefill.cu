@@ -86,9 +86,10 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.y;
-  const int slot = p.items[4 * blockIdx.x], row0 = p.items[4 * blockIdx.x + 1];
-  const int n_tok = p.items[4 * blockIdx.x + 2], pos0 = p.items[4 * blockIdx.x + 3];
+  // the items are sorted by weight: all heads of the heaviest first (see attn_order.cuh)
+  const int item = blockIdx.x / p.Hkv, kvh = blockIdx.x - item * p.Hkv;
+  const int slot = p.items[4 * item], row0 = p.items[4 * item + 1];
+  const int n_tok = p.items[4 * item + 2], pos0 = p.items[4 * item + 3];
   // tokens and key blocks of each tile
   int nt[2], nb[2];
   // blocks of pooled means, which the item's last token sees, then blocks of keys: number n_pool of this item is key block j0
@@ -422,7 +423,7 @@ static int launch_prefill(const CUtensorMap& tq, const CUtensorMap& tk, const CU
     FT_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     attr_set[device] = true;
   }
-  kern<<<dim3(n_items, p.Hkv), PP_THREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, tkp, tvp, p);
+  kern<<<dim3(static_cast<unsigned>(n_items) * p.Hkv), PP_THREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, tkp, tvp, p);
   FT_CUDA_CHECK(cudaGetLastError());
   count_launch();
   return FT_E_OK;

@@ -165,3 +165,14 @@ def test_flash_bwd_ragged_parts_of_a_query_tile(Sq, Sk, causal, Hq, Hkv):
     from ferrotorch_b200.ops.attention import flash_attention
 
     _flash_bwd_case(flash_attention, 2, Sq, Sk, Hq, Hkv, 128, causal)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("B,S,Hq,Hkv,D", [(3, 700, 6, 2, 128), (2, 129, 3, 3, 64), (1, 1153, 5, 1, 128), (5, 64, 2, 1, 64)])
+def test_every_block_of_every_head_is_taken_once(B, S, Hq, Hkv, D, causal):
+    # the order of the work depends on the mask; numbers of blocks, heads and sequences that do not divide each other
+    from ferrotorch_b200.ops.attention import flash_attention
+
+    _flash_bwd_case(flash_attention, B, S, S, Hq, Hkv, D, causal)
+    q, k, v = _rand(B, S, Hq, D), _rand(B, S, Hkv, D), _rand(B, S, Hkv, D)
+    _close(F.flash_attn_fwd(q, k, v, causal)[0], R.attention(q, k, v, causal)[0], 2e-2, 2e-2, "out")
