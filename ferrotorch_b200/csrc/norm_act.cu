@@ -307,6 +307,58 @@ __global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __re
   }
 }
 
+// Rotation (pair (d, d + D/2)) of the q and k heads of packed rows x [T, ld] (Hq query, Hkv key, Hkv value heads of D), the keys and values
+// going to their cache pages: q in place, k rotated into the cache (the row's k stays as it is), v copied.  One launch and one read of
+// k and v instead of a rotation in place and an append behind it; a thread owns eight pairs, or eight elements of v.
+__global__ void rope_append_kernel(__nv_bfloat16* x, const float* __restrict__ cos_t, const float* __restrict__ sin_t, const int* pos,
+                                   const int* slots, const int* block_table, uint4* k_cache, uint4* v_cache, int T, int Hq, int Hkv, int D,
+                                   long long ld, int block_size, int max_blocks, int num_blocks) {
+  grid_dependency_launch();
+  grid_dependency_wait();
+  const int half = D >> 1, pairs = half >> 3, vecs = D >> 3;
+  const int q_items = Hq * pairs, k_items = Hkv * pairs, items = q_items + k_items + Hkv * vecs;
+  const long long total = static_cast<long long>(T) * items;
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int t = static_cast<int>(i / items), r = static_cast<int>(i - static_cast<long long>(t) * items);
+    const int p = pos[t];
+    long long row = -1;                                          // this token's place in the cache
+    if (r >= q_items) {
+      const int blk = block_table[static_cast<long long>(slots[t]) * max_blocks + p / block_size];
+      if (blk < 0 || blk >= num_blocks) continue;                // a row of no sequence
+      row = (static_cast<long long>(blk) * block_size + p % block_size) * Hkv * vecs;
+    }
+    __nv_bfloat16* token = x + static_cast<size_t>(t) * ld;
+    if (r >= q_items + k_items) {
+      const int v = r - q_items - k_items;
+      v_cache[row + v] = reinterpret_cast<const uint4*>(token + static_cast<size_t>(Hq + Hkv) * D)[v];
+      continue;
+    }
+    const int h = r / pairs, d = (r - h * pairs) << 3;           // head among q and k, first pair
+    const float4* cp = reinterpret_cast<const float4*>(cos_t + static_cast<size_t>(p) * half + d);
+    const float4* sp = reinterpret_cast<const float4*>(sin_t + static_cast<size_t>(p) * half + d);
+    const float4 c0 = cp[0], c1 = cp[1], s0 = sp[0], s1 = sp[1];
+    const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+    const float sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+    uint4* p1 = reinterpret_cast<uint4*>(token + static_cast<size_t>(h) * D + d);
+    uint4* p2 = reinterpret_cast<uint4*>(token + static_cast<size_t>(h) * D + d + half);
+    float a[8], b[8], oa[8], ob[8];
+    unpack8(*p1, a);
+    unpack8(*p2, b);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      oa[j] = a[j] * c[j] - b[j] * sn[j];
+      ob[j] = b[j] * c[j] + a[j] * sn[j];
+    }
+    if (h >= Hq) {
+      p1 = k_cache + row + (h - Hq) * vecs + (d >> 3);
+      p2 = p1 + (half >> 3);
+    }
+    *p1 = pack8(oa);
+    *p2 = pack8(ob);
+  }
+}
+
 // ---------------------------------------------------------------- SwiGLU
 // gu: [T, 2F] (gate = [:, :F], up = [:, F:]), out: [T, F].  act: 0 silu, 1 relu, 2 gelu(tanh).
 __device__ __forceinline__ float act_fwd(float g, int act) {
@@ -661,6 +713,27 @@ FT_API int ft_rope(void* x, const float* cos_t, const float* sin_t, const int* p
         static_cast<__nv_bfloat16*>(x), cos_t, sin_t, pos, T, n_rot_heads, D, ld, seq_len, pos_offset,
         interleaved, backward ? -1.f : 1.f);
   FT_CUDA_CHECK(cudaGetLastError());
+  count_launch();
+  return FT_E_OK;
+}
+
+// See rope_append_kernel.  x: bf16 rows of (Hq + 2 Hkv) heads of D (stride ld elements); the caches are [num_blocks, block_size, Hkv, D];
+// pos, slots: int32 [T]; cos_t, sin_t: fp32 [positions, D / 2].
+FT_API int ft_rope_append(void* x, const float* cos_t, const float* sin_t, const int* pos, const int* slots, const int* block_table,
+                          void* k_cache, void* v_cache, int T, int Hq, int Hkv, int D, long long ld, int block_size, int max_blocks,
+                          int num_blocks, int device, cudaStream_t stream) {
+  if (int _rc = ft::ensure_device(device)) return _rc;
+  FT_REQUIRE(x && cos_t && sin_t && pos && slots && block_table && k_cache && v_cache, "ft_rope_append: null pointer");
+  FT_REQUIRE(Hq > 0 && Hkv > 0 && D > 0 && D % 16 == 0 && ld % 8 == 0 && block_size > 0 && max_blocks > 0 && num_blocks > 0,
+             "ft_rope_append: heads of %d must be multiples of 16, rows of 8", D);
+  FT_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t) |
+               reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0,
+             "ft_rope_append: pointers must be 16-byte aligned");
+  if (T <= 0) return FT_E_OK;
+  const long long work = static_cast<long long>(T) * ((Hq + Hkv) * (D / 16) + Hkv * (D / 8));
+  FT_CUDA_CHECK(launch_dependent(rope_append_kernel, blocks_for(work, 256, device), 256, 0, stream, static_cast<__nv_bfloat16*>(x), cos_t, sin_t,
+                                 pos, slots, block_table, static_cast<uint4*>(k_cache), static_cast<uint4*>(v_cache), T, Hq, Hkv, D, ld,
+                                 block_size, max_blocks, num_blocks));
   count_launch();
   return FT_E_OK;
 }

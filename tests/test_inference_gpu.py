@@ -152,3 +152,33 @@ def test_engine_q4_0_single_gpu():
 @pytest.mark.multigpu
 def test_engine_q4_0_tensor_parallel_2():
     _run(2, 29553, weights="q4_0")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,Hq,Hkv", [(64, 4, 4), (128, 8, 2), (16, 1, 1), (96, 6, 2)])
+def test_rotation_into_the_pages_is_rotation_then_append(D, Hq, Hkv):
+    # rows of several sequences at positions within, at the edge of and past a page, and a padding row of no sequence
+    from ferrotorch_b200.nn.layers import RotaryPositionEmbedding
+    from ferrotorch_b200.nn.paged import RaggedBatch
+
+    torch.manual_seed(D + Hq)
+    rope = RotaryPositionEmbedding(D, 256)
+    with torch.no_grad():
+        results = []
+        packed = torch.randn(1 + 1 + 40, Hq + 2 * Hkv, D, device="cuda").to(torch.bfloat16)
+        for fused in (True, False):
+            cache = PagedKVCache(2, Hkv, D, num_blocks=16, max_seqs=3, max_seq_len=256, block_size=16)
+            mgr = PagedAttentionManager(cache)
+            for n in (17, 60, 40):
+                mgr.add_sequence(n)
+            batch = RaggedBatch([(0, [1], 16, [0]), (cache.pad_slot, [1], 0, [0]), (1, list(range(40)), 15, [39])], "cuda")
+            x = packed.clone()
+            if fused:
+                cache.append_rotated(1, x, rope, batch, Hq)
+            else:
+                x = rope(x[None], positions=batch.positions, n_rot_heads=Hq + Hkv)[0]
+                cache.append(1, x[:, Hq:Hq + Hkv], x[:, Hq + Hkv:], batch.positions, batch.slots)
+            results.append((x[:, :Hq].clone(), cache.k[1], cache.v[1], cache.k[0]))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert bool(results[0][1].any()) and not bool(results[0][3].any())
