@@ -1,9 +1,9 @@
-// GEMM for few rows against a large weight (decode):  C[M, N] (+)= X[M, K] W[N, K]^T, M <= 128, bf16, fp32 accumulation.
+// GEMM for few rows against a large weight (decode, short prompts):  C[M, N] (+)= X[M, K] W[N, K]^T, bf16, fp32 accumulation.
 //
 // Such a product is bound by the bytes of W (64 rows of a 4096 x 14336 product: 117 MB, 18 us at 6.6 TB/s; 0.5 us of tensor-core time)
 // and, where W is small, by the chain of latencies of one launch:
-//   * W is the 128-row operand of the MMA, the rows of X are its N dimension (16 .. 128, a multiple of 16), so that no tensor-core row
-//     is padding and X costs little shared memory;
+//   * W is the 128-row operand of the MMA, the rows of X are its N dimension (16 .. 256, a multiple of 16; more rows are cut into equal
+//     row tiles), so that no tensor-core row is padding and X costs little shared memory;
 //   * a thread-block cluster of up to eight CTAs works on one 128-row tile of W, each on its part of the contraction, so that even a
 //     weight of 2048 rows is read by 128 SMs;
 //   * the parts meet in shared memory: CTA j of the cluster is sent its 128 / S columns of every part, adds them in the order of the
@@ -30,7 +30,9 @@ constexpr int ST_A_BYTES = ST_BM * ST_BK * 2;
 constexpr int ST_BUF_BYTES = 216 * 1024;   // ring of operand tiles, then the parts that this CTA adds
 constexpr int ST_MAX_STAGES = 11;
 constexpr int ST_SMEM = ST_BUF_BYTES + 1024 + 512;
-constexpr int ST_MAX_ROWS = 128;
+constexpr int ST_MAX_ROWS = 256;           // rows of X in a tile
+constexpr int ST_PART_ROWS = 64;           // rows whose parts meet at a time
+constexpr int ST_PARTS_BYTES = ST_BM * ST_PART_ROWS * 4;
 constexpr int ST_MAX_CLUSTER = 8;
 constexpr int ST_PREFETCH = 24;            // k-blocks of W that a CTA asks for while the kernel before it ends
 
@@ -41,7 +43,7 @@ struct StreamParams {
   const float *alpha, *dyt_w, *dyt_b;   // dynamic tanh of the new values (fp32 results only)
   __nv_bfloat16* dyt_out;
   float dyt_scale;
-  int M, N, tiles, k_blocks, cluster, bn, stages, flags, accumulate, vec, vec_r;
+  int M, N, tiles, m_tiles, k_blocks, cluster, bn, stages, flags, accumulate, vec, vec_r;
   long long ldc, ldr, ldd;
   int* status;
 };
@@ -147,8 +149,10 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     // W does not come from the kernel before this one in most uses, but it may: it is only brought into L2 ahead of the wait, and read
     // behind it
     int left = ST_PREFETCH;
-    for (int tile = first; tile < p.tiles && left > 0; tile += step)
-      for (int kb = kb0; kb < kb1 && left > 0; ++kb, --left) tma_prefetch_l2_2d(&tmW, kb * ST_BK, tile * ST_BM);
+    for (int tile = first; tile < p.tiles && left > 0; tile += step) {
+      const int n0 = p.m_tiles == 1 ? tile * ST_BM : tile / p.m_tiles * ST_BM;
+      for (int kb = kb0; kb < kb1 && left > 0; ++kb, --left) tma_prefetch_l2_2d(&tmW, kb * ST_BK, n0);
+    }
   }
   if (warp == 2) {
     tmem_alloc(smem_u32(tmem_slot), tmem_cols);
@@ -168,13 +172,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       uint32_t phase = 0;
       bool ok = true;
       for (int tile = first; tile < p.tiles && ok; tile += step) {
+        const int wt = p.m_tiles == 1 ? tile : tile / p.m_tiles, n0 = wt * ST_BM, m0 = (tile - wt * p.m_tiles) * p.bn;
         for (int kb = kb0; kb < kb1; ++kb) {
           ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER);
           if (!ok) break;
           const uint32_t sW = smem_base + stage * stage_bytes;
           mbar_expect_tx(full_bar(stage), stage_bytes);
-          tma_load_2d(sW, &tmW, full_bar(stage), kb * ST_BK, tile * ST_BM);
-          tma_load_2d(sW + ST_A_BYTES, &tmX, full_bar(stage), kb * ST_BK, 0);
+          tma_load_2d(sW, &tmW, full_bar(stage), kb * ST_BK, n0);
+          tma_load_2d(sW + ST_A_BYTES, &tmX, full_bar(stage), kb * ST_BK, m0);
           if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -220,56 +225,62 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     const uint32_t parts = smem_base + static_cast<uint32_t>(stages) * stage_bytes;
     // Parts lie as [CTA that sent it][row of X][column]: the lanes of a warp write and read neighbouring words.  (Four rows of a column
     // as one 16-byte store to the peer took three times as long.)
-    const uint32_t mine = mapa_shared(parts, col / cols) + static_cast<uint32_t>(rank * p.bn * cols + col % cols) * 4u;
+    const uint32_t mine = mapa_shared(parts, col / cols) + static_cast<uint32_t>(rank * ST_PART_ROWS * cols + col % cols) * 4u;
     const float* all = reinterpret_cast<const float*>(smem + stages * stage_bytes);
     const int mc = (threadIdx.x - 128) % (cols / 4) * 4, mr = (threadIdx.x - 128) / (cols / 4), m_step = ST_EPI_WARPS * 32 / (cols / 4);
     int acc = 0;
-    uint32_t acc_phase = 0, tile_phase = 0;
-    for (int tile = first; tile < p.tiles; tile += step, tile_phase ^= 1u) {
-      if (!mbar_wait(tfull_bar(acc), acc_phase, abort_word, FT_ERR_TIMEOUT_EPILOGUE)) break;
-      if (tile != first && !mbar_wait_cluster(parts_free, tile_phase ^ 1u, abort_word, FT_ERR_TIMEOUT_EPILOGUE)) break;
-      tc_fence_after();
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * p.bn);
-#pragma unroll 1
-      for (int c = half * 16; c < p.M; c += 32) {
-        uint32_t r[16];
-        tmem_ld_32x16(t_row + c, r);
-        tmem_ld_wait();
+    uint32_t acc_phase = 0, meeting = 0;
+    bool ok = true;
+    for (int tile = first; tile < p.tiles && ok; tile += step) {
+      const int wt = p.m_tiles == 1 ? tile : tile / p.m_tiles, m0 = (tile - wt * p.m_tiles) * p.bn, rows = min(p.bn, p.M - m0);
+      const int n = wt * ST_BM + rank * cols + mc, left = p.N - n;
+      float bias[4] = {0.f, 0.f, 0.f, 0.f};
+      if (p.flags & (GEMM_BIAS | GEMM_BIAS_F32)) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (c + j < p.M) st_cluster(mine + static_cast<uint32_t>((c + j) * cols) * 4u, r[j]);
+        for (int j = 0; j < 4; ++j)
+          if (j < left)
+            bias[j] = (p.flags & GEMM_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + n + j)
+                                                : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n + j]);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane < S) mbar_arrive_cluster(mapa_shared(parts_full, lane));
-      if (lane == 0) mbar_arrive(tempty_bar(acc));
+      ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), acc_phase, abort_word, FT_ERR_TIMEOUT_EPILOGUE));
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * p.bn);
+      for (int r0 = 0; r0 < rows && ok; r0 += ST_PART_ROWS, ++meeting) {
+        const int here = min(ST_PART_ROWS, rows - r0);
+        if (meeting) ok = __all_sync(0xffffffffu, mbar_wait_cluster(parts_free, (meeting ^ 1u) & 1u, abort_word, FT_ERR_TIMEOUT_EPILOGUE));
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = half * 16; c < here; c += 32) {
+          uint32_t r[16];
+          tmem_ld_32x16(t_row + r0 + c, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c + j < here) st_cluster(mine + static_cast<uint32_t>((c + j) * cols) * 4u, r[j]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane < S) mbar_arrive_cluster(mapa_shared(parts_full, lane));
+        if (lane == 0 && r0 + ST_PART_ROWS >= rows) mbar_arrive(tempty_bar(acc));
+        ok = __all_sync(0xffffffffu, mbar_wait_cluster(parts_full, meeting & 1u, abort_word, FT_ERR_TIMEOUT_EPILOGUE));
+        if (!ok) break;
+        // a thread adds four columns of every so many rows
+        if (left > 0)
+          for (int m = mr; m < here; m += m_step) {
+            const float* src = all + m * cols + mc;
+            float4 sum = *reinterpret_cast<const float4*>(src);
+#pragma unroll 4
+            for (int s = 1; s < S; ++s) {
+              const float4 v = *reinterpret_cast<const float4*>(src + s * ST_PART_ROWS * cols);
+              sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+            }
+            stream_finish(p, m0 + r0 + m, n, left, bias, sum);
+          }
+        __syncwarp();
+        if (lane < S) mbar_arrive_cluster(mapa_shared(parts_free, lane));
+      }
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
-      if (!mbar_wait_cluster(parts_full, tile_phase, abort_word, FT_ERR_TIMEOUT_EPILOGUE)) break;
-      // a thread adds four columns of every so many rows
-      const int n = tile * ST_BM + rank * cols + mc, left = p.N - n;
-      if (left > 0) {
-        float bias[4] = {0.f, 0.f, 0.f, 0.f};
-        if (p.flags & (GEMM_BIAS | GEMM_BIAS_F32)) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (j < left)
-              bias[j] = (p.flags & GEMM_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + n + j)
-                                                  : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n + j]);
-        }
-        for (int m = mr; m < p.M; m += m_step) {
-          const float* src = all + m * cols + mc;
-          float4 sum = *reinterpret_cast<const float4*>(src);
-#pragma unroll 4
-          for (int s = 1; s < S; ++s) {
-            const float4 v = *reinterpret_cast<const float4*>(src + s * p.bn * cols);
-            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-          }
-          stream_finish(p, m, n, left, bias, sum);
-        }
-      }
-      __syncwarp();
-      if (lane < S) mbar_arrive_cluster(mapa_shared(parts_free, lane));
     }
   }
 
@@ -285,12 +296,13 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
 static int launch_stream(const void* X, const void* W, StreamParams p, int K, long long ldx, long long ldw, int device, cudaStream_t stream) {
   static int max_clusters[64][4] = {};    // clusters of 1, 2, 4, 8 CTAs that are resident at a time (148, 74, 33, 15)
-  p.bn = (p.M + 15) / 16 * 16;
-  const int parts_bytes = ST_BM * p.bn * 4;
-  p.stages = (ST_BUF_BYTES - parts_bytes) / (ST_A_BYTES + p.bn * ST_BK * 2);
+  p.m_tiles = (p.M + ST_MAX_ROWS - 1) / ST_MAX_ROWS;
+  p.bn = ((p.M + p.m_tiles - 1) / p.m_tiles + 15) / 16 * 16;
+  p.m_tiles = (p.M + p.bn - 1) / p.bn;
+  p.stages = (ST_BUF_BYTES - ST_PARTS_BYTES) / (ST_A_BYTES + p.bn * ST_BK * 2);
   if (p.stages > ST_MAX_STAGES) p.stages = ST_MAX_STAGES;
   p.k_blocks = (K + ST_BK - 1) / ST_BK;
-  p.tiles = (p.N + ST_BM - 1) / ST_BM;
+  p.tiles = (p.N + ST_BM - 1) / ST_BM * p.m_tiles;
   p.status = device_status_word(device);
   cudaLaunchAttribute attr[2] = {};
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -333,26 +345,33 @@ static bool aligned(const void* p, int bytes) { return (reinterpret_cast<uintptr
 
 }  // namespace ft
 
-// C[M, N] = act(X[M, K] W[N, K]^T (+ bias[N]) (+ residual[M, N])) for a small batch M <= 128 (decode), all bf16, K-major, strides in
-// elements.  workspace and ksplit are not needed any more; a residual with ksplit 1 stays refused.
-FT_API int ft_gemm_small_m(const void* X, const void* W, void* C, const void* bias, const void* residual,
-                           float* workspace, int M, int N, int K, long long ldx, long long ldw, long long ldc,
-                           long long ldr, int flags, int ksplit, int device, cudaStream_t stream) {
+// C[M, N] = act(X[M, K] W[N, K]^T (+ bias[N]) (+ residual[M, N])), all bf16, K-major, strides in elements; any number of rows.
+FT_API int ft_gemm_stream(const void* X, const void* W, void* C, const void* bias, const void* residual, int M, int N, int K,
+                          long long ldx, long long ldw, long long ldc, long long ldr, int flags, int device, cudaStream_t stream) {
   if (int _rc = ft::ensure_device(device)) return _rc;
   using namespace ft;
-  (void)workspace;
-  FT_REQUIRE(X && W && C, "ft_gemm_small_m: null operand");
-  FT_REQUIRE(M > 0 && M <= ST_MAX_ROWS && N > 0 && K > 0, "ft_gemm_small_m: M=%d must be in 1..128 (N=%d K=%d)", M, N, K);
-  FT_REQUIRE(ldx % 8 == 0 && ldw % 8 == 0 && N % 8 == 0, "ft_gemm_small_m: strides and N must be multiples of 8");
-  FT_REQUIRE(!(flags & (GEMM_OUT_F32 | GEMM_ACCUMULATE)), "ft_gemm_small_m: bf16 output, no accumulation");
-  FT_REQUIRE(!(flags & (GEMM_BIAS | GEMM_BIAS_F32)) || bias, "ft_gemm_small_m: bias flag without bias");
-  FT_REQUIRE(ksplit != 1 || !residual, "ft_gemm_small_m: the residual is added by the split path only");
+  FT_REQUIRE(X && W && C, "ft_gemm_stream: null operand");
+  FT_REQUIRE(M > 0 && N > 0 && K > 0, "ft_gemm_stream: empty problem %dx%dx%d", M, N, K);
+  FT_REQUIRE(ldx % 8 == 0 && ldw % 8 == 0 && N % 8 == 0, "ft_gemm_stream: strides and N must be multiples of 8");
+  FT_REQUIRE(!(flags & (GEMM_OUT_F32 | GEMM_ACCUMULATE)), "ft_gemm_stream: bf16 output, no accumulation");
+  FT_REQUIRE(!(flags & (GEMM_BIAS | GEMM_BIAS_F32)) || bias, "ft_gemm_stream: bias flag without bias");
   StreamParams p{};
   p.C = C; p.bias = bias; p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.M = M; p.N = N; p.flags = flags & 0xFFFF; p.ldc = ldc; p.ldr = ldr;
   p.vec = ldc % 4 == 0 && aligned(C, 8);
   p.vec_r = ldr % 4 == 0 && aligned(residual, 8);
   return launch_stream(X, W, p, K, ldx, ldw, device, stream);
+}
+
+// The same for a small batch M <= 128 (decode).  workspace and ksplit are not needed any more; a residual with ksplit 1 stays refused.
+FT_API int ft_gemm_small_m(const void* X, const void* W, void* C, const void* bias, const void* residual,
+                           float* workspace, int M, int N, int K, long long ldx, long long ldw, long long ldc,
+                           long long ldr, int flags, int ksplit, int device, cudaStream_t stream) {
+  using namespace ft;
+  (void)workspace;
+  FT_REQUIRE(M > 0 && M <= 128 && N > 0 && K > 0, "ft_gemm_small_m: M=%d must be in 1..128 (N=%d K=%d)", M, N, K);
+  FT_REQUIRE(ksplit != 1 || !residual, "ft_gemm_small_m: the residual is added by the split path only");
+  return ft_gemm_stream(X, W, C, bias, residual, M, N, K, ldx, ldw, ldc, ldr, flags, device, stream);
 }
 
 // C[M, N] (fp32) (+)= X[M, K] W[N, K]^T for a small batch M <= 128; with dyt_out also the next layer's dynamic tanh of the new values,
@@ -366,7 +385,7 @@ FT_API int ft_gemm_small_m_f32(const void* X, const void* W, float* C, int accum
   using namespace ft;
   (void)workspace; (void)ksplit;
   FT_REQUIRE(X && W && C, "ft_gemm_small_m_f32: null operand");
-  FT_REQUIRE(M > 0 && M <= ST_MAX_ROWS && N > 0 && K > ST_BK, "ft_gemm_small_m_f32: M=%d must be in 1..128, K=%d above %d (N=%d)", M, K, ST_BK, N);
+  FT_REQUIRE(M > 0 && M <= 128 && N > 0 && K > ST_BK, "ft_gemm_small_m_f32: M=%d must be in 1..128, K=%d above %d (N=%d)", M, K, ST_BK, N);
   FT_REQUIRE(ldx % 8 == 0 && ldw % 8 == 0, "ft_gemm_small_m_f32: strides must be multiples of 8");
   FT_REQUIRE(!dyt_out || (alpha && dyt_w && dyt_b), "ft_gemm_small_m_f32: the fused norm needs its parameters");
   StreamParams p{};

@@ -25,6 +25,7 @@ _ACT_FLAGS = {None: 0, "relu": GEMM_RELU, "gelu": GEMM_GELU, "silu": GEMM_SILU, 
 stats = {"gemm_native": 0, "gemm_library": 0, "gemm_small_m": 0}
 
 _native.register_protos({
+    "ft_gemm_stream": (_native._i, [_native._vp] * 5 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 2 + [_native._vp]),
     "ft_gemm_small_m": (_native._i, [_native._vp] * 6 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 3 + [_native._vp]),
 })
 
@@ -57,8 +58,33 @@ def gemm_small_m(x: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None 
     return out
 
 
+
+def _gemm_stream(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | None, flags: int) -> torch.Tensor:
+    bias_ptr = None
+    if bias is not None:
+        bias = bias.contiguous()
+        flags |= GEMM_BIAS_F32 if bias.dtype == torch.float32 else GEMM_BIAS
+        assert bias.dtype in (torch.float32, torch.bfloat16)
+        bias_ptr = bias.data_ptr()
+    (M, K), N = a.shape, b.shape[0]
+    rc = _native.kernels().ft_gemm_stream(a.data_ptr(), b.data_ptr(), out.data_ptr(), bias_ptr, None, M, N, K, a.stride(0), b.stride(0),
+                                          out.stride(0), 0, flags, _dev(a), _stream())
+    _native.check(rc, "ft_gemm_stream")
+    stats["gemm_native"] += 1
+    return out
+
+
 _NATIVE = True
 _GEMM_CTA_LIMIT = 0
+
+
+def _streams(M: int, N: int, K: int) -> bool:
+    """Whether a product has too few 256-wide tiles for the pair kernel, so that clusters which share a contraction are faster (us, pair /
+    stream kernel; 214 rows: 4096 x 14336 98 / 39, 2048 x 8192 40 / 30, 3072 x 2048 23 / 15, 6144 x 4096 25 / 29, 2048 x 1408 10 / 13;
+    524 rows: 4096 x 14336 141 / 86, 6144 x 4096 45 / 34, 2048 x 2048 18 / 20, 16384 x 2048 39 / 63; 1024 rows: equal or slower)."""
+    if M <= 128:
+        return N >= 1024 and K >= 512
+    return M <= 256 and N <= 4096 and K >= 2048 or M <= 640 and N <= 6144 and K >= 4096
 
 
 def set_gemm_cta_limit(n: int) -> int:
@@ -179,6 +205,9 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = Non
         # decode-sized batch against a large weight: the weight-stationary kernel
         return gemm_small_m(a, b, bias=bias, out=out, activation=activation)
     flags = _ACT_FLAGS[activation]
+    if (128 < M and _streams(M, N, K) and not accumulate and out.dtype == torch.bfloat16 and la[0] == 0
+            and lb[0] == 0 and bn == 0 and max_ctas == 0 and _GEMM_CTA_LIMIT == 0):
+        return _gemm_stream(a, b, out, bias, flags)
     if out.dtype == torch.float32:
         flags |= GEMM_OUT_F32
     if accumulate:

@@ -401,3 +401,21 @@ def test_parity_sweep_on_gpu():
     rows = parity.sweep(None, "cuda")
     bad = [r for r in rows if not r["ok"]]
     assert not bad, bad
+
+
+@pytest.mark.parametrize("M", [129, 192, 255, 256, 257, 400, 640])
+@pytest.mark.parametrize("N,K", [(1032, 2056), (4096, 4104), (3072, 2048)])
+def test_gemm_stream_row_tiles(M, N, K):
+    # one and several row tiles, meetings of 64 rows of which the last is ragged, ragged last tiles of W and of the contraction
+    torch.manual_seed(M + N + K)
+    x, w, bias = _rand(M, K), _rand(N, K) * 0.05, _rand(N)
+    want = x.double() @ w.double().t()
+    bound = 2.0 ** -8 * want.abs() + 0.05 * K ** 0.5 * 2.0 ** -18          # fp32 sums, one rounding to bf16
+    out = torch.full((M + 1, N), 7.0, device=DEV, dtype=torch.bfloat16)
+    y = F._gemm_stream(x, w, out[:M], None, 0)
+    assert bool(((y.double() - want).abs() <= bound).all()) and bool((out[M] == 7).all())
+    assert torch.equal(F.gemm_nt(x, w), y) == F._streams(M, N, K) or not F._streams(M, N, K)
+    want = torch.relu(want + bias.double())
+    got = F._gemm_stream(x, w, torch.empty_like(y), bias, F._ACT_FLAGS["relu"])
+    assert bool(((got.double() - want).abs() <= bound + 2.0 ** -8 * want.abs() + 2.0 ** -18).all())
+    assert _native.device_status(0) == 0
