@@ -16,6 +16,9 @@
 //   now                       13.6 / 14.9     10.9 / 12.2    42.3 / 48.3    23.4 / 26.0    156 / 166        6.0 / 7.4     14.6 / 16.1
 //   weight bytes at 6.65 TB/s  7.6             5.0           35.3           17.7           158              1.3            7.6
 //
+// With a gated weight [2 N, K] (gate rows, then up rows) a tile holds 64 gate rows and the 64 up rows beside them, and the results are
+// act(gate) * up straight from the fp32 sums: the activation needs no pass of its own over rows that were rounded in between.
+//
 //   warp 0: TMA producer   warp 1: MMA issuer   warp 2: tensor memory   warps 4-11: parts and results
 // Every wait is bounded.
 #include "ft_host.h"
@@ -44,6 +47,8 @@ struct StreamParams {
   __nv_bfloat16* dyt_out;
   float dyt_scale;
   int M, N, tiles, m_tiles, k_blocks, cluster, bn, stages, flags, accumulate, vec, vec_r;
+  int n_tile;           // columns of C in a tile: 128, or 64 with a gated weight
+  int glu;              // 0: none; 1 / 2 / 3: silu / relu / gelu (tanh form) of the gate
   long long ldc, ldr, ldd;
   int* status;
 };
@@ -106,6 +111,14 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) {
   asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
+// act(gate) * up, the activations of the SwiGLU kernel (norm_act.cu).
+__device__ __forceinline__ float stream_glu(float g, float u, int kind) {
+  if (kind == 1) return g / (1.f + __expf(-g)) * u;
+  if (kind == 2) return fmaxf(g, 0.f) * u;
+  const float k = 0.7978845608028654f * (g + 0.044715f * g * g * g);
+  return 0.5f * g * (1.f + tanhf(k)) * u;
+}
+
 __global__ void __launch_bounds__(ST_THREADS, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const StreamParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -150,8 +163,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     // behind it
     int left = ST_PREFETCH;
     for (int tile = first; tile < p.tiles && left > 0; tile += step) {
-      const int n0 = p.m_tiles == 1 ? tile * ST_BM : tile / p.m_tiles * ST_BM;
-      for (int kb = kb0; kb < kb1 && left > 0; ++kb, --left) tma_prefetch_l2_2d(&tmW, kb * ST_BK, n0);
+      const int n0 = (p.m_tiles == 1 ? tile : tile / p.m_tiles) * p.n_tile;
+      for (int kb = kb0; kb < kb1 && left > 0; ++kb, --left) {
+        tma_prefetch_l2_2d(&tmW, kb * ST_BK, n0);
+        if (p.glu) tma_prefetch_l2_2d(&tmW, kb * ST_BK, p.N + n0);
+      }
     }
   }
   if (warp == 2) {
@@ -172,13 +188,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       uint32_t phase = 0;
       bool ok = true;
       for (int tile = first; tile < p.tiles && ok; tile += step) {
-        const int wt = p.m_tiles == 1 ? tile : tile / p.m_tiles, n0 = wt * ST_BM, m0 = (tile - wt * p.m_tiles) * p.bn;
+        const int wt = p.m_tiles == 1 ? tile : tile / p.m_tiles, n0 = wt * p.n_tile, m0 = (tile - wt * p.m_tiles) * p.bn;
         for (int kb = kb0; kb < kb1; ++kb) {
           ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER);
           if (!ok) break;
           const uint32_t sW = smem_base + stage * stage_bytes;
           mbar_expect_tx(full_bar(stage), stage_bytes);
           tma_load_2d(sW, &tmW, full_bar(stage), kb * ST_BK, n0);
+          if (p.glu) tma_load_2d(sW + ST_A_BYTES / 2, &tmW, full_bar(stage), kb * ST_BK, p.N + n0);
           tma_load_2d(sW + ST_A_BYTES, &tmX, full_bar(stage), kb * ST_BK, m0);
           if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
@@ -225,15 +242,18 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     const uint32_t parts = smem_base + static_cast<uint32_t>(stages) * stage_bytes;
     // Parts lie as [CTA that sent it][row of X][column]: the lanes of a warp write and read neighbouring words.  (Four rows of a column
     // as one 16-byte store to the peer took three times as long.)
-    const uint32_t mine = mapa_shared(parts, col / cols) + static_cast<uint32_t>(rank * ST_PART_ROWS * cols + col % cols) * 4u;
+    // with a gated weight a CTA adds as many gate columns as up columns, the up columns behind the others
+    const int own = p.n_tile / S, gate_col = p.glu ? col & 63 : col;
+    const int place = gate_col % own + (p.glu && col >= 64 ? own : 0);
+    const uint32_t mine = mapa_shared(parts, gate_col / own) + static_cast<uint32_t>(rank * ST_PART_ROWS * cols + place) * 4u;
     const float* all = reinterpret_cast<const float*>(smem + stages * stage_bytes);
-    const int mc = (threadIdx.x - 128) % (cols / 4) * 4, mr = (threadIdx.x - 128) / (cols / 4), m_step = ST_EPI_WARPS * 32 / (cols / 4);
+    const int mc = (threadIdx.x - 128) % (own / 4) * 4, mr = (threadIdx.x - 128) / (own / 4), m_step = ST_EPI_WARPS * 32 / (own / 4);
     int acc = 0;
     uint32_t acc_phase = 0, meeting = 0;
     bool ok = true;
     for (int tile = first; tile < p.tiles && ok; tile += step) {
       const int wt = p.m_tiles == 1 ? tile : tile / p.m_tiles, m0 = (tile - wt * p.m_tiles) * p.bn, rows = min(p.bn, p.M - m0);
-      const int n = wt * ST_BM + rank * cols + mc, left = p.N - n;
+      const int n = wt * p.n_tile + rank * own + mc, left = p.N - n;
       float bias[4] = {0.f, 0.f, 0.f, 0.f};
       if (p.flags & (GEMM_BIAS | GEMM_BIAS_F32)) {
 #pragma unroll
@@ -274,6 +294,16 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
               const float4 v = *reinterpret_cast<const float4*>(src + s * ST_PART_ROWS * cols);
               sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
             }
+            if (p.glu) {
+              float4 up = *reinterpret_cast<const float4*>(src + own);
+#pragma unroll 4
+              for (int s = 1; s < S; ++s) {
+                const float4 v = *reinterpret_cast<const float4*>(src + own + s * ST_PART_ROWS * cols);
+                up.x += v.x; up.y += v.y; up.z += v.z; up.w += v.w;
+              }
+              sum = make_float4(stream_glu(sum.x, up.x, p.glu), stream_glu(sum.y, up.y, p.glu), stream_glu(sum.z, up.z, p.glu),
+                                stream_glu(sum.w, up.w, p.glu));
+            }
             stream_finish(p, m0 + r0 + m, n, left, bias, sum);
           }
         __syncwarp();
@@ -302,7 +332,8 @@ static int launch_stream(const void* X, const void* W, StreamParams p, int K, lo
   p.stages = (ST_BUF_BYTES - ST_PARTS_BYTES) / (ST_A_BYTES + p.bn * ST_BK * 2);
   if (p.stages > ST_MAX_STAGES) p.stages = ST_MAX_STAGES;
   p.k_blocks = (K + ST_BK - 1) / ST_BK;
-  p.tiles = (p.N + ST_BM - 1) / ST_BM * p.m_tiles;
+  p.n_tile = p.glu ? ST_BM / 2 : ST_BM;
+  p.tiles = (p.N + p.n_tile - 1) / p.n_tile * p.m_tiles;
   p.status = device_status_word(device);
   cudaLaunchAttribute attr[2] = {};
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -332,7 +363,7 @@ static int launch_stream(const void* X, const void* W, StreamParams p, int K, lo
   cfg.gridDim = (p.tiles < max_clusters[device][lg] ? p.tiles : max_clusters[device][lg]) * p.cluster;
   cfg.numAttrs = 2;
   CUtensorMap tmW, tmX;
-  int rc = make_tmap_2d(&tmW, W, 2, K, p.N, ldw * 2, ST_BK, ST_BM, 3);
+  int rc = make_tmap_2d(&tmW, W, 2, K, p.glu ? 2ull * p.N : p.N, ldw * 2, ST_BK, p.n_tile, 3);
   if (rc) return rc;
   rc = make_tmap_2d(&tmX, X, 2, K, p.M, ldx * 2, ST_BK, p.bn, 3);
   if (rc) return rc;
@@ -360,6 +391,20 @@ FT_API int ft_gemm_stream(const void* X, const void* W, void* C, const void* bia
   p.M = M; p.N = N; p.flags = flags & 0xFFFF; p.ldc = ldc; p.ldr = ldr;
   p.vec = ldc % 4 == 0 && aligned(C, 8);
   p.vec_r = ldr % 4 == 0 && aligned(residual, 8);
+  return launch_stream(X, W, p, K, ldx, ldw, device, stream);
+}
+
+// C[M, F] = act(gate) * up of X [M, K] with a gated weight W [2 F, K] (gate rows, then up rows); act: 0 silu, 1 relu, 2 gelu (tanh form).
+FT_API int ft_gemm_stream_glu(const void* X, const void* W, void* C, int M, int F, int K, long long ldx, long long ldw, long long ldc, int act,
+                              int device, cudaStream_t stream) {
+  if (int _rc = ft::ensure_device(device)) return _rc;
+  using namespace ft;
+  FT_REQUIRE(X && W && C, "ft_gemm_stream_glu: null operand");
+  FT_REQUIRE(M > 0 && F > 0 && K > 0 && act >= 0 && act <= 2, "ft_gemm_stream_glu: bad problem %dx%dx%d", M, F, K);
+  FT_REQUIRE(ldx % 8 == 0 && ldw % 8 == 0 && F % 8 == 0, "ft_gemm_stream_glu: strides and F must be multiples of 8");
+  StreamParams p{};
+  p.C = C; p.M = M; p.N = F; p.glu = act + 1; p.ldc = ldc;
+  p.vec = ldc % 4 == 0 && aligned(C, 8);
   return launch_stream(X, W, p, K, ldx, ldw, device, stream);
 }
 

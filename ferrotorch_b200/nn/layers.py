@@ -139,7 +139,11 @@ class SwiGLU(nn.Module):
         self.activation, self.activation_param = activation, activation_param
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return self.down_proj(F.swiglu(self.gate_up_proj(x), self.activation, self.activation_param))
+        up = self.gate_up_proj
+        if type(up) is Linear and up.bias is None and not torch.is_grad_enabled() and not (up._forward_hooks or up._forward_pre_hooks
+                                                                                           or nn.modules.module._has_any_global_hook()):
+            return self.down_proj(F.linear_swiglu(x, up.weight, self.activation, self.activation_param))
+        return self.down_proj(F.swiglu(up(x), self.activation, self.activation_param))
 
 
 class KVCache:

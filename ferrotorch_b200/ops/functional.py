@@ -26,6 +26,7 @@ stats = {"gemm_native": 0, "gemm_library": 0, "gemm_small_m": 0}
 
 _native.register_protos({
     "ft_gemm_stream": (_native._i, [_native._vp] * 5 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 2 + [_native._vp]),
+    "ft_gemm_stream_glu": (_native._i, [_native._vp] * 3 + [_native._i] * 3 + [_native._ll] * 3 + [_native._i] * 2 + [_native._vp]),
     "ft_gemm_small_m": (_native._i, [_native._vp] * 6 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 3 + [_native._vp]),
 })
 
@@ -128,11 +129,16 @@ class _NoContext:
                 torch.autograd.graph.increment_version(t)
 
 
+def _transformed() -> bool:
+    """Whether a function transform, a forward-mode level or a tracer looks at the calls."""
+    return (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
+            or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling())
+
+
 def _apply(fn, *args):
     """``fn.apply(*args)``; without gradients, function transforms, forward-mode levels or tracing the forward by itself (a decoder layer's
     16 us a call for a node that is thrown away)."""
-    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
-            or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling()):
+    if torch.is_grad_enabled() or _transformed():
         return fn.apply(*args)
     return fn.forward(_NoContext(), *args)
 
@@ -602,6 +608,25 @@ def swiglu(gu: torch.Tensor, activation: str = "silu", param: float | None = Non
     if not _NATIVE or not gu.is_cuda or gu.dtype != torch.bfloat16 or (gu.shape[-1] // 2) % 8:
         return ref.swiglu(gu, act)
     return _apply(_SwiGLUFn, gu, act)
+
+
+def linear_swiglu(x: torch.Tensor, w: torch.Tensor, activation: str = "silu", param: float | None = None) -> torch.Tensor:
+    """``act(x Wg^T) * (x Wu^T)`` for a fused ``[gate | up]`` weight ``w [2F, K]``; few rows without gradients run as one kernel that
+    does not round the projections in between."""
+    K, F2 = x.shape[-1], w.shape[0]
+    rows = x.numel() // K if K else 0
+    if (_NATIVE and x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and not torch.is_grad_enabled() and activation in _ACT_ID
+            and 0 < rows and _streams(rows, F2, K) and F2 % 16 == 0 and K % 8 == 0 and w.stride(1) == 1 and w.stride(0) % 8 == 0
+            and _GEMM_CTA_LIMIT == 0 and not _transformed()):
+        x2 = x.reshape(rows, K)
+        if x2.stride(1) == 1 and (rows == 1 or x2.stride(0) >= K) and x2.stride(0) % 8 == 0 and (x2.data_ptr() | w.data_ptr()) % 16 == 0:
+            out = torch.empty((*x.shape[:-1], F2 // 2), device=x.device, dtype=x.dtype)
+            rc = _native.kernels().ft_gemm_stream_glu(x2.data_ptr(), w.data_ptr(), out.data_ptr(), rows, F2 // 2, K, x2.stride(0), w.stride(0),
+                                                      F2 // 2, _ACT_ID[activation], _dev(x), _stream())
+            _native.check(rc, "ft_gemm_stream_glu")
+            stats["gemm_small_m"] += 1
+            return out
+    return swiglu(linear(x, w), activation, param)
 
 
 # --------------------------------------------------------------------------- embedding
