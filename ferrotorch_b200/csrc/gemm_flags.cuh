@@ -25,4 +25,12 @@ __device__ __forceinline__ float apply_act(float v, int flags) {
   return v;
 }
 
+// act(gate) * up, the activations of the SwiGLU kernel (norm_act.cu).  kind: 1 silu, 2 relu, 3 gelu (tanh form).
+__device__ __forceinline__ float glu(float g, float u, int kind) {
+  if (kind == 1) return g / (1.f + __expf(-g)) * u;
+  if (kind == 2) return fmaxf(g, 0.f) * u;
+  const float k = 0.7978845608028654f * (g + 0.044715f * g * g * g);
+  return 0.5f * g * (1.f + tanhf(k)) * u;
+}
+
 }  // namespace ft

@@ -111,14 +111,6 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) {
   asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
-// act(gate) * up, the activations of the SwiGLU kernel (norm_act.cu).
-__device__ __forceinline__ float stream_glu(float g, float u, int kind) {
-  if (kind == 1) return g / (1.f + __expf(-g)) * u;
-  if (kind == 2) return fmaxf(g, 0.f) * u;
-  const float k = 0.7978845608028654f * (g + 0.044715f * g * g * g);
-  return 0.5f * g * (1.f + tanhf(k)) * u;
-}
-
 __global__ void __launch_bounds__(ST_THREADS, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const StreamParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -301,8 +293,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 const float4 v = *reinterpret_cast<const float4*>(src + own + s * ST_PART_ROWS * cols);
                 up.x += v.x; up.y += v.y; up.z += v.z; up.w += v.w;
               }
-              sum = make_float4(stream_glu(sum.x, up.x, p.glu), stream_glu(sum.y, up.y, p.glu), stream_glu(sum.z, up.z, p.glu),
-                                stream_glu(sum.w, up.w, p.glu));
+              sum = make_float4(glu(sum.x, up.x, p.glu), glu(sum.y, up.y, p.glu), glu(sum.z, up.z, p.glu),
+                                glu(sum.w, up.w, p.glu));
             }
             stream_finish(p, m0 + r0 + m, n, left, bias, sum);
           }

@@ -27,6 +27,7 @@ stats = {"gemm_native": 0, "gemm_library": 0, "gemm_small_m": 0}
 _native.register_protos({
     "ft_gemm_stream": (_native._i, [_native._vp] * 5 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 2 + [_native._vp]),
     "ft_gemm_stream_glu": (_native._i, [_native._vp] * 3 + [_native._i] * 3 + [_native._ll] * 3 + [_native._i] * 2 + [_native._vp]),
+    "ft_gemm_glu": (_native._i, [_native._vp] * 3 + [_native._i] * 3 + [_native._ll] * 3 + [_native._i] * 2 + [_native._vp]),
     "ft_gemm_small_m": (_native._i, [_native._vp] * 6 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 3 + [_native._vp]),
 })
 
@@ -611,20 +612,24 @@ def swiglu(gu: torch.Tensor, activation: str = "silu", param: float | None = Non
 
 
 def linear_swiglu(x: torch.Tensor, w: torch.Tensor, activation: str = "silu", param: float | None = None) -> torch.Tensor:
-    """``act(x Wg^T) * (x Wu^T)`` for a fused ``[gate | up]`` weight ``w [2F, K]``; few rows without gradients run as one kernel that
-    does not round the projections in between."""
+    """``act(x Wg^T) * (x Wu^T)`` for a fused ``[gate | up]`` weight ``w [2F, K]``; without gradients one kernel, which does not round the
+    projections in between: few rows on the clusters that share a contraction, more on CTA pairs where their 256 x 128 tiles fill half
+    of the GPU (with fewer the plain product has narrower tiles to choose from)."""
     K, F2 = x.shape[-1], w.shape[0]
     rows = x.numel() // K if K else 0
     if (_NATIVE and x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and not torch.is_grad_enabled() and activation in _ACT_ID
-            and 0 < rows and _streams(rows, F2, K) and F2 % 16 == 0 and K % 8 == 0 and w.stride(1) == 1 and w.stride(0) % 8 == 0
+            and rows > 0 and F2 >= 1024 and K >= 512 and F2 % 16 == 0 and K % 8 == 0 and w.stride(1) == 1
+            and w.stride(0) % 8 == 0 and (rows <= 128 or ((rows + 255) // 256) * ((F2 + 255) // 256) >= 37)
             and _GEMM_CTA_LIMIT == 0 and not _transformed()):
         x2 = x.reshape(rows, K)
         if x2.stride(1) == 1 and (rows == 1 or x2.stride(0) >= K) and x2.stride(0) % 8 == 0 and (x2.data_ptr() | w.data_ptr()) % 16 == 0:
             out = torch.empty((*x.shape[:-1], F2 // 2), device=x.device, dtype=x.dtype)
-            rc = _native.kernels().ft_gemm_stream_glu(x2.data_ptr(), w.data_ptr(), out.data_ptr(), rows, F2 // 2, K, x2.stride(0), w.stride(0),
-                                                      F2 // 2, _ACT_ID[activation], _dev(x), _stream())
-            _native.check(rc, "ft_gemm_stream_glu")
-            stats["gemm_small_m"] += 1
+            lib = _native.kernels()
+            rc = (lib.ft_gemm_stream_glu if rows <= 128 else lib.ft_gemm_glu)(
+                x2.data_ptr(), w.data_ptr(), out.data_ptr(), rows, F2 // 2, K, x2.stride(0), w.stride(0), F2 // 2, _ACT_ID[activation],
+                _dev(x), _stream())
+            _native.check(rc, "linear_swiglu")
+            stats["gemm_small_m" if rows <= 128 else "gemm_native"] += 1
             return out
     return swiglu(linear(x, w), activation, param)
 

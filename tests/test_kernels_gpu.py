@@ -419,3 +419,27 @@ def test_gemm_stream_row_tiles(M, N, K):
     got = F._gemm_stream(x, w, torch.empty_like(y), bias, F._ACT_FLAGS["relu"])
     assert bool(((got.double() - want).abs() <= bound + 2.0 ** -8 * want.abs() + 2.0 ** -18).all())
     assert _native.device_status(0) == 0
+
+
+@pytest.mark.parametrize("M", [1, 16, 65, 128, 129, 257, 600])
+@pytest.mark.parametrize("F_,K", [(512, 512), (1032, 520), (7168, 2048), (5608, 1032)])
+@pytest.mark.parametrize("act", ["silu", "relu", "gelu"])
+def test_linear_swiglu_in_one_kernel(M, F_, K, act):
+    # gate and up rows of a tile, ragged last tiles whose gate rows run into the up rows; clusters up to 128 rows, CTA pairs above
+    if M > 128 and F_ < 4700:
+        pytest.skip("two kernels, which round in between")
+    torch.manual_seed(M + F_ + K)
+    x, w = _rand(M, K), _rand(2 * F_, K) * (2.0 / K ** 0.5)
+    with torch.no_grad():
+        got = F.linear_swiglu(x, w, act)
+        assert torch.equal(F.linear_swiglu(x[None], w, act)[0], got)
+    gu = x.double() @ w.double().t()
+    g, u = gu[:, :F_], gu[:, F_:]
+    want = {"silu": torch.nn.functional.silu, "relu": torch.relu, "gelu": lambda t: torch.nn.functional.gelu(t, approximate="tanh")}[act](g) * u
+    # fp32 projections (error K^0.5 2^-20 of their size), activations to 2^-20, one rounding to bf16
+    bound = 2.0 ** -8 * want.abs() + 2.0 ** -15 * (1 + u.abs()) * (1 + g.abs())
+    assert got.shape == (M, F_) and bool(((got.double() - want).abs() <= bound).all())
+    # with gradients the two kernels run as before
+    xg = x.clone().requires_grad_()
+    F.linear_swiglu(xg, w, act).sum().backward()
+    assert xg.grad is not None and _native.device_status(0) == 0
