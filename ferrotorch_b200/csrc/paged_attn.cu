@@ -432,8 +432,28 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
     const bool has_k = unit * 8 < D, has_v = unit * 8 < Dv;   // this thread's 16-byte column exists
     const uint32_t chunk_off = static_cast<uint32_t>(unit >> 3) * Cfg::CHUNK;
     constexpr int AHEAD = PT_STAGES - 1;
+    const int shift = (block_size & (block_size - 1)) == 0 ? __ffs(block_size) - 1 : -1;
     bool ok = true;
     for (int t = 0; t < n_tiles + AHEAD; ++t) {
+      // Where the tile's 16 rows of this thread lie in the cache, looked up together and ahead of the waits: one at a time between the
+      // copies (which no load may pass), each row cost the latency of its table entry (a decode step of four layers with 64
+      // sequences of 1800 tokens, 32 / 8 heads of 128: 1290 us, 1250 now).
+      unsigned token[16];
+      const bool keys = t < n_tiles && tile_lo + t >= pool_tiles;
+      const int key0 = (key_tile + tile_lo + t) * PT_TILE;
+      if (keys) {
+        int page[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int key = key0 + row0 + 8 * i;
+          page[i] = shift >= 0 ? key >> shift : key / block_size;
+          token[i] = static_cast<unsigned>(key - page[i] * block_size);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) page[i] = (key0 + row0 + 8 * i < len && page[i] < max_blocks) ? bt[page[i]] : 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) token[i] += static_cast<unsigned>(min(max(page[i], 0), num_blocks - 1)) * static_cast<unsigned>(block_size);
+      }
       // First hand over tile t - AHEAD (groups are committed once per iteration, so "at most
       // AHEAD - 1 groups pending" means its copies have landed).  This must come before the
       // wait below: the MMA warp needs tile t - AHEAD + 1 ... to make progress towards freeing
@@ -469,15 +489,10 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
               copy(row, kp, vp, src, there);
             }
           } else {
-            const int key0 = (key_tile + tile_lo + t) * PT_TILE;
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const int row = row0 + 8 * i;
-              const int key = key0 + row;
-              const int page = key / block_size;
-              int blk = (key < len && page < max_blocks) ? bt[page] : 0;
-              blk = min(max(blk, 0), num_blocks - 1);
-              copy(row, k_cache, v_cache, (static_cast<long long>(blk) * block_size + key % block_size) * Hkv + kvh, key < len);
+              copy(row, k_cache, v_cache, static_cast<long long>(token[i]) * Hkv + kvh, key0 + row < len);
             }
           }
         }
