@@ -84,9 +84,9 @@ def _streams(M: int, N: int, K: int) -> bool:
     """Whether a product has too few 256-wide tiles for the pair kernel, so that clusters which share a contraction are faster (us, pair /
     stream kernel; 214 rows: 4096 x 14336 98 / 39, 2048 x 8192 40 / 30, 3072 x 2048 23 / 15, 6144 x 4096 25 / 29, 2048 x 1408 10 / 13;
     524 rows: 4096 x 14336 141 / 86, 6144 x 4096 45 / 34, 2048 x 2048 18 / 20, 16384 x 2048 39 / 63; 1024 rows: equal or slower)."""
-    if M <= 128:
-        return N >= 1024 and K >= 512
-    return M <= 256 and N <= 4096 and K >= 2048 or M <= 640 and N <= 6144 and K >= 4096
+    if N < 1024 or K < 512:
+        return False
+    return M <= 128 or M <= 256 and N <= 4096 and K >= 2048 or M <= 640 and N <= 6144 and K >= 4096
 
 
 def set_gemm_cta_limit(n: int) -> int:
