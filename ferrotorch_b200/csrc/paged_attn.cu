@@ -309,15 +309,17 @@ __global__ void paged_decode_combine_kernel(const float* part_o, const float* pa
 // (padded) 16-wide N dimension of two small MMAs per tile:
 //     S^T[key, head] = K_tile[key, :] . Q[head, :]          (M = 128 keys, N = 16, K = head_dim)
 //     O^T[dim, head] += V_tile^T[dim, key] . P^T[key, head]  (M = head_dim rows, N = 16, K = 128 keys)
-// so the cached K and V rows go from HBM to shared memory with 16-byte cp.async copies (a page of
-// 16 tokens x one head is only 2 KB per 64-wide half, too small a box for TMA to move at
-// bandwidth; four loader warps keep three 64 KB tiles in flight instead) and from there straight
+// so the cached K and V rows go from HBM to shared memory and from there straight
 // into the tensor core: no per-element CUDA-core arithmetic on the cache at all.  The four softmax warps (thread r = key r of the tile) only handle the
 // 128 x G scores: tile maximum over the keys (warp shuffles + one exchange through shared
 // memory), lazy rescale of O^T in tensor memory, P^T as bf16 into a small shared-memory operand.
 //   warp 1: MMA issuer     warp 2: TMEM allocator     warps 4-7: softmax / epilogue
-//   warps 8-11: loaders (block-table lookups, cp.async into the 128-byte-swizzled operand
-//   layout, rows past the context zero-filled; 3-stage ring of {K, V} tiles)
+//   warps 8-11: loaders, 3-stage ring of {K, V} tiles in the 128-byte-swizzled operand layout
+// The rows of a page come as TMA boxes of one head, 64 columns and as many tokens as lie together (2 KB for pages of 16): no copy
+// instruction, no address and no register for each 16 bytes, and all three stages in flight.  cp.async copies stopped at 3.7 TB/s whatever
+// the shape.  The last tile of a sequence, whose rows past the context have to read as zeros whatever the page holds, pooled blocks,
+// head sizes below 64 and pages that are no multiple of eight tokens are copied with cp.async.  A decode step of four layers with 64
+// sequences of 1800 tokens, 32 / 8 heads of 128: 1251 us with cp.async, 1114 now.
 // Partial results use the same (m, l, o) scratch layout as paged_decode_kernel, so the combine
 // pass is shared.  All waits are bounded.
 constexpr int PT_THREADS = 384;
@@ -348,7 +350,8 @@ struct PtCfg {  // HD: width of the K tile (64 or 128)
 // head sizes, multiples of 16.
 template <int HD, int G>
 __global__ void __launch_bounds__(PT_THREADS, 1)
-paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
+paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, int box,
+                       const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
                        const __nv_bfloat16* q, const int* block_table,
                        const int* row_slot, const int* ctx_len, __nv_bfloat16* __restrict__ out,
                        float* __restrict__ part_o, float* __restrict__ part_ml, int Hq, int Hkv, int D, int Dv, int g_real,
@@ -375,7 +378,7 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
   if (threadIdx.x == 0) {
     *abort_word = 0;
     for (int s = 0; s < PT_STAGES; ++s) {
-      mbar_init(bar(KV_FULL + s), PT_LOADERS);   // every loader thread arrives once its copies have landed
+      mbar_init(bar(KV_FULL + s), box ? 1 : PT_LOADERS);   // without boxes every loader thread arrives once its copies have landed
       mbar_init(bar(ST_EMPTY + s), 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -434,26 +437,86 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
     constexpr int AHEAD = PT_STAGES - 1;
     const int shift = (block_size & (block_size - 1)) == 0 ? __ffs(block_size) - 1 : -1;
     bool ok = true;
+    // where the token of a key lies in the cache (pages that are not there: page 0, as everywhere)
+    auto page_of = [&](int key) { return shift >= 0 ? key >> shift : key / block_size; };
+    auto copy = [&](int st, int row, const __nv_bfloat16* k, const __nv_bfloat16* v, long long src, bool there) {
+      const uint32_t sK = sbase + st * Cfg::STAGE_BYTES + chunk_off, sV = sK + Cfg::K_BYTES;
+      const uint32_t dst = static_cast<uint32_t>(row) * 128u + (static_cast<uint32_t>((unit & 7) ^ (row & 7)) << 4);
+      const uint32_t nbytes = there ? 16u : 0u;       // rows past the context are zero-filled
+      if (has_k)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sK + dst),
+                     "l"(k + src * D + unit * 8), "r"(nbytes) : "memory");
+      if (has_v)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sV + dst),
+                     "l"(v + src * Dv + unit * 8), "r"(nbytes) : "memory");
+    };
+    // Where the tile's 16 rows of this thread lie in the cache, looked up together and ahead of the waits: one at a time between the
+    // copies (which no load may pass), each row cost the latency of its table entry (a decode step of four layers with 64
+    // sequences of 1800 tokens, 32 / 8 heads of 128: 1290 us, 1250 then).
+    unsigned token[16];
+    auto look_up = [&](int key0) {
+      int page[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int key = key0 + row0 + 8 * i;
+        page[i] = page_of(key);
+        token[i] = static_cast<unsigned>(key - page[i] * block_size);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) page[i] = (key0 + row0 + 8 * i < len && page[i] < max_blocks) ? bt[page[i]] : 0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) token[i] += static_cast<unsigned>(min(max(page[i], 0), num_blocks - 1)) * static_cast<unsigned>(block_size);
+    };
+    if (box) {
+      const int n_full = min(n_tiles, max(0, len / PT_TILE - key_tile - tile_lo));   // tiles whose rows all lie inside the context
+      if (warp == 8) {
+        const int nb = PT_TILE / box, k_chunks = (D + 63) / 64, copies = nb * (k_chunks + (Dv + 63) / 64);
+        for (int t = 0; t < n_full && ok; ++t) {
+          const int st = t % PT_STAGES;
+          int first_token = 0;                        // of this lane's box
+          if (lane < nb) {
+            const int key = (key_tile + tile_lo + t) * PT_TILE + lane * box, page = page_of(key);
+            const int blk = page < max_blocks ? bt[page] : 0;
+            first_token = min(max(blk, 0), num_blocks - 1) * block_size + key - page * block_size;
+          }
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(ST_EMPTY + st), ((t / PT_STAGES) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER));
+          if (!ok) break;
+          if (lane == 0) mbar_expect_tx(bar(KV_FULL + st), copies / nb * Cfg::CHUNK);
+          __syncwarp();
+          for (int i0 = 0; i0 < copies; i0 += 32) {
+            const int i = i0 + lane, j = i & (nb - 1), c = i / nb;
+            const int token0 = __shfl_sync(0xffffffffu, first_token, j);
+            const uint32_t dst = sbase + st * Cfg::STAGE_BYTES + j * box * 128;
+            if (i < copies) {
+              if (c < k_chunks) tma_load_3d(dst + c * Cfg::CHUNK, &tmK, bar(KV_FULL + st), c * 64, kvh, token0);
+              else tma_load_3d(dst + Cfg::K_BYTES + (c - k_chunks) * Cfg::CHUNK, &tmV, bar(KV_FULL + st), (c - k_chunks) * 64, kvh, token0);
+            }
+          }
+        }
+      }
+      if (n_full < n_tiles) {                         // the ragged last tile
+        const int st = n_full % PT_STAGES, key0 = (key_tile + tile_lo + n_full) * PT_TILE;
+        look_up(key0);
+        if (warp == 8) ok = ok && mbar_wait(bar(ST_EMPTY + st), ((n_full / PT_STAGES) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER);
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          copy(st, row0 + 8 * i, k_cache, v_cache, static_cast<long long>(token[i]) * Hkv + kvh, key0 + row0 + 8 * i < len);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        fence_proxy_async_smem();
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+        if (threadIdx.x == 256 && ok) mbar_arrive(bar(KV_FULL + st));
+      }
+      if (*abort_word && warp == 8) {
+        // give the boxes already asked for a bounded time to land before the shared memory is released
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+      }
+    } else {
     for (int t = 0; t < n_tiles + AHEAD; ++t) {
-      // Where the tile's 16 rows of this thread lie in the cache, looked up together and ahead of the waits: one at a time between the
-      // copies (which no load may pass), each row cost the latency of its table entry (a decode step of four layers with 64
-      // sequences of 1800 tokens, 32 / 8 heads of 128: 1290 us, 1250 now).
-      unsigned token[16];
       const bool keys = t < n_tiles && tile_lo + t >= pool_tiles;
       const int key0 = (key_tile + tile_lo + t) * PT_TILE;
-      if (keys) {
-        int page[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int key = key0 + row0 + 8 * i;
-          page[i] = shift >= 0 ? key >> shift : key / block_size;
-          token[i] = static_cast<unsigned>(key - page[i] * block_size);
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) page[i] = (key0 + row0 + 8 * i < len && page[i] < max_blocks) ? bt[page[i]] : 0;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) token[i] += static_cast<unsigned>(min(max(page[i], 0), num_blocks - 1)) * static_cast<unsigned>(block_size);
-      }
+      if (keys) look_up(key0);
       // First hand over tile t - AHEAD (groups are committed once per iteration, so "at most
       // AHEAD - 1 groups pending" means its copies have landed).  This must come before the
       // wait below: the MMA warp needs tile t - AHEAD + 1 ... to make progress towards freeing
@@ -467,17 +530,6 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
         const int st = t % PT_STAGES;
         ok = mbar_wait(bar(ST_EMPTY + st), ((t / PT_STAGES) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER);
         if (ok) {
-          const uint32_t sK = sbase + st * Cfg::STAGE_BYTES + chunk_off, sV = sK + Cfg::K_BYTES;
-          auto copy = [&](int row, const __nv_bfloat16* k, const __nv_bfloat16* v, long long src, bool there) {
-            const uint32_t dst = static_cast<uint32_t>(row) * 128u + (static_cast<uint32_t>((unit & 7) ^ (row & 7)) << 4);
-            const uint32_t nbytes = there ? 16u : 0u;       // rows past the context are zero-filled
-            if (has_k)
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sK + dst),
-                           "l"(k + src * D + unit * 8), "r"(nbytes) : "memory");
-            if (has_v)
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sV + dst),
-                           "l"(v + src * Dv + unit * 8), "r"(nbytes) : "memory");
-          };
           if (tile_lo + t < pool_tiles) {
             const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(pooled.k);
             const __nv_bfloat16* vp = static_cast<const __nv_bfloat16*>(pooled.v);
@@ -486,13 +538,13 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
               const int row = row0 + 8 * i, block = (tile_lo + t) * PT_TILE + row;
               const bool there = block < n_pool;
               const long long src = there ? pooled.row(block, bt, block_size, max_blocks, num_blocks) * Hkv + kvh : 0;
-              copy(row, kp, vp, src, there);
+              copy(st, row, kp, vp, src, there);
             }
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const int row = row0 + 8 * i;
-              copy(row, k_cache, v_cache, static_cast<long long>(token[i]) * Hkv + kvh, key0 + row < len);
+              copy(st, row, k_cache, v_cache, static_cast<long long>(token[i]) * Hkv + kvh, key0 + row < len);
             }
           }
         }
@@ -500,6 +552,7 @@ paged_decode_tc_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfl
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0 && n_tiles > 0) {
@@ -909,6 +962,18 @@ FT_API int ft_paged_decode(const void* q, const void* k_cache, const void* v_cac
                            ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
   if (tensor_core) {
     int* status = device_status_word(device);
+    // tokens of a box: what a tile and a page have in common, so that a box never crosses a page
+    CUtensorMap tmK{}, tmV{};
+    int box = block_size & -block_size;
+    if (box > PT_TILE) box = PT_TILE;
+    if (box < 8 || pool || D < 64 || Dv < 64 || static_cast<long long>(num_blocks) * block_size >= (1ll << 31)) box = 0;
+    if (box) {
+      const uint64_t tokens = static_cast<uint64_t>(num_blocks) * block_size;
+      int rc = make_tmap_3d(&tmK, k_cache, 2, D, Hkv, tokens, D * 2ull, static_cast<uint64_t>(Hkv) * D * 2, 64, 1, box, 3);
+      if (rc) return rc;
+      rc = make_tmap_3d(&tmV, v_cache, 2, Dv, Hkv, tokens, Dv * 2ull, static_cast<uint64_t>(Hkv) * Dv * 2, 64, 1, box, 3);
+      if (rc) return rc;
+    }
 #define FT_PT_LAUNCH(HH, GG)                                                                                    \
   {                                                                                                             \
     auto kern = paged_decode_tc_kernel<HH, GG>;                                                                 \
@@ -917,7 +982,7 @@ FT_API int ft_paged_decode(const void* q, const void* k_cache, const void* v_cac
       FT_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PtCfg<HH>::SMEM_BYTES)); \
       attr_set[device] = true;                                                                                  \
     }                                                                                                           \
-    FT_CUDA_CHECK(launch_dependent(kern, grid, PT_THREADS, PtCfg<HH>::SMEM_BYTES, stream,                       \
+    FT_CUDA_CHECK(launch_dependent(kern, grid, PT_THREADS, PtCfg<HH>::SMEM_BYTES, stream, tmK, tmV, box,        \
         static_cast<const __nv_bfloat16*>(k_cache), static_cast<const __nv_bfloat16*>(v_cache),                \
         static_cast<const __nv_bfloat16*>(q), block_table, row_slot, ctx_len, static_cast<__nv_bfloat16*>(out), \
         part_o, part_ml, Hq, Hkv, D, Dv, G, ldq, ldo, block_size, max_blocks, num_blocks, sl2, n_splits, range, pooled, slopes, sink, hg, out_scale, status)); \

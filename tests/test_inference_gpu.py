@@ -182,3 +182,29 @@ def test_rotation_into_the_pages_is_rotation_then_append(D, Hq, Hkv):
     for a, b in zip(*results):
         assert torch.equal(a, b)
     assert bool(results[0][1].any()) and not bool(results[0][3].any())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bs,D,Dv", [(16, 128, 128), (8, 128, 64), (24, 96, 128), (48, 112, 80), (256, 64, 128), (20, 128, 128), (16, 48, 64)])
+@pytest.mark.parametrize("splits,window", [(1, 0), (3, 0), (1, 150)])
+def test_paged_decode_reads_nothing_past_the_context(bs, D, Dv, splits, window):
+    # boxes of 8 to 128 tokens and rows that are copied (pages of 20, heads of 48); contexts that end on a tile, one key past it and inside
+    # a page; what the pages hold behind the context is not finite
+    torch.manual_seed(bs + D)
+    Hkv, G, lens = 2, 4, [1, 128, 129, 256, 700, 1031]
+    cache = PagedKVCache(1, Hkv, D, num_blocks=sum((n + bs - 1) // bs for n in lens) + 2, max_seqs=len(lens), max_seq_len=1056, block_size=bs, v_head_dim=Dv)
+    cache.k[0].fill_(float("nan")), cache.v[0].fill_(float("nan"))
+    mgr = PagedAttentionManager(cache)
+    ks, vs = [], []
+    for b, n in enumerate(lens):
+        assert mgr.add_sequence(n) == b
+        ks.append(torch.randn(n, Hkv, D, device="cuda").to(torch.bfloat16)), vs.append(torch.randn(n, Hkv, Dv, device="cuda").to(torch.bfloat16))
+        cache.append(0, ks[b], vs[b], torch.arange(n, device="cuda", dtype=torch.int32), torch.full((n,), b, device="cuda", dtype=torch.int32))
+    q = torch.randn(len(lens), Hkv * G, D, device="cuda").to(torch.bfloat16)
+    out = cache.decode(0, q, torch.tensor(lens, device="cuda", dtype=torch.int32), n_splits=splits, window=window)
+    for b, n in enumerate(lens):
+        k, v = (t[b][max(0, n - window) if window else 0:].float().repeat_interleave(G, 1) for t in (ks, vs))
+        p = torch.softmax(torch.einsum("hd,thd->ht", q[b].float(), k) * D ** -0.5, -1)
+        want = torch.einsum("ht,thd->hd", p, v)
+        # P and the result are rounded to bf16
+        assert bool(((out[b].float() - want).abs() <= 2.0 ** -7 * (1 + want.abs())).all()), "sequence of %d" % n
