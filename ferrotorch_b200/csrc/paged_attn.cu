@@ -314,32 +314,35 @@ __global__ void paged_decode_combine_kernel(const float* part_o, const float* pa
 // 128 x G scores: tile maximum over the keys (warp shuffles + one exchange through shared
 // memory), lazy rescale of O^T in tensor memory, P^T as bf16 into a small shared-memory operand.
 //   warp 1: MMA issuer     warp 2: TMEM allocator     warps 4-7: softmax / epilogue
-//   warps 8-11: loaders, 3-stage ring of {K, V} tiles in the 128-byte-swizzled operand layout
+//   warps 8-11: loaders, ring of tiles (K of a tile, its V, the next K ...) in the 128-byte-swizzled operand layout
 // The rows of a page come as TMA boxes of one head, 64 columns and as many tokens as lie together (2 KB for pages of 16): no copy
-// instruction, no address and no register for each 16 bytes, and all three stages in flight.  cp.async copies stopped at 3.7 TB/s whatever
+// instruction, no address and no register for each 16 bytes.  cp.async copies stopped at 3.7 TB/s whatever
 // the shape.  The last tile of a sequence, whose rows past the context have to read as zeros whatever the page holds, pooled blocks,
 // head sizes below 64 and pages that are no multiple of eight tokens are copied with cp.async.  A decode step of four layers with 64
-// sequences of 1800 tokens, 32 / 8 heads of 128: 1251 us with cp.async, 1114 now.
+// sequences of 1800 tokens, 32 / 8 heads of 128: 1251 us with cp.async, 1114 with boxes, 1020 with two CTAs per SM.
 // Partial results use the same (m, l, o) scratch layout as paged_decode_kernel, so the combine
 // pass is shared.  All waits are bounded.
 constexpr int PT_THREADS = 384;
 constexpr int PT_LOADERS = 128;  // warps 8-11
 constexpr int PT_TILE = 128;   // keys per tile
-constexpr int PT_STAGES = 3;
 constexpr int PT_N = 16;       // MMA N: query heads of the group, zero-padded
 constexpr float PT_RESCALE = 8.f;
 
 constexpr int PT_VD = 128;     // rows of O^T
 
-template <int HD>
+// SLOTS tiles in the ring: six, or three so that two CTAs share an SM and the start of a CTA, its end, and the chain scores - maximum - P -
+// O of a tile run under the other one's loads.  With no more CTAs than SMs the long ring is better (148 CTAs of 8000 keys: 125 us against
+// 153; 512 of 1800: 129 against 105), and groups above four heads need its registers.
+template <int HD, int SLOTS_>
 struct PtCfg {  // HD: width of the K tile (64 or 128)
   static constexpr int K_BYTES = PT_TILE * HD * 2;
   static constexpr int V_BYTES = PT_TILE * PT_VD * 2;
-  static constexpr int STAGE_BYTES = K_BYTES + V_BYTES;
+  static constexpr int SLOT_BYTES = V_BYTES;              // HD <= PT_VD
+  static constexpr int SLOTS = SLOTS_;
   static constexpr int CHUNK = PT_TILE * 128;             // one 64-wide column chunk of a tile
   static constexpr int Q_BYTES = PT_N * HD * 2;           // Q^T operand: 16 rows x key head size
   static constexpr int P_BYTES = PT_N * PT_TILE * 2;      // P^T operand: 16 rows x 128 keys
-  static constexpr int OFF_Q = PT_STAGES * STAGE_BYTES;
+  static constexpr int OFF_Q = SLOTS * SLOT_BYTES;
   static constexpr int OFF_P = OFF_Q + Q_BYTES;           // two buffers
   static constexpr int OFF_RED = OFF_P + 2 * P_BYTES;     // [4 warps][16] floats
   static constexpr int OFF_BAR = OFF_RED + 4 * PT_N * 4;
@@ -348,8 +351,8 @@ struct PtCfg {  // HD: width of the K tile (64 or 128)
 
 // G: query heads of a group, rounded up to 1 / 2 / 4 / 8 / 16 (g_real of them exist).  D, Dv: key and value
 // head sizes, multiples of 16.
-template <int HD, int G>
-__global__ void __launch_bounds__(PT_THREADS, 1)
+template <int HD, int G, int SLOTS>
+__global__ void __launch_bounds__(PT_THREADS, SLOTS == 3 ? 2 : 1)
 paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, int box,
                        const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
                        const __nv_bfloat16* q, const int* block_table,
@@ -358,14 +361,14 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
                        long long ldq, long long ldo, int block_size, int max_blocks, int num_blocks, float scale_log2,
                        int n_splits, KeyRange range, PooledKeys pooled, const float* __restrict__ slopes, const float* __restrict__ sink,
                        HeadGate gate, float out_scale, int* status) {
-  using Cfg = PtCfg<HD>;
+  using Cfg = PtCfg<HD, SLOTS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   const uint32_t sbase = smem_u32(smem);
   const uint32_t sQ = sbase + Cfg::OFF_Q, sP = sbase + Cfg::OFF_P;
   float* s_red = reinterpret_cast<float*>(smem + Cfg::OFF_RED);
-  enum { KV_FULL = 0, ST_EMPTY = KV_FULL + PT_STAGES, S_FULL = ST_EMPTY + PT_STAGES,
+  enum { KV_FULL = 0, ST_EMPTY = KV_FULL + SLOTS, S_FULL = ST_EMPTY + SLOTS,
          P_FULL = S_FULL + 2, O_DONE = P_FULL + 2, NBARS = O_DONE + 1 };
   const uint32_t bar0 = sbase + Cfg::OFF_BAR;
   auto bar = [&](int i) { return bar0 + 8u * i; };
@@ -377,7 +380,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   grid_dependency_launch();
   if (threadIdx.x == 0) {
     *abort_word = 0;
-    for (int s = 0; s < PT_STAGES; ++s) {
+    for (int s = 0; s < SLOTS; ++s) {
       mbar_init(bar(KV_FULL + s), box ? 1 : PT_LOADERS);   // without boxes every loader thread arrives once its copies have landed
       mbar_init(bar(ST_EMPTY + s), 1);
     }
@@ -393,13 +396,9 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     tmem_relinquish();
   }
   // Q^T operand (bf16, rows past the group zero; the scale is applied to the fp32 scores) and zeroed
-  // P^T buffers, written by all threads.  Head sizes below the tile's: the columns that the loaders
-  // never write are zeroed in every stage.
+  // P^T buffers, written by all threads.
   for (int i = threadIdx.x; i < (Cfg::Q_BYTES + 2 * Cfg::P_BYTES) / 16; i += blockDim.x)
     reinterpret_cast<uint4*>(smem + Cfg::OFF_Q)[i] = make_uint4(0u, 0u, 0u, 0u);
-  if (D < HD || Dv < PT_VD)
-    for (int i = threadIdx.x; i < PT_STAGES * Cfg::STAGE_BYTES / 16; i += blockDim.x)
-      reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
   grid_dependency_wait();
   const int len = ctx_len[b];
   const int first = range.first_visible(len);
@@ -427,28 +426,26 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
 
   if (warp >= 8) {
     // ------------------------------------------------------------------ loaders
-    // Thread lt copies 16-byte unit (lt & 15) of rows (lt >> 4) + 8 i, i = 0..15, of the K tile
-    // and of the V tile: 16 consecutive threads read one 256-byte cache row.
+    // Thread lt copies 16-byte unit (lt & 15) of rows (lt >> 4) + 8 i, i = 0..15, of a K or V tile: 16 consecutive threads read one
+    // 256-byte cache row.
     const int lt = threadIdx.x - 256;
     const int unit = lt & 15, row0 = lt >> 4;
     const int* bt = block_table + static_cast<long long>(row_slot ? row_slot[b] : b) * max_blocks;
-    const bool has_k = unit * 8 < D, has_v = unit * 8 < Dv;   // this thread's 16-byte column exists
     const uint32_t chunk_off = static_cast<uint32_t>(unit >> 3) * Cfg::CHUNK;
-    constexpr int AHEAD = PT_STAGES - 1;
+    constexpr int AHEAD = SLOTS - 1;
     const int shift = (block_size & (block_size - 1)) == 0 ? __ffs(block_size) - 1 : -1;
     bool ok = true;
     // where the token of a key lies in the cache (pages that are not there: page 0, as everywhere)
     auto page_of = [&](int key) { return shift >= 0 ? key >> shift : key / block_size; };
-    auto copy = [&](int st, int row, const __nv_bfloat16* k, const __nv_bfloat16* v, long long src, bool there) {
-      const uint32_t sK = sbase + st * Cfg::STAGE_BYTES + chunk_off, sV = sK + Cfg::K_BYTES;
-      const uint32_t dst = static_cast<uint32_t>(row) * 128u + (static_cast<uint32_t>((unit & 7) ^ (row & 7)) << 4);
-      const uint32_t nbytes = there ? 16u : 0u;       // rows past the context are zero-filled
-      if (has_k)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sK + dst),
-                     "l"(k + src * D + unit * 8), "r"(nbytes) : "memory");
-      if (has_v)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sV + dst),
-                     "l"(v + src * Dv + unit * 8), "r"(nbytes) : "memory");
+    // rows past the context and columns past the head size are zero-filled
+    auto copy = [&](int h, int row, const __nv_bfloat16* from, long long src, bool there) {
+      const int size = h & 1 ? Dv : D;
+      if (unit * 8 >= (h & 1 ? PT_VD : HD)) return;
+      const bool has = unit * 8 < size;
+      const uint32_t dst = sbase + h % SLOTS * Cfg::SLOT_BYTES + chunk_off + static_cast<uint32_t>(row) * 128u +
+                           (static_cast<uint32_t>((unit & 7) ^ (row & 7)) << 4);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(from + src * size + (has ? unit * 8 : 0)),
+                   "r"(there && has ? 16u : 0u) : "memory");
     };
     // Where the tile's 16 rows of this thread lie in the cache, looked up together and ahead of the waits: one at a time between the
     // copies (which no load may pass), each row cost the latency of its table entry (a decode step of four layers with 64
@@ -470,42 +467,41 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     if (box) {
       const int n_full = min(n_tiles, max(0, len / PT_TILE - key_tile - tile_lo));   // tiles whose rows all lie inside the context
       if (warp == 8) {
-        const int nb = PT_TILE / box, k_chunks = (D + 63) / 64, copies = nb * (k_chunks + (Dv + 63) / 64);
-        for (int t = 0; t < n_full && ok; ++t) {
-          const int st = t % PT_STAGES;
-          int first_token = 0;                        // of this lane's box
-          if (lane < nb) {
-            const int key = (key_tile + tile_lo + t) * PT_TILE + lane * box, page = page_of(key);
+        const int nb = PT_TILE / box;
+        int first_token = 0;                          // of this lane's box
+        for (int h = 0; h < 2 * n_full; ++h) {
+          const int st = h % SLOTS, copies = nb * (((h & 1 ? Dv : D) + 63) / 64);
+          if (!(h & 1) && lane < nb) {
+            const int key = (key_tile + tile_lo + (h >> 1)) * PT_TILE + lane * box, page = page_of(key);
             const int blk = page < max_blocks ? bt[page] : 0;
             first_token = min(max(blk, 0), num_blocks - 1) * block_size + key - page * block_size;
           }
-          ok = __all_sync(0xffffffffu, mbar_wait(bar(ST_EMPTY + st), ((t / PT_STAGES) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER));
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(ST_EMPTY + st), ((h / SLOTS) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER));
           if (!ok) break;
           if (lane == 0) mbar_expect_tx(bar(KV_FULL + st), copies / nb * Cfg::CHUNK);
           __syncwarp();
           for (int i0 = 0; i0 < copies; i0 += 32) {
             const int i = i0 + lane, j = i & (nb - 1), c = i / nb;
             const int token0 = __shfl_sync(0xffffffffu, first_token, j);
-            const uint32_t dst = sbase + st * Cfg::STAGE_BYTES + j * box * 128;
-            if (i < copies) {
-              if (c < k_chunks) tma_load_3d(dst + c * Cfg::CHUNK, &tmK, bar(KV_FULL + st), c * 64, kvh, token0);
-              else tma_load_3d(dst + Cfg::K_BYTES + (c - k_chunks) * Cfg::CHUNK, &tmV, bar(KV_FULL + st), (c - k_chunks) * 64, kvh, token0);
-            }
+            if (i < copies) tma_load_3d(sbase + st * Cfg::SLOT_BYTES + c * Cfg::CHUNK + j * box * 128, h & 1 ? &tmV : &tmK, bar(KV_FULL + st), c * 64, kvh, token0);
           }
         }
       }
       if (n_full < n_tiles) {                         // the ragged last tile
-        const int st = n_full % PT_STAGES, key0 = (key_tile + tile_lo + n_full) * PT_TILE;
+        const int key0 = (key_tile + tile_lo + n_full) * PT_TILE;
         look_up(key0);
-        if (warp == 8) ok = ok && mbar_wait(bar(ST_EMPTY + st), ((n_full / PT_STAGES) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER);
-        asm volatile("bar.sync 2, 128;" ::: "memory");
+        for (int h = 2 * n_full; h < 2 * n_full + 2; ++h) {
+          const int st = h % SLOTS;
+          if (warp == 8) ok = ok && mbar_wait(bar(ST_EMPTY + st), ((h / SLOTS) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER);
+          asm volatile("bar.sync 2, 128;" ::: "memory");
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          copy(st, row0 + 8 * i, k_cache, v_cache, static_cast<long long>(token[i]) * Hkv + kvh, key0 + row0 + 8 * i < len);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        fence_proxy_async_smem();
-        asm volatile("bar.sync 2, 128;" ::: "memory");
-        if (threadIdx.x == 256 && ok) mbar_arrive(bar(KV_FULL + st));
+          for (int i = 0; i < 16; ++i)
+            copy(h, row0 + 8 * i, h & 1 ? v_cache : k_cache, static_cast<long long>(token[i]) * Hkv + kvh, key0 + row0 + 8 * i < len);
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          fence_proxy_async_smem();
+          asm volatile("bar.sync 2, 128;" ::: "memory");
+          if (threadIdx.x == 256 && ok) mbar_arrive(bar(KV_FULL + st));
+        }
       }
       if (*abort_word && warp == 8) {
         // give the boxes already asked for a bounded time to land before the shared memory is released
@@ -513,45 +509,35 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
         while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
       }
     } else {
-    for (int t = 0; t < n_tiles + AHEAD; ++t) {
-      const bool keys = t < n_tiles && tile_lo + t >= pool_tiles;
-      const int key0 = (key_tile + tile_lo + t) * PT_TILE;
-      if (keys) look_up(key0);
-      // First hand over tile t - AHEAD (groups are committed once per iteration, so "at most
-      // AHEAD - 1 groups pending" means its copies have landed).  This must come before the
-      // wait below: the MMA warp needs tile t - AHEAD + 1 ... to make progress towards freeing
-      // the stage this iteration is about to wait for.
-      if (t >= AHEAD) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD - 1) : "memory");
-        fence_proxy_async_smem();
-        if (ok) mbar_arrive(bar(KV_FULL + (t - AHEAD) % PT_STAGES));
-      }
-      if (t < n_tiles && ok) {
-        const int st = t % PT_STAGES;
-        ok = mbar_wait(bar(ST_EMPTY + st), ((t / PT_STAGES) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER);
-        if (ok) {
-          if (tile_lo + t < pool_tiles) {
-            const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(pooled.k);
-            const __nv_bfloat16* vp = static_cast<const __nv_bfloat16*>(pooled.v);
+      for (int h = 0; h < 2 * n_tiles + AHEAD; ++h) {
+        const int t = h >> 1, key0 = (key_tile + tile_lo + t) * PT_TILE;
+        if (!(h & 1) && t < n_tiles && tile_lo + t >= pool_tiles) look_up(key0);
+        // First hand over tile h - AHEAD (groups are committed once per iteration, so "at most AHEAD - 1 groups pending" means its copies
+        // have landed).  This must come before the wait below: V of a tile is given back only after the next tile's K has been multiplied.
+        if (h >= AHEAD) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD - 1) : "memory");
+          fence_proxy_async_smem();
+          if (ok) mbar_arrive(bar(KV_FULL + (h - AHEAD) % SLOTS));
+        }
+        if (h < 2 * n_tiles && ok) {
+          ok = mbar_wait(bar(ST_EMPTY + h % SLOTS), ((h / SLOTS) & 1) ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER);
+          if (ok && tile_lo + t < pool_tiles) {
+            const __nv_bfloat16* pool = static_cast<const __nv_bfloat16*>(h & 1 ? pooled.v : pooled.k);
 #pragma unroll 4
             for (int i = 0; i < 16; ++i) {
               const int row = row0 + 8 * i, block = (tile_lo + t) * PT_TILE + row;
               const bool there = block < n_pool;
-              const long long src = there ? pooled.row(block, bt, block_size, max_blocks, num_blocks) * Hkv + kvh : 0;
-              copy(st, row, kp, vp, src, there);
+              copy(h, row, pool, there ? pooled.row(block, bt, block_size, max_blocks, num_blocks) * Hkv + kvh : 0, there);
             }
-          } else {
+          } else if (ok) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const int row = row0 + 8 * i;
-              copy(st, row, k_cache, v_cache, static_cast<long long>(token[i]) * Hkv + kvh, key0 + row < len);
-            }
+            for (int i = 0; i < 16; ++i)
+              copy(h, row0 + 8 * i, h & 1 ? v_cache : k_cache, static_cast<long long>(token[i]) * Hkv + kvh, key0 + row0 + 8 * i < len);
           }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+      asm volatile("cp.async.wait_all;" ::: "memory");
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
@@ -559,7 +545,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       constexpr uint32_t idesc_qk = make_idesc_f16(PT_TILE, PT_N, 1, 0, 0);   // keys x heads, both K-major
       constexpr uint32_t idesc_pv = make_idesc_f16(PT_VD, PT_N, 1, 1, 0);     // dims x heads, A (V^T) MN-major
       auto issue_qk = [&](int t) {
-        const uint32_t sK = sbase + (t % PT_STAGES) * Cfg::STAGE_BYTES;
+        const uint32_t sK = sbase + (2 * t % SLOTS) * Cfg::SLOT_BYTES;
         const uint32_t d = tmem_base + COL_S + (t & 1) * PT_N;
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
@@ -569,6 +555,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
                       idesc_qk, kk > 0 ? 1u : 0u);
         }
         umma_commit(bar(S_FULL + (t & 1)));
+        umma_commit(bar(ST_EMPTY + 2 * t % SLOTS));
       };
       bool ok = mbar_wait(bar(KV_FULL + 0), 0, abort_word, FT_ERR_TIMEOUT_MMA);
       if (ok) {
@@ -578,16 +565,17 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       for (int t = 0; t < n_tiles && ok; ++t) {
         if (t + 1 < n_tiles) {
           // S buffer (t+1)&1 was last read by the softmax of tile t-1, which has arrived on P_FULL
-          ok = mbar_wait(bar(KV_FULL + (t + 1) % PT_STAGES), ((t + 1) / PT_STAGES) & 1, abort_word, FT_ERR_TIMEOUT_MMA);
+          ok = mbar_wait(bar(KV_FULL + (2 * t + 2) % SLOTS), ((2 * t + 2) / SLOTS) & 1, abort_word, FT_ERR_TIMEOUT_MMA);
           if (!ok) break;
           tc_fence_after();
           issue_qk(t + 1);
         }
-        const int st = t % PT_STAGES;
-        ok = mbar_wait(bar(P_FULL + (t & 1)), (t >> 1) & 1, abort_word, FT_ERR_TIMEOUT_MMA);
+        const int st = (2 * t + 1) % SLOTS;
+        ok = mbar_wait(bar(KV_FULL + st), ((2 * t + 1) / SLOTS) & 1, abort_word, FT_ERR_TIMEOUT_MMA) &&
+             mbar_wait(bar(P_FULL + (t & 1)), (t >> 1) & 1, abort_word, FT_ERR_TIMEOUT_MMA);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t sV = sbase + st * Cfg::STAGE_BYTES + Cfg::K_BYTES;
+        const uint32_t sV = sbase + st * Cfg::SLOT_BYTES;
         const uint32_t pb = sP + (t & 1) * Cfg::P_BYTES;
 #pragma unroll
         for (int kk = 0; kk < PT_TILE / 16; ++kk) {
@@ -966,7 +954,7 @@ FT_API int ft_paged_decode(const void* q, const void* k_cache, const void* v_cac
     CUtensorMap tmK{}, tmV{};
     int box = block_size & -block_size;
     if (box > PT_TILE) box = PT_TILE;
-    if (box < 8 || pool || D < 64 || Dv < 64 || static_cast<long long>(num_blocks) * block_size >= (1ll << 31)) box = 0;
+    if (box < 8 || pool || D < 64 || Dv <= 64 || static_cast<long long>(num_blocks) * block_size >= (1ll << 31)) box = 0;
     if (box) {
       const uint64_t tokens = static_cast<uint64_t>(num_blocks) * block_size;
       int rc = make_tmap_3d(&tmK, k_cache, 2, D, Hkv, tokens, D * 2ull, static_cast<uint64_t>(Hkv) * D * 2, 64, 1, box, 3);
@@ -974,27 +962,30 @@ FT_API int ft_paged_decode(const void* q, const void* k_cache, const void* v_cac
       rc = make_tmap_3d(&tmV, v_cache, 2, Dv, Hkv, tokens, Dv * 2ull, static_cast<uint64_t>(Hkv) * Dv * 2, 64, 1, box, 3);
       if (rc) return rc;
     }
-#define FT_PT_LAUNCH(HH, GG)                                                                                    \
+#define FT_PT_LAUNCH(HH, GG, SS)                                                                                 \
   {                                                                                                             \
-    auto kern = paged_decode_tc_kernel<HH, GG>;                                                                 \
+    auto kern = paged_decode_tc_kernel<HH, GG, SS>;                                                             \
     static bool attr_set[64] = {false};                                                                         \
     if (!attr_set[device]) {                                                                                    \
-      FT_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PtCfg<HH>::SMEM_BYTES)); \
+      FT_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PtCfg<HH, SS>::SMEM_BYTES)); \
       attr_set[device] = true;                                                                                  \
     }                                                                                                           \
-    FT_CUDA_CHECK(launch_dependent(kern, grid, PT_THREADS, PtCfg<HH>::SMEM_BYTES, stream, tmK, tmV, box,        \
+    FT_CUDA_CHECK(launch_dependent(kern, grid, PT_THREADS, PtCfg<HH, SS>::SMEM_BYTES, stream, tmK, tmV, box,        \
         static_cast<const __nv_bfloat16*>(k_cache), static_cast<const __nv_bfloat16*>(v_cache),                \
         static_cast<const __nv_bfloat16*>(q), block_table, row_slot, ctx_len, static_cast<__nv_bfloat16*>(out), \
         part_o, part_ml, Hq, Hkv, D, Dv, G, ldq, ldo, block_size, max_blocks, num_blocks, sl2, n_splits, range, pooled, slopes, sink, hg, out_scale, status)); \
   }
+#define FT_PT_BY_SLOTS(HH, GG) { if (two) FT_PT_LAUNCH(HH, GG, 3) else FT_PT_LAUNCH(HH, GG, 6) }
 #define FT_PT_BY_G(HH)                     \
-  if (G == 1) FT_PT_LAUNCH(HH, 1)          \
-  else if (G == 2) FT_PT_LAUNCH(HH, 2)     \
-  else if (G <= 4) FT_PT_LAUNCH(HH, 4)     \
-  else if (G <= 8) FT_PT_LAUNCH(HH, 8)     \
-  else FT_PT_LAUNCH(HH, 16)
+  if (G == 1) FT_PT_BY_SLOTS(HH, 1)        \
+  else if (G == 2) FT_PT_BY_SLOTS(HH, 2)   \
+  else if (G <= 4) FT_PT_BY_SLOTS(HH, 4)   \
+  else if (G <= 8) FT_PT_LAUNCH(HH, 8, 6)  \
+  else FT_PT_LAUNCH(HH, 16, 6)
+    const bool two = static_cast<long long>(n_splits) * Hkv * B > sm_count(device);
     if (D > 64) { FT_PT_BY_G(128) } else { FT_PT_BY_G(64) }
 #undef FT_PT_BY_G
+#undef FT_PT_BY_SLOTS
 #undef FT_PT_LAUNCH
   } else {
     FT_REQUIRE(pool == 0, "ft_paged_decode: blocks of keys need head sizes that are multiples of 16 up to 128, 16-byte aligned rows");
