@@ -301,6 +301,10 @@ __device__ __forceinline__ void cluster_sync_all() {
   cluster_arrive();
   cluster_wait();
 }
+// A word to the shared memory of a CTA of the cluster (address from mapa_shared).
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 // Arrive on an mbarrier that lives in another CTA of the cluster (address from mapa_shared).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar)

@@ -107,10 +107,6 @@ __device__ __forceinline__ void stream_finish(const StreamParams& p, int m, int 
   }
 }
 
-__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-
 __global__ void __launch_bounds__(ST_THREADS, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const StreamParams p) {
   extern __shared__ uint8_t smem_raw[];

@@ -5,7 +5,7 @@
 // src/gpu_gguf.rs:14-27).  Here the raw blocks are uploaded once (0.56 - 1.06 bytes per element) and
 // expanded in place on the device to the dtype the model runs in; the arithmetic is the header
 // shared with the host reader (gguf_blocks.h), so host and device agree bit for bit in fp32.
-// Q4_0 matrices that feed a linear layer need not be expanded at all (quant_gemm.cu).
+// Q4_0 matrices that feed a linear layer need not be expanded at all (q4_gemm.cu).
 //
 // One thread decodes the element pair (i, i + 16) of a block; 16 consecutive threads share a block.
 #include <cuda_bf16.h>

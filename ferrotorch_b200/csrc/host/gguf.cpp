@@ -2,7 +2,7 @@
 // block formats the reference supports (Q4_0, Q4_1, Q5_0, Q5_1, Q8_0, Q8_1, F16, BF16, F32 --
 // ferrotorch-serialize/src/gguf.rs:56-927; block = 32 elements, Q4_0 = fp16 scale + 16 nibble
 // bytes) and re-lay Q4_0 weights out for the fused dequant-GEMM kernel (separate scale and nibble
-// planes, csrc/quant_gemm.cu).
+// planes, csrc/q4_gemm.cu).
 //
 // Element order inside a block.  The GGML file format (what llama.cpp writes) puts element j in
 // the low nibble of byte j and element j + 16 in the high nibble, and bit j / bit j + 16 of the

@@ -1,20 +1,8 @@
-// GEMMs whose weight operand is expanded on the fly inside the tcgen05 main loop (sm_100a):
-//
-//   mode Q4_0   Y[M,N] = X[M,K] * dequant(Wq)[N,K]^T, GGUF Q4_0 weights (32-element blocks, fp16
-//               scale + 16 nibble bytes, value = (q - 8) * d; element j = low nibble of byte j,
-//               element j+16 = high nibble, the GGML file format's order.  The reference's decoder
-//               emits the nibbles of byte j as elements 2j, 2j+1 instead, ferrotorch-serialize/src/
-//               gguf.rs:543-577; data in that convention is re-packed on the host,
-//               csrc/host/gguf.cpp ftg_repack_nibbles).  The
-//               reference dequantises the whole tensor to f32 on the GPU, bounces it through the
-//               host and stores bf16 (ferrotorch-llama/src/gpu_gguf.rs:14-27); it has no fused
-//               dequant-GEMM.  Here the weights stay 4-bit in HBM (0.5625 bytes / element).
-//   mode SP24   Y = X * W^T with W in 2:4 semi-structured form: per group of 4 consecutive K
-//               elements two kept values (bf16) and two 2-bit positions (one metadata nibble per
-//               group).  The reference calls cuSPARSELt (ferrotorch-gpu/src/cusparselt.rs:547-932);
-//               this kernel keeps the compressed form in HBM (0.5625 bytes / element-slot) and
-//               expands tiles in the producer, so memory-bound shapes gain the bandwidth while the
-//               math runs as dense MMAs.
+// GEMM whose 2:4-sparse weight operand is expanded on the fly inside the tcgen05 main loop (sm_100a):  Y = X * W^T with W in 2:4
+// semi-structured form: per group of 4 consecutive K elements two kept values (bf16) and two 2-bit positions (one metadata nibble per
+// group).  The reference calls cuSPARSELt (ferrotorch-gpu/src/cusparselt.rs:547-932); this kernel keeps the compressed form in HBM
+// (0.5625 bytes / element-slot) and expands tiles in the producer, so memory-bound shapes gain the bandwidth while the math runs as
+// dense MMAs.  (Q4_0 weights: q4_gemm.cu.)
 //
 // Structure = the dense GEMM (gemm_tcgen05.cu) with the B-side TMA load replaced by eight
 // "expander" warps in two groups that alternate k-blocks: a thread owns row r of the 128 x 64 B
@@ -42,11 +30,10 @@ constexpr int QG_BAR_OFF = QG_COMP_OFF + 2 * QG_COMP_SLOT;
 constexpr int QG_SMEM = QG_BAR_OFF + 1024 + 256;
 
 struct QgParams {
-  int mode;  // 0 = Q4_0, 1 = SP24
   void* C; long long ldc; int out_f32;
   const void* bias;
   int M, N, K;
-  // Q4_0: nibbles [N, K/2] u8, scales [N, K/32] fp16.  SP24: values [N, K/2] bf16, meta [N, K/8] u8
+  // values [N, K/2] bf16, meta [N, K/8] u8
   const uint8_t* w0;
   const uint8_t* w1;
   int* status;
@@ -59,67 +46,39 @@ __device__ __forceinline__ void store_row_unit(uint32_t row_base, int r, int u, 
 
 // Expand one 64-wide k-block of row r (compressed bytes in q0..q3 / aux0, aux1) into the 128-byte
 // row of the swizzled K-major B tile at row_base.
-template <int MODE>
 __device__ __forceinline__ void expand_row(uint32_t row_base, int r, const uint4& q0, const uint4& q1, const uint4& q2,
                                            const uint4& q3, uint32_t aux0, uint32_t aux1) {
-  if (MODE == 0) {
-    const uint32_t nib[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+  // 16 groups of 4 slots; group g: two bf16 values (one word) at slots (m & 3), (m >> 2)
+  const uint32_t vals[16] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w,
+                             q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z, q3.w};
 #pragma unroll
-    for (int blk = 0; blk < 2; ++blk) {
-      const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(blk ? (aux0 >> 16) : (aux0 & 0xFFFF))));
+  for (int u = 0; u < 8; ++u) {        // one 16-byte unit = 8 slots = 2 groups
+    uint32_t outw[4];
 #pragma unroll
-      for (int hi = 0; hi < 2; ++hi) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          // 8 elements: nibbles (low or high) of bytes [half*8, half*8+8) of this block
-          const uint32_t w0 = nib[blk * 4 + half * 2] >> (hi * 4), w1 = nib[blk * 4 + half * 2 + 1] >> (hi * 4);
-          float f[8];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            // 0x4B000000 | q is the float 2^23 + q: the nibble becomes a float without an I2F
-            f[e] = (__uint_as_float(((w0 >> (8 * e)) & 0xFu) | 0x4B000000u) - 8388616.f) * d;
-            f[4 + e] = (__uint_as_float(((w1 >> (8 * e)) & 0xFu) | 0x4B000000u) - 8388616.f) * d;
-          }
-          uint4 o;
-          o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
-          o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
-          store_row_unit(row_base, r, blk * 4 + hi * 2 + half, o);
-        }
-      }
+    for (int gg = 0; gg < 2; ++gg) {
+      const int g = u * 2 + gg;
+      const uint32_t m4 = ((g < 8 ? aux0 : aux1) >> ((g & 7) * 4)) & 0xF;
+      const uint32_t v_lo = vals[g] & 0xFFFFu, v_hi = vals[g] >> 16;
+      const uint32_t p0 = m4 & 3u, p1 = m4 >> 2;
+      // slot s of the group lives in half-word (s & 1) of word (s >> 1): build both words
+      // with selects instead of indexing a register array by a run-time value
+      outw[gg * 2] = (p0 == 0u ? v_lo : 0u) | (p0 == 1u ? v_lo << 16 : 0u) | (p1 == 1u ? v_hi << 16 : 0u);
+      outw[gg * 2 + 1] = (p0 == 2u ? v_lo : 0u) | (p1 == 2u ? v_hi : 0u) | (p1 == 3u ? v_hi << 16 : 0u);
     }
-  } else {
-    // 16 groups of 4 slots; group g: two bf16 values (one word) at slots (m & 3), (m >> 2)
-    const uint32_t vals[16] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w,
-                               q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z, q3.w};
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {        // one 16-byte unit = 8 slots = 2 groups
-      uint32_t outw[4];
-#pragma unroll
-      for (int gg = 0; gg < 2; ++gg) {
-        const int g = u * 2 + gg;
-        const uint32_t m4 = ((g < 8 ? aux0 : aux1) >> ((g & 7) * 4)) & 0xF;
-        const uint32_t v_lo = vals[g] & 0xFFFFu, v_hi = vals[g] >> 16;
-        const uint32_t p0 = m4 & 3u, p1 = m4 >> 2;
-        // slot s of the group lives in half-word (s & 1) of word (s >> 1): build both words
-        // with selects instead of indexing a register array by a run-time value
-        outw[gg * 2] = (p0 == 0u ? v_lo : 0u) | (p0 == 1u ? v_lo << 16 : 0u) | (p1 == 1u ? v_hi << 16 : 0u);
-        outw[gg * 2 + 1] = (p0 == 2u ? v_lo : 0u) | (p1 == 2u ? v_hi : 0u) | (p1 == 3u ? v_hi << 16 : 0u);
-      }
-      store_row_unit(row_base, r, u, make_uint4(outw[0], outw[1], outw[2], outw[3]));
-    }
+    store_row_unit(row_base, r, u, make_uint4(outw[0], outw[1], outw[2], outw[3]));
   }
 }
 
-// MODE: 0 = Q4_0, 1 = SP24.  TMA_W: the compressed weight bytes come through TMA into a small
-// shared-memory ring in 128-byte row segments (four k-blocks of Q4_0, two of 2:4 at a time), which
-// is what keeps HBM efficient -- a thread fetching 32 bytes of its own row per k-block opens a
+// TMA_W: the compressed weight bytes come through TMA into a small
+// shared-memory ring in 128-byte row segments (two k-blocks at a time), which
+// is what keeps HBM efficient -- a thread fetching 64 bytes of its own row per k-block opens a
 // DRAM page per access.  Without TMA_W (strides not multiples of 16 bytes) the expander threads
 // load their rows directly.
-template <int MODE, bool TMA_W>
+template <bool TMA_W>
 __global__ void __launch_bounds__(QG_THREADS, 1)
 expand_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW0,
                            const __grid_constant__ CUtensorMap tmW1, const QgParams p) {
-  constexpr int CK = MODE == 0 ? 4 : 2;   // k-blocks per compressed slot
+  constexpr int CK = 2;   // k-blocks per compressed slot
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + QG_BAR_OFF);
@@ -243,22 +202,15 @@ expand_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
                            : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(cmain + ((chunk ^ swz) << 4)) : "memory");
               return v;
             };
-            uint4 q0, q1, q2 = make_uint4(0, 0, 0, 0), q3 = q2;
-            uint32_t aux0, aux1 = 0;
-            if (MODE == 0) {
-              q0 = lds128(2 * j);
-              q1 = lds128(2 * j + 1);
-              asm volatile("ld.shared.u32 %0, [%1];" : "=r"(aux0) : "r"(caux + j * 4) : "memory");
-            } else {
-              q0 = lds128(4 * j); q1 = lds128(4 * j + 1); q2 = lds128(4 * j + 2); q3 = lds128(4 * j + 3);
-              asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(aux0), "=r"(aux1) : "r"(caux + j * 8) : "memory");
-            }
+            const uint4 q0 = lds128(4 * j), q1 = lds128(4 * j + 1), q2 = lds128(4 * j + 2), q3 = lds128(4 * j + 3);
+            uint32_t aux0, aux1;
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(aux0), "=r"(aux1) : "r"(caux + j * 8) : "memory");
             const long long seq = seq0 + kb;
             const int stage = static_cast<int>(seq % QG_STAGES);
             const uint32_t phase = static_cast<uint32_t>((seq / QG_STAGES) & 1);
             if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER)) { ok = false; break; }
             const uint32_t row_base = smem_base + stage * QG_STAGE + QG_A_BYTES + r * 128;
-            expand_row<MODE>(row_base, r, q0, q1, q2, q3, aux0, aux1);
+            expand_row(row_base, r, q0, q1, q2, q3, aux0, aux1);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(full_bar(stage));
@@ -270,7 +222,7 @@ expand_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
     } else {
     // compressed bytes of one 64-wide k-block of this thread's row
     struct Comp { uint4 q0, q1, q2, q3; uint32_t aux0, aux1; };
-    constexpr int PF = MODE == 0 ? 3 : 2;  // own k-blocks fetched ahead (every second k-block is this group's)
+    constexpr int PF = 2;  // own k-blocks fetched ahead (every second k-block is this group's)
     long long seq0 = 0;                    // running number of the tile's first k-block
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, seq0 += k_blocks) {
@@ -282,20 +234,13 @@ expand_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
         c.aux0 = c.aux1 = 0;
         const int k0 = kb * QG_BK;
         if (!row_ok || kb >= k_blocks || k0 + QG_BK > p.K) return;  // K is a multiple of 64 (checked by the host)
-        if (MODE == 0) {
-          const uint8_t* nb_ptr = p.w0 + static_cast<long long>(n) * (p.K >> 1) + (k0 >> 1);
-          c.q0 = __ldg(reinterpret_cast<const uint4*>(nb_ptr));
-          c.q1 = __ldg(reinterpret_cast<const uint4*>(nb_ptr) + 1);
-          c.aux0 = __ldg(reinterpret_cast<const uint32_t*>(p.w1 + (static_cast<long long>(n) * (p.K >> 5) + (k0 >> 5)) * 2));
-        } else {
-          const uint8_t* v_ptr = p.w0 + (static_cast<long long>(n) * (p.K >> 1) + (k0 >> 1)) * 2;
-          c.q0 = __ldg(reinterpret_cast<const uint4*>(v_ptr));
-          c.q1 = __ldg(reinterpret_cast<const uint4*>(v_ptr) + 1);
-          c.q2 = __ldg(reinterpret_cast<const uint4*>(v_ptr) + 2);
-          c.q3 = __ldg(reinterpret_cast<const uint4*>(v_ptr) + 3);
-          const uint2 mt = __ldg(reinterpret_cast<const uint2*>(p.w1 + static_cast<long long>(n) * (p.K >> 3) + (k0 >> 3)));
-          c.aux0 = mt.x; c.aux1 = mt.y;
-        }
+        const uint8_t* v_ptr = p.w0 + (static_cast<long long>(n) * (p.K >> 1) + (k0 >> 1)) * 2;
+        c.q0 = __ldg(reinterpret_cast<const uint4*>(v_ptr));
+        c.q1 = __ldg(reinterpret_cast<const uint4*>(v_ptr) + 1);
+        c.q2 = __ldg(reinterpret_cast<const uint4*>(v_ptr) + 2);
+        c.q3 = __ldg(reinterpret_cast<const uint4*>(v_ptr) + 3);
+        const uint2 mt = __ldg(reinterpret_cast<const uint2*>(p.w1 + static_cast<long long>(n) * (p.K >> 3) + (k0 >> 3)));
+        c.aux0 = mt.x; c.aux1 = mt.y;
       };
       const int kb_first = static_cast<int>((grp - seq0) & 1);   // first k-block of this tile that is ours
       Comp buf[PF];
@@ -314,7 +259,7 @@ expand_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
           const uint32_t phase = static_cast<uint32_t>((seq / QG_STAGES) & 1);
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER)) { ok = false; break; }
           const uint32_t row_base = smem_base + stage * QG_STAGE + QG_A_BYTES + r * 128;
-          expand_row<MODE>(row_base, r, q0, q1, q2, q3, aux0, aux1);
+          expand_row(row_base, r, q0, q1, q2, q3, aux0, aux1);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(full_bar(stage));
@@ -373,10 +318,10 @@ expand_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
   if (threadIdx.x == 0 && *abort_word != 0 && p.status) atomicCAS(p.status, 0, *abort_word);
 }
 
-template <int MODE, bool TMA_W>
+template <bool TMA_W>
 static int launch_expand_t(const CUtensorMap& tmA, const CUtensorMap& tmW0, const CUtensorMap& tmW1, const QgParams& p,
                            int device, int grid, cudaStream_t stream) {
-  auto kern = expand_gemm_tcgen05_kernel<MODE, TMA_W>;
+  auto kern = expand_gemm_tcgen05_kernel<TMA_W>;
   static bool attr_set[64] = {false};
   if (!attr_set[device]) {
     FT_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, QG_SMEM));
@@ -393,10 +338,10 @@ static int launch_expand(const void* x, const QgParams& p0, long long ldx, int d
   CUtensorMap tmA, tmW0, tmW1;
   int rc = make_tmap_2d(&tmA, x, 2, p.K, p.M, ldx * 2, QG_BK, QG_BM, 3);
   if (rc) return rc;
-  // compressed operands as byte matrices: main rows of K/2 (Q4_0 nibbles) or K (2:4 values) bytes,
-  // aux rows of K/16 (fp16 scales) or K/8 (metadata) bytes; TMA needs 16-byte strides and bases
-  const long long main_row = p.mode == 0 ? (p.K >> 1) : p.K;
-  const long long aux_row = p.mode == 0 ? (p.K >> 4) : (p.K >> 3);
+  // compressed operands as byte matrices: main rows of K bytes (values), aux rows of K/8 bytes (metadata); TMA needs 16-byte strides
+  // and bases
+  const long long main_row = p.K;
+  const long long aux_row = p.K >> 3;
   const bool tma_w = main_row % 16 == 0 && aux_row % 16 == 0 && (reinterpret_cast<uintptr_t>(p.w0) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(p.w1) & 15) == 0;
   if (tma_w) {
@@ -411,31 +356,13 @@ static int launch_expand(const void* x, const QgParams& p0, long long ldx, int d
   p.status = device_status_word(device);
   const int tiles = ((p.M + QG_BM - 1) / QG_BM) * ((p.N + QG_BN - 1) / QG_BN);
   const int grid = tiles < sm_count(device) ? tiles : sm_count(device);
-  if (p.mode == 0)
-    return tma_w ? launch_expand_t<0, true>(tmA, tmW0, tmW1, p, device, grid, stream)
-                 : launch_expand_t<0, false>(tmA, tmW0, tmW1, p, device, grid, stream);
-  return tma_w ? launch_expand_t<1, true>(tmA, tmW0, tmW1, p, device, grid, stream)
-               : launch_expand_t<1, false>(tmA, tmW0, tmW1, p, device, grid, stream);
+  return tma_w ? launch_expand_t<true>(tmA, tmW0, tmW1, p, device, grid, stream)
+               : launch_expand_t<false>(tmA, tmW0, tmW1, p, device, grid, stream);
 }
 
 }  // namespace ft
 
 using namespace ft;
-
-// y[M,N] = x[M,K] (bf16, row stride ldx) * dequant_q4_0(nibbles [N, K/2], scales fp16 [N, K/32])^T (+ bias).
-FT_API int ft_q4_0_gemm(const void* x, const void* nibbles, const void* scales, void* y, const void* bias, int M,
-                        int N, int K, long long ldx, long long ldy, int out_f32, int device, cudaStream_t stream) {
-  if (int _rc = ft::ensure_device(device)) return _rc;
-  FT_REQUIRE(x && nibbles && scales && y, "ft_q4_0_gemm: null pointer");
-  FT_REQUIRE(M > 0 && N > 0 && K > 0 && K % 64 == 0 && N % 8 == 0 && ldx % 8 == 0 && ldy % (out_f32 ? 4 : 8) == 0,
-             "ft_q4_0_gemm: K must be a multiple of 64, N of 8");
-  FT_REQUIRE((reinterpret_cast<uintptr_t>(nibbles) & 15) == 0 && (reinterpret_cast<uintptr_t>(scales) & 3) == 0,
-             "ft_q4_0_gemm: nibble plane must be 16-byte aligned");
-  QgParams p{};
-  p.mode = 0; p.C = y; p.ldc = ldy; p.out_f32 = out_f32; p.bias = bias; p.M = M; p.N = N; p.K = K;
-  p.w0 = static_cast<const uint8_t*>(nibbles); p.w1 = static_cast<const uint8_t*>(scales);
-  return launch_expand(x, p, ldx, device, stream);
-}
 
 // y[M,N] = x[M,K] * W^T with W 2:4-compressed: values bf16 [N, K/2], meta u8 [N, K/8] (one nibble
 // per group of 4: bits 0-1 = slot of the first kept value, bits 2-3 = slot of the second).
@@ -449,7 +376,7 @@ FT_API int ft_sparse24_gemm(const void* x, const void* values, const void* meta,
   FT_REQUIRE((reinterpret_cast<uintptr_t>(values) & 15) == 0 && (reinterpret_cast<uintptr_t>(meta) & 7) == 0,
              "ft_sparse24_gemm: value plane must be 16-byte aligned, metadata 8-byte aligned");
   QgParams p{};
-  p.mode = 1; p.C = y; p.ldc = ldy; p.out_f32 = out_f32; p.bias = bias; p.M = M; p.N = N; p.K = K;
+  p.C = y; p.ldc = ldy; p.out_f32 = out_f32; p.bias = bias; p.M = M; p.N = N; p.K = K;
   p.w0 = static_cast<const uint8_t*>(values); p.w1 = static_cast<const uint8_t*>(meta);
   return launch_expand(x, p, ldx, device, stream);
 }

@@ -18,7 +18,7 @@ run with an empty collective part.
 ``weight_format="q4_0"`` keeps the linear weights as GGUF Q4_0 planes (0.5625 bytes per element,
 ferrotorch-serialize/src/gguf.rs:543-545; the reference dequantises whole tensors to bf16 at load
 time, ferrotorch-llama/src/gpu_gguf.rs:336).  The column-parallel layers then run as this
-library's gather kernel followed by the dequant-GEMM (``csrc/quant_gemm.cu``) on the gathered
+library's gather kernel followed by the dequant-GEMM (``csrc/q4_gemm.cu``) on the gathered
 rows, the row-parallel ones as the dequant-GEMM followed by an NCCL reduce-scatter and the
 residual add: two launches per layer instead of one fused kernel.
 """

@@ -1,5 +1,5 @@
-"""Quantised and semi-structured-sparse linear algebra on the expand-GEMM kernel
-(``csrc/quant_gemm.cu``).
+"""Quantised and semi-structured-sparse linear algebra on GEMMs that expand their weight operand
+(``csrc/q4_gemm.cu``, ``csrc/quant_gemm.cu``).
 
 * GGUF Q4_0 weights: :func:`q4_0_planes` splits raw blocks into the nibble / scale planes the
   kernel reads; :func:`q4_0_linear` computes ``x @ dequant(W).T`` without ever materialising the

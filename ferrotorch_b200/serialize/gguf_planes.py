@@ -5,7 +5,7 @@ The reference's portable GPU crate splits a block stream on the host into typed 
 them and expands them with one kernel per block type (ferrotorch-cubecl/src/quant.rs:
 ``GgufBlockKind`` :74, ``split_q4_0_blocks`` :130 ... ``split_q8_1_blocks`` :301,
 ``dequantize_q4_0_to_gpu`` :536 and its five siblings).  The fast path of this package does not
-split: ``csrc/gguf_dequant.cu`` decodes the raw blocks on the device and ``csrc/quant_gemm.cu``
+split: ``csrc/gguf_dequant.cu`` decodes the raw blocks on the device and ``csrc/q4_gemm.cu``
 consumes Q4_0 inside the GEMM.  The plane form is kept for code written against the reference's
 API and as an independent oracle: the split is numpy slicing, the expansion a handful of torch
 ops that run wherever the planes live.

@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from ferrotorch_b200 import _native
 from ferrotorch_b200.ops import quant as Q
 from ferrotorch_b200.ops import reference as R
 from ferrotorch_b200.serialize.gguf import quantize_q4_0
@@ -78,3 +79,35 @@ def test_sparse24_gemm_gpu(M, N, K):
     want = x.float().cpu() @ w.float().t()
     err = (y.float().cpu() - want).abs().max().item()
     assert err < 0.02 * (K ** 0.5) * 0.05 * 4 + 0.05, err
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 16, 33, 128, 129, 256, 300])
+@pytest.mark.parametrize("N,K", [(8, 64), (136, 320), (520, 1088), (3080, 4096)])
+def test_q4_0_product_at_tile_edges(M, N, K):
+    # one and several row tiles, ragged last tiles of W and of the contraction, clusters of 1 to 8 CTAs.  The weights are what an fp32
+    # product rounded to bf16 gives, so against those weights only the sum and the result are rounded
+    torch.manual_seed(M + N + K)
+    nib = torch.randint(0, 256, (N, K // 2), device="cuda", dtype=torch.uint8)
+    sc = (torch.randn(N, K // 32, device="cuda") * 0.01).to(torch.float16)
+    sc[0, 0], sc[-1, -1] = 6e-8, 0.0                              # the smallest fp16, and a block of zeros
+    x, bias = torch.randn(M, K, device="cuda").to(torch.bfloat16), torch.randn(N, device="cuda").to(torch.bfloat16)
+    w = Q.dequant_q4_0_planes(nib, sc).to(torch.bfloat16).double()
+    want = x.double() @ w.t()
+    bound = 2.0 ** -22 * K ** 0.5 * (x.double().abs() @ w.abs().t()) + 1e-12      # sums of K fp32 products
+    got = Q.q4_0_linear(x, nib, sc, out_dtype=torch.float32)
+    assert bool(((got.double() - want).abs() <= bound).all())
+    got = Q.q4_0_linear(x, nib, sc, bias).double()
+    assert bool(((got - want - bias.double()).abs() <= bound + 2.0 ** -8 * (want + bias.double()).abs() + 2.0 ** -20).all())
+    assert torch.equal(Q.q4_0_linear(x, nib, sc), Q.q4_0_linear(x, nib, sc))
+    assert _native.device_status(0) == 0
+
+
+@pytest.mark.gpu
+def test_q4_0_scales_that_are_not_finite():
+    x = torch.ones(2, 64, device="cuda", dtype=torch.bfloat16)
+    nib = torch.full((8, 32), 0x99, device="cuda", dtype=torch.uint8)              # every weight is 1 * scale
+    sc = torch.full((8, 2), 0.5, device="cuda", dtype=torch.float16)
+    sc[1, 0], sc[2, 0], sc[3, 1] = float("inf"), float("nan"), float("-inf")
+    got = Q.q4_0_linear(x, nib, sc).float()
+    assert got[0, 0] == 32 and got[0, 1] == float("inf") and bool(got[0, 2].isnan()) and got[1, 3] == float("-inf")
