@@ -92,6 +92,60 @@ __global__ void im2col_nhwc_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfl
   }
 }
 
+// Patch rows of images with four channels (an RGB image padded by one): a warp builds a row, a lane two taps, one 16-byte store.  With
+// one thread per tap and 64-bit index divisions in each, 256 x 112 x 112 rows of 200 took 1.31 ms; writing them takes 0.2.
+__global__ void __launch_bounds__(256)
+im2col_c4_kernel(const uint2* __restrict__ x, uint4* __restrict__ out, int N, int H, int W, int KH, int KW, int stride, int ph, int pw, int dil,
+                 int Ho, int Wo, int row_vecs) {
+  const int lane = threadIdx.x & 31, taps = KH * KW;
+  const int rows = N * Ho * Wo, step = gridDim.x * (blockDim.x >> 5);
+  for (int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); m < rows; m += step) {
+    const int line = m / Wo, n = line / Ho;
+    const int h0 = (line - n * Ho) * stride - ph, w0 = (m - line * Wo) * stride - pw;
+    const uint2* image = x + static_cast<long long>(n) * H * W;
+    for (int v = lane; v < row_vecs; v += 32) {
+      uint2 q[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int tap = 2 * v + i, kh = tap / KW, h = h0 + kh * dil, w = w0 + (tap - kh * KW) * dil;
+        q[i] = tap < taps && h >= 0 && h < H && w >= 0 && w < W ? __ldg(image + h * W + w) : make_uint2(0u, 0u);
+      }
+      out[static_cast<long long>(m) * row_vecs + v] = make_uint4(q[0].x, q[0].y, q[1].x, q[1].y);
+    }
+  }
+}
+
+// dst[i0, i1, i2] (+)= src[i0, i1, i2] between any strides and types (0 bf16, 1 fp32): filters into the rows that the GEMMs read, filter
+// gradients into the parameter's layout.  order: which place of src along dimension order_dim each index of dst means.
+struct FilterCopy {
+  int n[3];
+  long long ss[3], ds[3];
+  int src_f32, dst_f32, accumulate, order_dim;
+  unsigned char order[64];
+};
+__global__ void __launch_bounds__(256)
+filter_copy_kernel(const void* __restrict__ src, void* __restrict__ dst, const FilterCopy f) {
+  const int total = f.n[0] * f.n[1] * f.n[2];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int r = i / f.n[2], at[3] = {r / f.n[1], r % f.n[1], i - r * f.n[2]};
+    long long s = 0, d = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      s += f.ss[k] * (k == f.order_dim ? f.order[at[k]] : at[k]);
+      d += f.ds[k] * at[k];
+    }
+    float v = f.src_f32 ? static_cast<const float*>(src)[s] : __bfloat162float(static_cast<const __nv_bfloat16*>(src)[s]);
+    if (f.dst_f32) {
+      float* o = static_cast<float*>(dst) + d;
+      *o = f.accumulate ? *o + v : v;
+    } else {
+      __nv_bfloat16* o = static_cast<__nv_bfloat16*>(dst) + d;
+      // what was an addition of a bf16 gradient stays one
+      *o = f.accumulate ? __float2bfloat16(__bfloat162float(*o) + __bfloat162float(__float2bfloat16(v))) : __float2bfloat16(v);
+    }
+  }
+}
+
 static inline int layout_grid(long long work, int device) {
   const long long blocks = (work + 255) / 256;
   const long long cap = static_cast<long long>(sm_count(device)) * 16;
@@ -155,9 +209,43 @@ FT_API int ft_im2col_nhwc(const void* x, void* out, int N, int H, int W, int C, 
   FT_REQUIRE(Kpad >= KH * KW * C && Kpad % 8 == 0, "ft_im2col_nhwc: Kpad=%d too small or not a multiple of 8", Kpad);
   const int Ho = eh / stride + 1, Wo = ew / stride + 1;
   const long long total = static_cast<long long>(N) * Ho * Wo * (KH * KW + 1);
+  if (C == 4 && Kpad % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) & 7) | (reinterpret_cast<uintptr_t>(out) & 15)) == 0 &&
+      static_cast<long long>(N) * Ho * Wo < (1ll << 31) - (1 << 20) && static_cast<long long>(H) * W < (1ll << 31)) {
+    im2col_c4_kernel<<<sm_count(device) * 8, 256, 0, stream>>>(static_cast<const uint2*>(x), static_cast<uint4*>(out), N, H, W, KH, KW, stride,
+                                                               ph, pw, dil, Ho, Wo, Kpad / 8);
+    FT_CUDA_CHECK(cudaGetLastError());
+    count_launch();
+    return FT_E_OK;
+  }
   im2col_nhwc_kernel<<<layout_grid(total, device), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), N, H, W, C, KH, KW, stride, ph, pw,
       dil, Ho, Wo, Kpad);
+  FT_CUDA_CHECK(cudaGetLastError());
+  count_launch();
+  return FT_E_OK;
+}
+
+// dst (+)= src over n0 x n1 x n2 elements with their own strides (elements); *_f32: fp32 instead of bf16; order (or null): n[order_dim]
+// places of src along that dimension, at most 64.
+FT_API int ft_filter_copy(const void* src, void* dst, const int* n, const long long* src_strides, const long long* dst_strides, int src_f32,
+                          int dst_f32, int accumulate, int order_dim, const int* order, int device, cudaStream_t stream) {
+  if (int _rc = ft::ensure_device(device)) return _rc;
+  FT_REQUIRE(src && dst && n && src_strides && dst_strides, "ft_filter_copy: null pointer");
+  FilterCopy f{};
+  long long total = 1;
+  for (int k = 0; k < 3; ++k) {
+    FT_REQUIRE(n[k] > 0, "ft_filter_copy: empty dimension");
+    f.n[k] = n[k]; f.ss[k] = src_strides[k]; f.ds[k] = dst_strides[k];
+    total *= n[k];
+  }
+  FT_REQUIRE(total < (1ll << 31) - (1 << 22), "ft_filter_copy: too many elements");
+  f.src_f32 = src_f32; f.dst_f32 = dst_f32; f.accumulate = accumulate; f.order_dim = -1;
+  if (order) {
+    FT_REQUIRE(order_dim >= 0 && order_dim < 3 && n[order_dim] <= 64, "ft_filter_copy: bad order");
+    f.order_dim = order_dim;
+    for (int i = 0; i < n[order_dim]; ++i) f.order[i] = static_cast<unsigned char>(order[i]);
+  }
+  filter_copy_kernel<<<layout_grid(total, device), 256, 0, stream>>>(src, dst, f);
   FT_CUDA_CHECK(cudaGetLastError());
   count_launch();
   return FT_E_OK;

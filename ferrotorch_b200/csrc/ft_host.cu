@@ -155,6 +155,40 @@ int make_tmap_4d(CUtensorMap* out, const void* base, int dtype_bytes, uint64_t d
   return encode(out, base, dtype_bytes, 4, dims, strides, box, swizzle, is_bf16);
 }
 
+typedef CUresult (*EncodeIm2colFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const int*,
+                                   const int*, cuuint32_t, cuuint32_t, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+int make_tmap_im2col(CUtensorMap* out, const void* base, int C, int W, int H, int N, int low_w, int low_h, int high_w, int high_h,
+                     int channels, int pixels, int step) {
+  static EncodeIm2colFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<EncodeIm2colFn>(p) : nullptr;
+  }();
+  if (!fn) {
+    set_last_error("cuTensorMapEncodeIm2col is not available (no CUDA driver)");
+    return FT_E_NO_DRIVER;
+  }
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || C % 8 != 0) {
+    set_last_error("TMA base address %p or pixel of %d channels is not 16-byte aligned", base, C);
+    return FT_E_BAD_ARG;
+  }
+  const cuuint64_t dims[4] = {static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(W), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(N)};
+  const cuuint64_t strides[3] = {2ull * C, 2ull * C * W, 2ull * C * W * H};
+  const int low[2] = {low_w, low_h}, high[2] = {high_w, high_h};
+  const cuuint32_t steps[4] = {1, static_cast<cuuint32_t>(step), static_cast<cuuint32_t>(step), 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, low, high, channels, pixels, steps,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_last_error("cuTensorMapEncodeIm2col failed with CUresult %d", (int)r);
+    return FT_E_CUDA;
+  }
+  return FT_E_OK;
+}
+
 }  // namespace ft
 
 // Number of kernels this library has launched since load (monotonic).

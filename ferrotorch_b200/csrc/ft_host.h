@@ -44,6 +44,11 @@ int make_tmap_4d(CUtensorMap* out, const void* base, int dtype_bytes, uint64_t d
                  uint64_t d2, uint64_t d3, uint64_t s1, uint64_t s2, uint64_t s3, uint32_t b0,
                  uint32_t b1, uint32_t b2, uint32_t b3, int swizzle, bool is_bf16 = true);
 
+// Encode a tensor map in im2col form over an NHWC bf16 tensor [N, H, W, C] (128-byte swizzle): a load brings `pixels` pixels of `channels`
+// channels; base pixels walk the box from (low_h, low_w) to (H - 1 + high_h, W - 1 + high_w) in steps of `step`.
+int make_tmap_im2col(CUtensorMap* out, const void* base, int C, int W, int H, int N, int low_w, int low_h, int high_w, int high_h,
+                     int channels, int pixels, int step);
+
 int sm_count(int device);
 
 // Make `device` current for this library's CUDA runtime on the calling thread (checked against

@@ -350,6 +350,18 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       : "r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+// The same for a tensor map in im2col form: as many pixels as the map says, from base pixel (w, h) of image n on, each (dw, dh) further on;
+// 64 channels from c on.
+__device__ __forceinline__ void tma_load_im2col_pair(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c, int w, int h, int n,
+                                                     int dw, int dh) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+      :
+      : "r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(static_cast<uint16_t>(dw)),
+        "h"(static_cast<uint16_t>(dh))
+      : "memory");
+}
 // C (+)= tile from shared memory, added by the memory system (no read back to the SM).
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* m, uint32_t src, int x, int y) {
   asm volatile(

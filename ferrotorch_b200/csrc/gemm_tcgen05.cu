@@ -66,7 +66,11 @@ struct GemmParams {
   // MODE 1 output: GEMM row p = (n * gHp + i) * gWp + j is written to row
   // (n * cHo + i - c_oh) * cWo + j - c_ow of C when (i - c_oh, j - c_ow) lies inside the
   // cHo x cWo window, and dropped otherwise (cHo == 0: rows are stored as they are).
+  // MODE 3 with cHo > 0: GEMM row (n, i, j) of gHp x gWp grids goes to row (n * cHo + 2 i + c_oh) * cWo + 2 j + c_ow of C.
   int gHp, gWp, cHo, cWo, c_oh, c_ow;
+  // MODE 3: output pixel m = (n * out_h + i) * out_w + j reads the input pixel (i * step + low_h, j * step + low_w) of image n, and
+  // tap t the one shift[t] >> 16 rows and shift[t] & 0xFFFF columns further on (pixels outside the image are zero).
+  int out_h, out_w, step, low_h, low_w;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, int m_blocks, int n_blocks, int& mb, int& nb) {
@@ -266,6 +270,31 @@ __device__ __forceinline__ void epilogue_crop(const GemmParams& p, uint32_t t_ro
 }
 
 
+// MODE 3 epilogue of one parity of a stride-2 input gradient: row (n, i, j) to its pixel of the input, bf16, no bias.
+template <int BN>
+__device__ __forceinline__ void epilogue_scatter(const GemmParams& p, uint32_t t_row, int row, int n0) {
+  const int r = row / p.gWp, n = r / p.gHp;
+  const long long dst = (static_cast<long long>(n) * p.cHo + 2 * (r - n * p.gHp) + p.c_oh) * p.cWo + 2 * (row - r * p.gWp) + p.c_ow;
+  __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.C) + dst * p.ldc + n0;
+#pragma unroll 1
+  for (int c = 0; c < BN / 32; ++c) {
+    uint32_t v[32];
+    tmem_ld_32x32(t_row + c * 32, v);
+    tmem_ld_wait();
+    if (row >= p.M) continue;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      if (n0 + c * 32 + g * 8 + 8 > p.N) continue;
+      uint4 o;
+      o.x = pack_bf16x2(__uint_as_float(v[g * 8]), __uint_as_float(v[g * 8 + 1]));
+      o.y = pack_bf16x2(__uint_as_float(v[g * 8 + 2]), __uint_as_float(v[g * 8 + 3]));
+      o.z = pack_bf16x2(__uint_as_float(v[g * 8 + 4]), __uint_as_float(v[g * 8 + 5]));
+      o.w = pack_bf16x2(__uint_as_float(v[g * 8 + 6]), __uint_as_float(v[g * 8 + 7]));
+      *reinterpret_cast<uint4*>(out + c * 32 + g * 8) = o;
+    }
+  }
+}
+
 template <int BN, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
@@ -464,6 +493,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 //          operands MN-major, tiles added into an fp32 dW with the TMA reduce-add epilogue.
 // Rows of the padded border hold zeros in the input of MODE 1 / in dY of MODE 2, and the caller
 // drops the border rows of a MODE 1 output.
+//
+// MODE 3 is MODE 1 straight from the unpadded NHWC input: the tiles of input pixels come through a tensor map in im2col form, which walks
+// the output pixels (also every second one) over the image rows and fills in the zeros, so neither a padded copy nor border rows exist
+// and the results leave through the ordinary store; the gradient of a stride-2 filter is four such products, one for each parity of the
+// input pixel.  The sums run over taps and channels as in MODE 1, so the results are the same bits.  ResNet-50 training step, 256 images:
+// 34.9 ms with padded copies, 31.7 now.
 // MODE 5 is a gated product without a pass of its own for the gate: B is [2 N, K], gate rows, then up rows; the two CTAs bring the gate and
 // the up rows of BN / 2 features, so that both accumulate side by side, and act(gate) * up leaves the epilogue (p.taps: the activation).
 // A prefill of four layers of 4096 / 14336: 12997 us with a pass over the rounded product behind it, 12608 now.
@@ -507,6 +542,15 @@ __host__ __device__ constexpr int pair_tile_cols() {
 template <int BN, int MODE>
 __device__ __forceinline__ int pair_num_tiles(const GemmParams& p, int m_blocks, int n_blocks) {
   return MODE == 2 ? m_blocks * n_blocks * p.taps * p.ksplit : m_blocks * n_blocks;
+}
+
+// Where the walk over the output pixels stands in the input, for output pixel m (MODE 3).
+struct PixelAt {
+  int n, h, w;
+};
+__device__ __forceinline__ PixelAt pixel_at(const GemmParams& p, int m) {
+  const int row = m / p.out_w, n = row / p.out_h;
+  return {n, (row - n * p.out_h) * p.step + p.low_h, (m - row * p.out_w) * p.step + p.low_w};
 }
 
 template <int MODE>
@@ -605,6 +649,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const PairTile t = pair_tile<MODE>(p, tile, m_blocks, n_blocks, k_blocks);
         const int m0 = t.mb * 2 * GEMM_BM + static_cast<int>(rank) * GEMM_BM;
         const int n0 = MODE == 5 ? t.nb * BNH + static_cast<int>(rank) * p.N : t.nb * BN + static_cast<int>(rank) * BNH;
+        PixelAt at{0, 0, 0};
+        if constexpr (MODE == 3) at = pixel_at(p, m0);
         for (int kb = t.kb_begin; kb < t.kb_end; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_word, FT_ERR_TIMEOUT_PRODUCER)) {
             ok = false;
@@ -620,6 +666,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             // k-block = (tap, 64 channels): A rows shifted by the tap's offset in the padded image
             const int tap = kb / p.cblocks;
             tma_load_2d_pair(sA, &tmA, fb, (kb - tap * p.cblocks) * GEMM_BK, m0 + p.shift[tap]);
+          } else if constexpr (MODE == 3) {
+            const int tap = kb / p.cblocks;
+            tma_load_im2col_pair(sA, &tmA, fb, (kb - tap * p.cblocks) * GEMM_BK, at.w, at.h, at.n, p.shift[tap] & 0xFFFF, p.shift[tap] >> 16);
           } else if constexpr (!A_MN) {
             tma_load_2d_pair(sA, &tmA, fb, k0, m0);
           } else {
@@ -710,7 +759,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) +
                              static_cast<uint32_t>(acc * BN);
-      if (MODE == 1 && p.cHo > 0) {
+      if (MODE == 3 && p.cHo > 0) {
+        epilogue_scatter<BN>(p, t_row, m0 + lane, n0);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty_bar(acc), 0));
+      } else if (MODE == 1 && p.cHo > 0) {
         epilogue_crop<BN>(p, t_row, m0 + lane, n0);
         tc_fence_before();
         __syncwarp();
@@ -1111,4 +1165,65 @@ FT_API int ft_conv_shift_wgrad(const void* dyp, const void* xp, float* dw, long 
   if (rc) return rc;
   if (bn == 256) return launch_pair<256, true, true, 2>(tmA, tmB, tmC, p, device, max_ctas, stream);
   return launch_pair<128, true, true, 2>(tmA, tmB, tmC, p, device, max_ctas, stream);
+}
+
+namespace ft {
+
+// Geometry of an im2col walk: {images, H, W, out_h, out_w, step, low_h, low_w}; see GemmParams.  offsets[t] = dh << 16 | dw of tap t.
+static int im2col_setup(GemmParams& p, CUtensorMap* map, const void* x, int C, const int* g, int taps, const int* offsets, int pixels) {
+  FT_REQUIRE(g[0] > 0 && g[1] > 0 && g[2] > 0 && g[3] > 0 && g[4] > 0 && g[5] >= 1 && g[5] <= 8, "convolution: bad geometry");
+  FT_REQUIRE(static_cast<long long>(g[0]) * g[3] * g[4] < (1ll << 31) - 65536, "convolution: too many output pixels");
+  FT_REQUIRE(C > 0 && C % 64 == 0 && taps >= 1 && taps <= GEMM_MAX_TAPS, "convolution: %d channels, %d taps", C, taps);
+  for (int t = 0; t < GEMM_MAX_TAPS; ++t) {
+    p.shift[t] = t < taps ? offsets[t] : 0;
+    FT_REQUIRE(p.shift[t] >= 0 && (p.shift[t] & 0xFFFF) <= 255 && (p.shift[t] >> 16) <= 255, "convolution: tap offset out of range");
+  }
+  p.out_h = g[3]; p.out_w = g[4]; p.step = g[5]; p.low_h = g[6]; p.low_w = g[7];
+  p.taps = taps; p.cblocks = C / GEMM_BK; p.ksplit = 1;
+  // the walk visits out_h x out_w positions: the last one is low + (out - 1) * step = extent - 1 + high
+  const int high_h = p.low_h + (p.out_h - 1) * p.step - (g[1] - 1), high_w = p.low_w + (p.out_w - 1) * p.step - (g[2] - 1);
+  for (int v : {p.low_h, p.low_w, high_h, high_w})
+    FT_REQUIRE(v >= -128 && v <= 127, "convolution: padding out of the range of the tensor map");
+  return make_tmap_im2col(map, x, C, g[2], g[1], g[0], p.low_w, p.low_h, high_w, high_h, GEMM_BK, pixels, p.step);
+}
+
+}  // namespace ft
+
+// Convolution of NHWC bf16 input x [images, H, W, Cin] without a padded copy (MODE 3 of the CTA-pair kernel): output pixel (n, i, j),
+// i < out_h, j < out_w, is the sum over taps t and channels of x[n, i * step + low_h + dh(t), j * step + low_w + dw(t), ci] *
+// w[co, t * Cin + ci] (zeros outside the image).  w: [Cout, ldw] bf16, tap-major.  geom and offsets: see im2col_setup.  y [images, out_h,
+// out_w, Cout] bf16 with row stride ldy; with scatter = {H, W, h0, w0}: pixel (i, j) goes to (2 i + h0, 2 j + w0) of [images, H, W, Cout].
+// bias / activation flags as in ft_gemm_bf16 (without scatter).  Cin % 64 == 0, Cout % 8 == 0.
+FT_API int ft_conv_im2col_gemm(const void* x, const void* w, void* y, const void* bias, const int* geom, int Cin, int Cout, int taps,
+                               const int* offsets, long long ldw, long long ldy, int flags, const int* scatter, int device,
+                               cudaStream_t stream) {
+  if (int _rc = ft::ensure_device(device)) return _rc;
+  using namespace ft;
+  FT_REQUIRE(x && w && y && geom && offsets, "ft_conv_im2col_gemm: null pointer");
+  FT_REQUIRE(Cout > 0 && Cout % 8 == 0 && ldw % 8 == 0 && ldw >= static_cast<long long>(taps) * Cin && ldy % 8 == 0 &&
+                 (reinterpret_cast<uintptr_t>(y) & 15) == 0,
+             "ft_conv_im2col_gemm: strides / output must be 16-byte aligned");
+  FT_REQUIRE(!(flags & (GEMM_OUT_F32 | GEMM_ACCUMULATE)), "ft_conv_im2col_gemm: bf16 output, no accumulation");
+  FT_REQUIRE(!(flags & (GEMM_BIAS | GEMM_BIAS_F32)) || bias, "ft_conv_im2col_gemm: bias flag without bias");
+  FT_REQUIRE(!scatter || !(flags & (GEMM_BIAS | GEMM_BIAS_F32 | GEMM_ACT_MASK)), "ft_conv_im2col_gemm: no bias or activation with a scatter");
+  GemmParams p{};
+  CUtensorMap tmA, tmB, tmC;
+  int rc = im2col_setup(p, &tmA, x, Cin, geom, taps, offsets, GEMM_BM);
+  if (rc) return rc;
+  p.C = y; p.bias = bias; p.M = geom[0] * geom[3] * geom[4]; p.N = Cout; p.K = taps * Cin; p.ldc = ldy;
+  p.flags = flags & 0xFFFF;
+  p.status = device_status_word(device);
+  if (scatter) {
+    p.gHp = geom[3]; p.gWp = geom[4]; p.cHo = scatter[0]; p.cWo = scatter[1]; p.c_oh = scatter[2]; p.c_ow = scatter[3];
+    FT_REQUIRE(p.c_oh >= 0 && p.c_oh < 2 && p.c_ow >= 0 && p.c_ow < 2 && 2 * (p.gHp - 1) + p.c_oh < p.cHo && 2 * (p.gWp - 1) + p.c_ow < p.cWo,
+               "ft_conv_im2col_gemm: the scattered pixels do not fit");
+  }
+  const int bn = Cout >= 256 ? 256 : (Cout > 64 ? 128 : 64);
+  rc = make_tmap_2d(&tmB, w, 2, static_cast<uint64_t>(taps) * Cin, Cout, static_cast<uint64_t>(ldw) * 2, GEMM_BK, bn / 2, 3);
+  if (rc) return rc;
+  rc = make_tmap_2d(&tmC, y, 2, Cout, scatter ? static_cast<uint64_t>(geom[0]) * scatter[0] * scatter[1] : static_cast<uint64_t>(p.M), ldy * 2, 64, 32, 3);
+  if (rc) return rc;
+  if (bn == 256) return launch_pair<256, false, false, 3>(tmA, tmB, tmC, p, device, 0, stream);
+  if (bn == 128) return launch_pair<128, false, false, 3>(tmA, tmB, tmC, p, device, 0, stream);
+  return launch_pair<64, false, false, 3>(tmA, tmB, tmC, p, device, 0, stream);
 }

@@ -8,7 +8,10 @@ on the CTA-pair GEMM kernel (``csrc/gemm_tcgen05.cu``):
 
 * **1 x 1 filters** are plain GEMMs over the ``[pixels, channels]`` view (a stride-2 filter first
   keeps every second pixel).
-* **k x k filters, stride 1 or 2** use the *shifted-row* form: the input is copied once into a
+* **k x k filters, stride 1 or 2**, read the input of the forward pass and of the input gradient through tensor maps in im2col form
+  (:class:`Walk`): the tiles of a GEMM are brought in pixel by pixel with the padding filled in, so nothing is copied first; the
+  input gradient of a stride-2 filter is one such GEMM for each parity of the input pixel.
+* **Their filter gradient, and filters outside the ranges of such a map**, use the *shifted-row* form: the input is copied once into a
   zero-padded grid (``csrc/conv_layout.cu``; for stride 2 split into its four parity planes), in
   which the pixel a filter tap reads is a constant row offset away from the output pixel.  The
   forward and input-gradient GEMMs then load their A tiles with ordinary 2-D TMA boxes at
@@ -49,6 +52,8 @@ _native.register_protos({
     "ft_conv_embed": (_i, [_vp, _vp] + [_i] * 11 + [_vp]),
     "ft_conv_crop": (_i, [_vp, _vp] + [_i] * 10 + [_vp]),
     "ft_im2col_nhwc": (_i, [_vp, _vp] + [_i] * 12 + [_vp]),
+    "ft_conv_im2col_gemm": (_i, [_vp] * 5 + [_i] * 3 + [_vp, _ll, _ll, _i, _vp, _i, _vp]),
+    "ft_filter_copy": (_i, [_vp] * 5 + [_i] * 4 + [_vp, _i, _vp]),
 })
 
 _enabled = os.environ.get("FT_CONV_NATIVE", "1") != "0"
@@ -295,6 +300,206 @@ def _ohwi(w: torch.Tensor) -> torch.Tensor:
     return w.to(torch.bfloat16).permute(0, 2, 3, 1).reshape(w.shape[0], -1).contiguous()
 
 
+# --------------------------------------------------------------------------- convolution by im2col walks
+class Walk:
+    """One product over im2col tiles: output pixel ``(n, i, j)`` of ``[N, out_h, out_w]`` reads the input pixel ``(i * step + low_h, j *
+    step + low_w)`` of image n, tap t the one ``offsets[t] = (dh, dw)`` further on; pixels outside the image are zero.  ``taps``: the
+    filter's taps ``kh * KW + kw`` in the order of ``offsets``; ``place``: ``(a, b)`` when output pixel (i, j) is pixel (2 i + a, 2 j + b)
+    of the result."""
+
+    def __init__(self, out_h, out_w, step, low_h, low_w, offsets, taps, place=None):
+        self.out_h, self.out_w, self.step, self.low_h, self.low_w = out_h, out_w, step, low_h, low_w
+        self.offsets, self.taps, self.place = offsets, taps, place
+
+    def high(self, H, W):
+        """How far the last base pixel lies behind the image's last one."""
+        return self.low_h + (self.out_h - 1) * self.step - (H - 1), self.low_w + (self.out_w - 1) * self.step - (W - 1)
+
+    def fits(self, H, W) -> bool:
+        """Within the ranges of a tensor map in im2col form."""
+        return (all(-128 <= v <= 127 for v in (self.low_h, self.low_w, *self.high(H, W)))
+                and all(0 <= v <= 255 for off in self.offsets for v in off))
+
+    def geometry(self, N, H, W):
+        return _int_array([N, H, W, self.out_h, self.out_w, self.step, self.low_h, self.low_w])
+
+    def offset_array(self):
+        return _int_array([dh << 16 | dw for dh, dw in self.offsets])
+
+
+def forward_walk(H, W, KH, KW, stride, ph, pw, dil) -> Walk:
+    return Walk(out_size(H, KH, stride, ph, dil), out_size(W, KW, stride, pw, dil), stride, -ph, -pw,
+                [(kh * dil, kw * dil) for kh in range(KH) for kw in range(KW)], list(range(KH * KW)))
+
+
+def input_gradient_walks(H, W, Ho, Wo, KH, KW, stride, ph, pw, dil) -> list:
+    """The products over dy whose results make up the input gradient: one for stride 1, one for each parity of the input pixel that a
+    stride-2 filter reaches.  Every walk reads dy at ``i + low + offset`` with the taps of one parity."""
+    if stride == 1:
+        return [Walk(H, W, 1, ph - (KH - 1) * dil, pw - (KW - 1) * dil,
+                     [(kh * dil, kw * dil) for kh in range(KH) for kw in range(KW)], list(range(KH * KW))[::-1])]
+    out = []
+    for a in range(min(2, H)):
+        for b in range(min(2, W)):
+            khs, kws = list(range((a + ph) & 1, KH, 2)), list(range((b + pw) & 1, KW, 2))
+            if not khs or not kws:
+                continue
+            R, T = len(khs) - 1, len(kws) - 1
+            out.append(Walk((H - a + 1) // 2, (W - b + 1) // 2, 1, (a + ph - khs[0]) // 2 - R, (b + pw - kws[0]) // 2 - T,
+                            [(R - r, T - t) for r in range(R + 1) for t in range(T + 1)], [kh * KW + kw for kh in khs for kw in kws], (a, b)))
+    return out
+
+
+def walk_reference(x: torch.Tensor, w2d: torch.Tensor, walk: Walk) -> torch.Tensor:
+    """The product of a walk with torch ops: ``x`` logical NCHW, ``w2d [Cout, taps * Cin]`` -> ``[N, Cout, out_h, out_w]``."""
+    N, C, H, W = x.shape
+    hs = torch.arange(walk.out_h) * walk.step + walk.low_h
+    ws = torch.arange(walk.out_w) * walk.step + walk.low_w
+    out = x.new_zeros(N, w2d.shape[0], walk.out_h, walk.out_w)
+    for t, (dh, dw) in enumerate(walk.offsets):
+        h, w = hs + dh, ws + dw
+        ok = ((h >= 0) & (h < H))[:, None] & ((w >= 0) & (w < W))[None]
+        pix = x[:, :, h.clamp(0, H - 1)][:, :, :, w.clamp(0, W - 1)] * ok
+        out += torch.einsum("nchw,oc->nohw", pix, w2d[:, t * C:(t + 1) * C])
+    return out
+
+
+def _ll_array(vals):
+    import ctypes
+
+    return (ctypes.c_longlong * len(vals))(*vals)
+
+
+def _filter_copy(src, dst, n, ss, ds, accumulate=False, order=None, order_dim=-1) -> None:
+    rc = _native.kernels().ft_filter_copy(src.data_ptr(), dst.data_ptr(), _int_array(n), _ll_array(ss), _ll_array(ds),
+                                          int(src.dtype == torch.float32), int(dst.dtype == torch.float32), int(accumulate), order_dim,
+                                          _int_array(order) if order is not None else None, F._dev(dst), F._stream())
+    _native.check(rc, "ft_filter_copy")
+
+
+def _filter_strides(w: torch.Tensor):
+    """Strides (Cout, Cin, tap) of a filter whose taps are evenly spaced, or None."""
+    so, si, sh, sw = w.stride()
+    if w.shape[2] == 1:
+        return so, si, sw if w.shape[3] > 1 else 1
+    if w.shape[3] == 1:
+        return so, si, sh
+    return (so, si, sw) if sh == w.shape[3] * sw else None
+
+
+def _filter_rows(w: torch.Tensor, order: list, transpose: bool) -> torch.Tensor:
+    """``[Cout, taps, Cin]`` bf16, or ``[Cin, taps, Cout]`` with ``transpose``, the taps in the order given."""
+    Cout, Cin, KH, KW = w.shape
+    st = _filter_strides(w)
+    if w.dtype not in (torch.bfloat16, torch.float32) or st is None:
+        w = w.to(torch.bfloat16).contiguous()
+        st = _filter_strides(w)
+    if not transpose and w.dtype == torch.bfloat16 and order == list(range(KH * KW)) and st == (KH * KW * Cin, 1, Cin):
+        return w.permute(0, 2, 3, 1).reshape(Cout, KH * KW, Cin)                    # channels-last storage is these rows
+    R, C = (Cin, Cout) if transpose else (Cout, Cin)
+    out = torch.empty((R, len(order), C), device=w.device, dtype=torch.bfloat16)
+    _filter_copy(w, out, out.shape, (st[1], st[2], st[0]) if transpose else (st[0], st[2], st[1]), out.stride(), order=order, order_dim=1)
+    return out
+
+
+def _deliver_filter_grad(w: torch.Tensor, dw: torch.Tensor, strides: tuple):
+    """``dw`` fp32 with strides ``(Cout, Cin, tap)``: added to ``w.main_grad`` when a flat-arena trainer owns the gradient (returns None),
+    else returned in ``w``'s layout and dtype."""
+    Cout, Cin, KH, KW = w.shape
+    mg = getattr(w, "main_grad", None)
+    dst = mg if mg is not None else torch.empty_like(w)
+    st = _filter_strides(dst)
+    if st is None or dst.dtype not in (torch.bfloat16, torch.float32):
+        g = torch.as_strided(dw, (Cout, KH, KW, Cin), (strides[0], KW * strides[2], strides[2], strides[1]))
+        return _deliver_weight_grad(w, g)
+    # walk dst in the order of its memory
+    dims = sorted(zip(st, (Cout, Cin, KH * KW), strides), key=lambda d: -d[0])
+    _filter_copy(dw, dst, [d[1] for d in dims], [d[2] for d in dims], [d[0] for d in dims], accumulate=mg is not None)
+    if mg is None:
+        return dst
+    hook = getattr(w, "grad_ready_hook", None)
+    if hook is not None:
+        hook(w)
+    return None
+
+
+def _walk_gemm(x: torch.Tensor, rows: torch.Tensor, row_taps: int, first_tap: int, walk: Walk, out: torch.Tensor, bias=None, relu=False) -> None:
+    """``out`` (logical NCHW, channels-last) from input ``x`` (likewise); the walk's filter rows are ``taps`` of the ``row_taps`` taps of
+    ``rows [Cout, row_taps, Cin]`` from ``first_tap`` on."""
+    N, C, H, W = x.shape
+    flags, bias_ptr = (F.GEMM_RELU if relu else 0), None
+    if bias is not None:
+        bias = bias.contiguous()
+        flags |= F.GEMM_BIAS_F32 if bias.dtype == torch.float32 else F.GEMM_BIAS
+        bias_ptr = bias.data_ptr()
+    scatter = _int_array([out.shape[2], out.shape[3], *walk.place]) if walk.place is not None else None
+    rc = _native.kernels().ft_conv_im2col_gemm(
+        x.data_ptr(), rows.data_ptr() + 2 * first_tap * C, out.data_ptr(), bias_ptr, walk.geometry(N, H, W), C, out.shape[1], len(walk.taps),
+        walk.offset_array(), row_taps * C, out.shape[1], flags, scatter, F._dev(x), F._stream())
+    _native.check(rc, "ft_conv_im2col_gemm")
+
+
+def _walks_ok(x, w, s, p, d) -> bool:
+    """Whether every product of the convolution fits an im2col walk (``_shift_supported`` given)."""
+    Cout, Cin, KH, KW = w.shape
+    H, W = x.shape[2:]
+    if Cin % 64 or Cout % 64 or KH * KW > 49:
+        return False
+    fw = forward_walk(H, W, KH, KW, s, p[0], p[1], d)
+    return fw.fits(H, W) and all(g.fits(fw.out_h, fw.out_w)
+                                 for g in input_gradient_walks(H, W, fw.out_h, fw.out_w, KH, KW, s, p[0], p[1], d))
+
+
+class _WalkConv(torch.autograd.Function):
+    """Convolution, stride 1 or 2, on im2col walks: one launch forward and one (stride 2: up to four) for the input gradient, no padded
+    copies for either.  The filter gradient sums over the padded grid, as in :class:`_ShiftConv`.  CUDA tensors only."""
+
+    @staticmethod
+    def forward(ctx, x, w, bias, stride, pad, dil, relu):
+        N, Cin, H, W = x.shape
+        Cout, _, KH, KW = w.shape
+        x = _nhwc(x)
+        walk = forward_walk(H, W, KH, KW, stride, pad[0], pad[1], dil)
+        y = torch.empty((N, Cout, walk.out_h, walk.out_w), device=x.device, dtype=torch.bfloat16, memory_format=CL)
+        _walk_gemm(x, _filter_rows(w, walk.taps, False), KH * KW, 0, walk, y, bias, relu)
+        ctx.save_for_backward(x if w.requires_grad else None, w, y if relu else None)
+        ctx.walk, ctx.cfg, ctx.xshape = walk, (stride, pad, dil, relu, bias is not None), tuple(x.shape)
+        return y
+
+    @staticmethod
+    def backward(ctx, gy):
+        x, w, y = ctx.saved_tensors
+        stride, pad, dil, relu, has_bias = ctx.cfg
+        N, Cin, H, W = ctx.xshape
+        Cout, _, KH, KW = w.shape
+        walk = ctx.walk
+        if relu:
+            gy = gy * (y > 0)
+        gy = _nhwc(gy.to(torch.bfloat16))
+        gx = gw = gb = None
+        if ctx.needs_input_grad[1]:
+            g = ShiftGeometry(N, H, W, KH, KW, stride, pad[0], pad[1], dil)
+            # dy where it lies in the padded input gradient's grid if that is the forward grid too, else at the output's own rows
+            same = stride == 1 and dil * (KH - 1) == 2 * g.ph and dil * (KW - 1) == 2 * g.pw and ctx.needs_input_grad[0]
+            oh, ow = (g.ph, g.pw) if same else (0, 0)
+            dw = _shift_wgrad(_embed(gy, g.Hp, g.Wp, oh, ow, 1), _embed(x, g.Hp, g.Wp, pad[0], pad[1], g.planes), g.P,
+                              [sh - oh * g.Wp - ow for sh in g.shifts()])
+            gw = _deliver_filter_grad(w, dw, (KH * KW * Cin, 1, Cin))
+        if ctx.needs_input_grad[0]:
+            walks = input_gradient_walks(H, W, walk.out_h, walk.out_w, KH, KW, stride, pad[0], pad[1], dil)
+            gx = torch.empty((N, Cin, H, W), device=gy.device, dtype=torch.bfloat16, memory_format=CL)
+            if stride == 2 and len(walks) < min(2, H) * min(2, W):
+                gx.zero_()                                       # pixels that no tap reaches
+            order = [t for g in walks for t in g.taps]
+            rows, first = _filter_rows(w, order, True), 0
+            for g in walks:
+                _walk_gemm(gy, rows, len(order), first, g, gx)
+                first += len(g.taps)
+        if has_bias and ctx.needs_input_grad[2]:
+            gb = gy.float().sum(dim=(0, 2, 3))
+        return gx, gw, gb, None, None, None, None
+
+
 def _deliver_weight_grad(w: torch.Tensor, dw_ohwi: torch.Tensor):
     """``dw_ohwi``: fp32 ``[Cout, KH, KW, Cin]``.  Adds into ``w.main_grad`` when a flat-arena trainer
     owns the gradient (and returns None), else returns the gradient in ``w``'s layout and dtype."""
@@ -436,10 +641,10 @@ class _PointwiseConv(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             if x2.is_cuda and Cin % 64 == 0 and Cout % 64 == 0:
                 # pixels are the contraction dimension: split over the GPU, tiles added in fp32
-                dw = _shift_wgrad(g2, x2, g2.shape[0], [0])
+                gw = _deliver_filter_grad(w, _shift_wgrad(g2, x2, g2.shape[0], [0]), (Cin, 1, 1))
             else:
                 dw = F.gemm_nt(g2.t(), x2.t(), out_dtype=torch.float32)          # [Cout, Cin]
-            gw = _deliver_weight_grad(w, dw.view(Cout, 1, 1, Cin))
+                gw = _deliver_weight_grad(w, dw.view(Cout, 1, 1, Cin))
         if ctx.needs_input_grad[0]:
             w2 = w.to(torch.bfloat16).reshape(Cout, Cin)
             if stride == 1:
@@ -558,7 +763,10 @@ def conv2d(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         s, p, d = _pair(stride)[0], _pair(padding), _pair(dilation)[0]
         fuse_relu = relu and residual is None
         stats[path] += 1
-        if path == "pointwise":
+        # walks outside the ranges of a tensor map (paddings above 127, taps more than 255 apart) keep the padded copy
+        if path == "shift" and _walks_ok(x, weight, s, p, d):
+            y = _WalkConv.apply(x, weight, bias, s, p, d, fuse_relu)
+        elif path == "pointwise":
             y = _PointwiseConv.apply(x, weight, bias, s, fuse_relu)
         elif path == "shift":
             y = _ShiftConv.apply(x, weight, bias, s, p, d, fuse_relu)

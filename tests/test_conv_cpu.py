@@ -149,3 +149,30 @@ def test_the_kernels_own_index_functions_reproduce_conv2d(cin, cout, k, stride, 
     got = (A @ w.permute(0, 2, 3, 1).reshape(cout, -1).t()).reshape(n, ref.shape[2], ref.shape[3], cout).permute(0, 3, 1, 2)
     torch.testing.assert_close(got, ref, rtol=1e-4, atol=1e-4)
     assert (off % 64 == 0)[off >= 0].all()                                           # every run starts on a 128-byte boundary
+
+
+@pytest.mark.parametrize("H,W", [(7, 9), (8, 8), (1, 5), (13, 6)])
+@pytest.mark.parametrize("KH,KW,stride,pad,dil", [
+    (3, 3, 1, (1, 1), 1), (3, 3, 2, (1, 1), 1), (1, 1, 2, (0, 0), 1), (2, 2, 2, (0, 0), 1), (5, 3, 2, (2, 1), 1), (3, 3, 1, (2, 2), 2), (5, 3, 1, (2, 0), 1)])
+def test_walks_cover_forward_and_input_gradient(H, W, KH, KW, stride, pad, dil):
+    if H + 2 * pad[0] < dil * (KH - 1) + 1 or W + 2 * pad[1] < dil * (KW - 1) + 1:
+        pytest.skip("the filter does not fit")
+    torch.manual_seed(H * W + KH)
+    x, w = torch.randn(2, 4, H, W, dtype=torch.double, requires_grad=True), torch.randn(3, 4, KH, KW, dtype=torch.double)
+    ref = tF.conv2d(x, w, None, stride, pad, dil)
+    gy = torch.randn_like(ref)
+    ref.backward(gy)
+    walk = C.forward_walk(H, W, KH, KW, stride, *pad, dil)
+    torch.testing.assert_close(C.walk_reference(x.detach(), w.permute(0, 2, 3, 1).reshape(3, -1), walk), ref.detach())
+    gx = torch.zeros_like(ref.new_zeros(x.shape))
+    for g in C.input_gradient_walks(H, W, walk.out_h, walk.out_w, KH, KW, stride, *pad, dil):
+        assert all(v >= 0 for off in g.offsets for v in off)
+        part = C.walk_reference(gy, w.flatten(2)[:, :, g.taps].permute(1, 2, 0).reshape(4, -1), g)
+        if g.place is None:
+            gx += part
+        else:
+            gx[:, :, g.place[0]::2, g.place[1]::2] = part
+        # the walk stays inside its own box: its last base pixel is where the box ends
+        hi = g.high(*ref.shape[2:])
+        assert g.low_h + (g.out_h - 1) * g.step == ref.shape[2] - 1 + hi[0] and g.low_w + (g.out_w - 1) * g.step == ref.shape[3] - 1 + hi[1]
+    torch.testing.assert_close(gx, x.grad)

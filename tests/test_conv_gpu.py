@@ -166,3 +166,41 @@ def test_folded_resnet_matches_eval_model():
         out = fused(x).float()
     assert torch.isfinite(out).all()
     torch.testing.assert_close(out, ref, rtol=0.1, atol=0.1 * float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("cin,cout,k,stride,pad,dil,n,hw", [
+    (64, 64, 3, 1, (1, 1), 1, 1, (1, 1)), (64, 128, 3, 2, (1, 1), 1, 1, (5, 7)), (128, 64, 1, 2, (0, 0), 1, 2, (9, 8)),
+    (64, 64, 3, 2, (1, 1), 1, 3, (97, 97)), (192, 320, 3, 1, (1, 1), 1, 2, (16, 8)), (64, 256, 2, 2, (0, 0), 1, 2, (8, 10)),
+    (64, 64, (5, 3), 1, (2, 0), 1, 2, (11, 6)), (64, 64, 3, 1, (4, 4), 4, 1, (20, 20)), (64, 64, 3, 2, (0, 0), 1, 2, (8, 8)),
+    (64, 64, 3, 1, (130, 130), 130, 1, (5, 4)),                       # outside a tensor map's range: the padded copy
+])
+@pytest.mark.parametrize("channels_last_filter", [False, True])
+def test_walks_against_torch(cin, cout, k, stride, pad, dil, n, hw, channels_last_filter):
+    # edges of the 256-pixel tiles and of the images, odd sizes, pixels that no tap reaches; filters in either memory format
+    from ferrotorch_b200 import _native
+    from ferrotorch_b200.ops import conv as C
+
+    torch.manual_seed(cin + cout + hw[0])
+    kh, kw = (k, k) if isinstance(k, int) else k
+    x = torch.randn(n, cin, *hw, device="cuda", dtype=torch.bfloat16).contiguous(memory_format=CL)
+    w = (torch.randn(cout, cin, kh, kw, device="cuda") / (cin * kh * kw) ** 0.5).to(torch.bfloat16)
+    w = w.contiguous(memory_format=CL) if channels_last_filter else w
+    xr, wr = x.double().cpu().requires_grad_(), w.double().cpu().requires_grad_()
+    ref = tF.conv2d(xr, wr, None, stride, pad, dil)
+    gy = torch.randn(ref.shape, device="cuda", dtype=torch.bfloat16)
+    ref.backward(gy.double().cpu())
+    xn, wn = x.clone(memory_format=torch.preserve_format).requires_grad_(), w.clone(memory_format=torch.preserve_format).requires_grad_()
+    y = C.conv2d(xn, wn, None, stride, pad, dil)
+    y.backward(gy)
+    # one rounding to bf16 (2^-9 relative) of fp32 sums; the filter gradient sums up to n * Ho * Wo products
+    for got, want in ((y, ref), (xn.grad, xr.grad), (wn.grad, wr.grad)):
+        want = want.detach().cuda()
+        assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -14 * want.abs().max()).all())
+    assert y.is_contiguous(memory_format=CL) and wn.grad.stride() == wn.stride() and _native.device_status(0) == 0
+    # a trainer's gradient arena, bf16 and fp32: the gradient is added to what is there
+    for dt in (torch.bfloat16, torch.float32):
+        wa = w.clone(memory_format=torch.contiguous_format).requires_grad_()
+        wa.main_grad = torch.ones(w.shape, device="cuda", dtype=dt)
+        C.conv2d(x, wa, None, stride, pad, dil).backward(gy)
+        want = wr.grad.cuda() + 1
+        assert wa.grad is None and bool(((wa.main_grad.double() - want).abs() <= 2.0 ** -7 * want.abs() + 2.0 ** -7).all())
