@@ -97,20 +97,37 @@ __global__ void im2col_nhwc_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfl
 __global__ void __launch_bounds__(256)
 im2col_c4_kernel(const uint2* __restrict__ x, uint4* __restrict__ out, int N, int H, int W, int KH, int KW, int stride, int ph, int pw, int dil,
                  int Ho, int Wo, int row_vecs) {
-  const int lane = threadIdx.x & 31, taps = KH * KW;
-  const int rows = N * Ho * Wo, step = gridDim.x * (blockDim.x >> 5);
-  for (int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); m < rows; m += step) {
-    const int line = m / Wo, n = line / Ho;
-    const int h0 = (line - n * Ho) * stride - ph, w0 = (m - line * Wo) * stride - pw;
+  // A warp takes sixteen pixels of an output line at a time: where a lane's two taps lie, and whether their image row exists, is found once
+  // for all of them (with these divisions for every row a ResNet-50 step of 256 images took 31.72 ms, 30.95 now).
+  constexpr int RUN = 16;
+  const int lane = threadIdx.x & 31, taps = KH * KW, runs = (Wo + RUN - 1) / RUN;
+  const int units = N * Ho * runs, step = gridDim.x * (blockDim.x >> 5);
+  for (int u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < units; u += step) {
+    const int line = u / runs, n = line / Ho, wo0 = (u - line * runs) * RUN, count = min(RUN, Wo - wo0);
+    const int h0 = (line - n * Ho) * stride - ph, w0 = wo0 * stride - pw;
     const uint2* image = x + static_cast<long long>(n) * H * W;
     for (int v = lane; v < row_vecs; v += 32) {
-      uint2 q[2];
+      const uint2* row[2];
+      int w[2];
+      bool there[2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int tap = 2 * v + i, kh = tap / KW, h = h0 + kh * dil, w = w0 + (tap - kh * KW) * dil;
-        q[i] = tap < taps && h >= 0 && h < H && w >= 0 && w < W ? __ldg(image + h * W + w) : make_uint2(0u, 0u);
+        const int tap = 2 * v + i, kh = tap / KW, h = h0 + kh * dil;
+        there[i] = tap < taps && h >= 0 && h < H;
+        row[i] = image + (there[i] ? h * W : 0);
+        w[i] = w0 + (tap - kh * KW) * dil;
       }
-      out[static_cast<long long>(m) * row_vecs + v] = make_uint4(q[0].x, q[0].y, q[1].x, q[1].y);
+      uint4* to = out + (static_cast<long long>(line) * Wo + wo0) * row_vecs + v;
+#pragma unroll 4
+      for (int m = 0; m < count; ++m) {
+        uint2 q[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int at = w[i] + m * stride;
+          q[i] = there[i] && at >= 0 && at < W ? __ldg(row[i] + at) : make_uint2(0u, 0u);
+        }
+        to[static_cast<long long>(m) * row_vecs] = make_uint4(q[0].x, q[0].y, q[1].x, q[1].y);
+      }
     }
   }
 }

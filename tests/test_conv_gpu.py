@@ -204,3 +204,18 @@ def test_walks_against_torch(cin, cout, k, stride, pad, dil, n, hw, channels_las
         C.conv2d(x, wa, None, stride, pad, dil).backward(gy)
         want = wr.grad.cuda() + 1
         assert wa.grad is None and bool(((wa.main_grad.double() - want).abs() <= 2.0 ** -7 * want.abs() + 2.0 ** -7).all())
+
+
+@pytest.mark.parametrize("n,hw,k,stride,pad,dil", [(2, (17, 35), (7, 7), 2, (3, 3), 1), (1, (9, 16), (3, 2), 1, (0, 1), 2), (3, (40, 33), (9, 9), 3, (4, 4), 1),
+                                                   (1, (5, 5), (5, 5), 1, (0, 0), 1)])
+def test_patch_rows_of_four_channels(n, hw, k, stride, pad, dil):
+    # runs of sixteen pixels that end with a line, rows of up to 41 vectors, taps and columns behind the filter's
+    from ferrotorch_b200.ops import conv as C
+
+    torch.manual_seed(hw[0])
+    x = torch.randn(n, 4, *hw, device="cuda", dtype=torch.bfloat16)
+    ho, wo = (C.out_size(hw[i], k[i], stride, pad[i], dil) for i in range(2))
+    kpad = (k[0] * k[1] * 4 + 15) // 8 * 8
+    got = C._im2col(x.contiguous(memory_format=CL).permute(0, 2, 3, 1).contiguous().permute(0, 3, 1, 2), *k, stride, pad, dil, ho, wo, kpad)
+    want = tF.unfold(x.float(), k, dil, pad, stride).view(n, 4, k[0] * k[1], ho * wo).permute(0, 3, 2, 1).reshape(n * ho * wo, -1)
+    assert torch.equal(got[:, :want.shape[1]].float(), want) and not bool(got[:, want.shape[1]:].any())
