@@ -415,6 +415,9 @@ def test_gemm_stream_row_tiles(M, N, K):
     y = F._gemm_stream(x, w, out[:M], None, 0)
     assert bool(((y.double() - want).abs() <= bound).all()) and bool((out[M] == 7).all())
     assert torch.equal(F.gemm_nt(x, w), y) == F._streams(M, N, K) or not F._streams(M, N, K)
+    with torch.no_grad():
+        assert torch.equal(F.linear(x, w), F.gemm_nt(x, w))
+    assert torch.equal(F.linear(x.clone().requires_grad_(), w), F.gemm_nt(x, w, split=False))
     want = torch.relu(want + bias.double())
     got = F._gemm_stream(x, w, torch.empty_like(y), bias, F._ACT_FLAGS["relu"])
     assert bool(((got.double() - want).abs() <= bound + 2.0 ** -8 * want.abs() + 2.0 ** -18).all())
