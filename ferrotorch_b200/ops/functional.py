@@ -170,9 +170,10 @@ def _gemm_ok(a: torch.Tensor, b: torch.Tensor, la, lb, N: int) -> bool:
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = None,
             out: torch.Tensor | None = None, accumulate: bool = False,
             out_dtype: torch.dtype | None = None, activation: str | None = None,
-            bn: int = 0, max_ctas: int = 0, split: bool = True) -> torch.Tensor:
-    """``out (+)= a @ b.T (+ bias)`` for logical ``a [M,K]``, ``b [N,K]`` (bf16 in, fp32 accumulate).  ``split=False``: above 128 rows
-    every sum runs from the first to the last of the contraction, in no parts."""
+            bn: int = 0, max_ctas: int = 0, split: bool = False) -> torch.Tensor:
+    """``out (+)= a @ b.T (+ bias)`` for logical ``a [M,K]``, ``b [N,K]`` (bf16 in, fp32 accumulate).  Above 128 rows every sum of a bf16
+    result runs from the first to the last of the contraction; ``split=True`` (inference) lets it be added up from parts where that is
+    faster (:func:`_streams`)."""
     M, K = a.shape
     N, K2 = b.shape
     assert K == K2, "gemm_nt: contraction mismatch %s x %s" % (tuple(a.shape), tuple(b.shape))
@@ -466,7 +467,7 @@ def linear_rows(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = No
     """``act(a [T, K] @ w.T + bias)`` for inference in the type of its operands (bf16 on the tcgen05 GEMM, fp32 as true
     fp32); ``bias`` fp32."""
     if a.dtype == torch.bfloat16:
-        return gemm_nt(a, w, bias=bias, activation=activation)
+        return gemm_nt(a, w, bias=bias, activation=activation, split=True)
     y = _mm_f32(a, w)
     if bias is not None:
         y += bias

@@ -414,13 +414,53 @@ def test_gemm_stream_row_tiles(M, N, K):
     out = torch.full((M + 1, N), 7.0, device=DEV, dtype=torch.bfloat16)
     y = F._gemm_stream(x, w, out[:M], None, 0)
     assert bool(((y.double() - want).abs() <= bound).all()) and bool((out[M] == 7).all())
-    assert torch.equal(F.gemm_nt(x, w), y) == F._streams(M, N, K) or not F._streams(M, N, K)
+    assert torch.equal(F.gemm_nt(x, w, split=True), y) == F._streams(M, N, K) or not F._streams(M, N, K)
     with torch.no_grad():
-        assert torch.equal(F.linear(x, w), F.gemm_nt(x, w))
+        assert torch.equal(F.linear(x, w), F.gemm_nt(x, w, split=True))
     assert torch.equal(F.linear(x.clone().requires_grad_(), w), F.gemm_nt(x, w, split=False))
     want = torch.relu(want + bias.double())
     got = F._gemm_stream(x, w, torch.empty_like(y), bias, F._ACT_FLAGS["relu"])
     assert bool(((got.double() - want).abs() <= bound + 2.0 ** -8 * want.abs() + 2.0 ** -18).all())
+    assert _native.device_status(0) == 0
+
+
+@pytest.mark.parametrize("M", [129, 192, 256])
+def test_training_forwards_keep_undivided_sums(M):
+    # every product of a training step's forward pass above 128 rows, for sizes that inference divides: plain, packed projection of
+    # attention, logits of the fused loss, convolutions of 1 x 1 and of patch rows
+    from ferrotorch_b200.ops import conv as C
+    from ferrotorch_b200.ops.attention import qkv_attention
+
+    torch.manual_seed(M)
+    H, N = 2048, 2048
+    assert F._streams(M, N, H)
+    h, w = _rand(M, H).requires_grad_(), (_rand(N, H) * 0.05).requires_grad_()
+    plain = F.gemm_nt(h.detach(), w.detach(), split=False)
+    assert torch.equal(F.linear(h, w), plain) and not torch.equal(F.gemm_nt(h.detach(), w.detach(), split=True), plain)
+
+    wq = (_rand(3072, H) * 0.05).requires_grad_()
+    out = qkv_attention(h[None], wq, None, None, None, n_heads=16, n_kv_heads=4, head_dim=128)
+    q = F.gemm_nt(h.detach(), wq.detach(), split=False).view(1, M, 24, 128)
+    assert torch.equal(out[0], F.flash_attn_fwd(q[:, :, :16], q[:, :, 16:20], q[:, :, 20:], True)[0].view(M, H))
+
+    target = torch.randint(0, N, (M,), device=DEV)
+    loss = F.linear_cross_entropy(h, w, target)
+    rows = F.cross_entropy_fwd_bwd_(plain.clone(), target, 1.0 / M, write_grad=False)
+    assert torch.equal(loss, rows.sum() / M)
+
+    x = _rand(1, H, M, 1).contiguous(memory_format=torch.channels_last)
+    x2 = x.permute(0, 2, 3, 1).reshape(M, H)
+    y = C.conv2d(x, w.detach().view(N, H, 1, 1).clone().requires_grad_())
+    assert torch.equal(y.permute(0, 2, 3, 1).reshape(M, N), F.gemm_nt(x2, w.detach(), split=False))
+    xs, ws = _rand(1, 255, M, 3).contiguous(memory_format=torch.channels_last), (_rand(N, 255, 3, 3) * 0.05).requires_grad_()
+    n0 = C.stats["im2col"]
+    y = C.conv2d(xs, ws, padding=(1, 0))
+    assert C.stats["im2col"] == n0 + 1
+    xp = C._pad_channels(xs, 256)
+    patches = C._im2col(xp, 3, 3, 1, (1, 0), 1, M, 1, 9 * 256)
+    w2 = torch.zeros(N, 9, 256, device=DEV, dtype=torch.bfloat16)
+    w2[:, :, :255] = ws.detach().permute(0, 2, 3, 1).reshape(N, 9, 255)
+    assert torch.equal(y.permute(0, 2, 3, 1).reshape(M, N), F.gemm_nt(patches, w2.view(N, -1), split=False))
     assert _native.device_status(0) == 0
 
 
