@@ -250,6 +250,7 @@ class LlamaForCausalLM(nn.Module):
         return PagedKVCache(c.num_hidden_layers, c.num_key_value_heads, c.head_dim, num_blocks, max_seqs, max_seq_len, block_size,
                             device=p.device, dtype=p.dtype)
 
+    @F.serving
     @torch.no_grad()
     def paged_forward(self, batch, cache) -> torch.Tensor:
         """One pass over a :class:`~ferrotorch_b200.nn.paged.RaggedBatch`: logits of its wanted rows ``[wanted, vocab]``."""

@@ -140,8 +140,8 @@ class SwiGLU(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         up = self.gate_up_proj
-        if type(up) is Linear and up.bias is None and not torch.is_grad_enabled() and not (up._forward_hooks or up._forward_pre_hooks
-                                                                                           or nn.modules.module._has_any_global_hook()):
+        if type(up) is Linear and up.bias is None and F.serves() and not (up._forward_hooks or up._forward_pre_hooks
+                                                                            or nn.modules.module._has_any_global_hook()):
             return self.down_proj(F.linear_swiglu(x, up.weight, self.activation, self.activation_param))
         return self.down_proj(F.swiglu(up(x), self.activation, self.activation_param))
 

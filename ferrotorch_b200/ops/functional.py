@@ -13,6 +13,9 @@ ferrotorch-core/src/grad_fns/linalg.rs:1440-1519).
 """
 from __future__ import annotations
 
+import functools
+import threading
+
 import torch
 
 from .. import _native
@@ -136,6 +139,33 @@ def _transformed() -> bool:
             or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling())
 
 
+class _Serving(threading.local):
+    on = False
+
+
+_serving = _Serving()
+
+
+def serving(fn):
+    """Decorator of a pass that only serves (``paged_forward``): without gradients its products may be added up from parts and a gated
+    projection may leave its GEMM as ``act(gate) * up``.  Everywhere else a module computes the same bits with and without gradients."""
+
+    @functools.wraps(fn)
+    def call(*args, **kwargs):
+        before, _serving.on = _serving.on, True
+        try:
+            return fn(*args, **kwargs)
+        finally:
+            _serving.on = before
+
+    return call
+
+
+def serves() -> bool:
+    """Whether the calling thread is in a pass that :func:`serving` marks, and records no gradients."""
+    return _serving.on and not torch.is_grad_enabled()
+
+
 def _apply(fn, *args):
     """``fn.apply(*args)``; without gradients, function transforms, forward-mode levels or tracing the forward by itself (a decoder layer's
     16 us a call for a node that is thrown away)."""
@@ -243,9 +273,7 @@ class _LinearFn(torch.autograd.Function):
         # the output is allocated in its final shape (not returned as a view) so that callers
         # may modify it in place
         y = torch.empty((*shp[:-1], w.shape[0]), device=x.device, dtype=x.dtype)
-        # training keeps undivided sums: parts gain 1 % of a step of 312 rows, and three steps later the gradients are further from what
-        # they were than rounding alone moves them
-        gemm_nt(x2, w, bias=bias, out=y.view(-1, w.shape[0]), split=isinstance(ctx, _NoContext))
+        gemm_nt(x2, w, bias=bias, out=y.view(-1, w.shape[0]), split=isinstance(ctx, _NoContext) and _serving.on)
         ctx.save_for_backward(x2, w)
         ctx.has_bias = bias is not None
         ctx.in_shape = shp

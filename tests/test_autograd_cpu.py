@@ -220,3 +220,30 @@ def test_a_forward_runs_alone_only_where_nothing_looks_at_it():
     w = torch.ones(2, requires_grad=True)
     F._apply(Twice, w * 1).sum().backward()
     assert not alone() and torch.equal(w.grad, torch.full((2,), 2.0))
+
+
+def test_a_serving_pass_is_one_of_its_thread_and_records_no_gradients():
+    import threading
+
+    from ferrotorch_b200.ops import functional as F
+
+    seen = {}
+
+    @F.serving
+    def outer(fail=False):
+        seen["grad"] = F.serves()
+        with torch.no_grad():
+            seen["here"] = F.serves()
+            F.serving(lambda: None)()
+            seen["after"] = F.serves()
+            t = threading.Thread(target=lambda: seen.update(there=F.serves()))
+            t.start(), t.join()
+        if fail:
+            raise ValueError
+
+    outer()
+    assert seen == dict(grad=False, here=True, after=True, there=False)
+    with pytest.raises(ValueError):
+        outer(fail=True)
+    with torch.no_grad():
+        assert not F.serves()

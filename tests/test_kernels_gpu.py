@@ -416,7 +416,7 @@ def test_gemm_stream_row_tiles(M, N, K):
     assert bool(((y.double() - want).abs() <= bound).all()) and bool((out[M] == 7).all())
     assert torch.equal(F.gemm_nt(x, w, split=True), y) == F._streams(M, N, K) or not F._streams(M, N, K)
     with torch.no_grad():
-        assert torch.equal(F.linear(x, w), F.gemm_nt(x, w, split=True))
+        assert torch.equal(F.serving(F.linear)(x, w), F.gemm_nt(x, w, split=True))
     assert torch.equal(F.linear(x.clone().requires_grad_(), w), F.gemm_nt(x, w, split=False))
     want = torch.relu(want + bias.double())
     got = F._gemm_stream(x, w, torch.empty_like(y), bias, F._ACT_FLAGS["relu"])
@@ -432,7 +432,7 @@ def test_training_forwards_keep_undivided_sums(M):
     from ferrotorch_b200.ops.attention import qkv_attention
 
     torch.manual_seed(M)
-    H, N = 2048, 2048
+    H, N = 4096, 2048
     assert F._streams(M, N, H)
     h, w = _rand(M, H).requires_grad_(), (_rand(N, H) * 0.05).requires_grad_()
     plain = F.gemm_nt(h.detach(), w.detach(), split=False)
@@ -461,6 +461,30 @@ def test_training_forwards_keep_undivided_sums(M):
     w2 = torch.zeros(N, 9, 256, device=DEV, dtype=torch.bfloat16)
     w2[:, :, :255] = ws.detach().permute(0, 2, 3, 1).reshape(N, 9, 255)
     assert torch.equal(y.permute(0, 2, 3, 1).reshape(M, N), F.gemm_nt(patches, w2.view(N, -1), split=False))
+    assert _native.device_status(0) == 0
+
+
+@pytest.mark.parametrize("M", [3, 128, 192, 320, 524])
+def test_modules_compute_the_same_with_and_without_gradients(M):
+    # sizes that a serving pass adds up from parts, or gates in the GEMM
+    from ferrotorch_b200.nn.layers import Linear, SwiGLU
+
+    torch.manual_seed(M)
+    x = _rand(1, M, 4096)
+    for layer in (Linear(4096, 2048), Linear(4096, 2048, bias=False), Linear(8192, 4096), SwiGLU(4096, 5504)):
+        layer = layer.to(DEV, torch.bfloat16)
+        h = x if isinstance(layer, SwiGLU) or layer.in_features == 4096 else torch.cat([x, x], -1)
+        y = layer(h)
+        assert y.requires_grad
+        with torch.no_grad():
+            assert torch.equal(layer(h), y)
+        with torch.inference_mode():
+            assert torch.equal(layer(h), y)
+        assert torch.equal(F.serving(layer)(h), y)              # gradients are recorded: nothing changes
+        # a pass that serves is as close to 64 bits
+        with torch.no_grad():
+            got = F.serving(layer)(h)
+        assert not F.serves() and float((got.double() - y.double()).norm() / y.double().norm()) < 2.0 ** -7
     assert _native.device_status(0) == 0
 
 
