@@ -452,23 +452,28 @@ def _walks_ok(x, w, s, p, d) -> bool:
 
 class _WalkConv(torch.autograd.Function):
     """Convolution, stride 1 or 2, on im2col walks: one launch forward and one (stride 2: up to four) for the input gradient, no padded
-    copies for either.  The filter gradient sums over the padded grid, as in :class:`_ShiftConv`.  CUDA tensors only."""
+    copies for either.  The filter gradient sums over the padded grid, as in :class:`_ShiftConv`; with ``train`` the forward pass makes
+    that copy of the input, so that a caller may change the input in place before the backward pass.  CUDA tensors only."""
 
     @staticmethod
-    def forward(ctx, x, w, bias, stride, pad, dil, relu):
+    def forward(ctx, x, w, bias, stride, pad, dil, relu, train):
         N, Cin, H, W = x.shape
         Cout, _, KH, KW = w.shape
         x = _nhwc(x)
         walk = forward_walk(H, W, KH, KW, stride, pad[0], pad[1], dil)
         y = torch.empty((N, Cout, walk.out_h, walk.out_w), device=x.device, dtype=torch.bfloat16, memory_format=CL)
         _walk_gemm(x, _filter_rows(w, walk.taps, False), KH * KW, 0, walk, y, bias, relu)
-        ctx.save_for_backward(x if w.requires_grad else None, w, y if relu else None)
+        xp = None
+        if train and w.requires_grad:
+            g = ShiftGeometry(N, H, W, KH, KW, stride, pad[0], pad[1], dil)
+            xp = _embed(x, g.Hp, g.Wp, pad[0], pad[1], g.planes)
+        ctx.save_for_backward(xp, w, y if relu else None)
         ctx.walk, ctx.cfg, ctx.xshape = walk, (stride, pad, dil, relu, bias is not None), tuple(x.shape)
         return y
 
     @staticmethod
     def backward(ctx, gy):
-        x, w, y = ctx.saved_tensors
+        xp, w, y = ctx.saved_tensors
         stride, pad, dil, relu, has_bias = ctx.cfg
         N, Cin, H, W = ctx.xshape
         Cout, _, KH, KW = w.shape
@@ -482,8 +487,7 @@ class _WalkConv(torch.autograd.Function):
             # dy where it lies in the padded input gradient's grid if that is the forward grid too, else at the output's own rows
             same = stride == 1 and dil * (KH - 1) == 2 * g.ph and dil * (KW - 1) == 2 * g.pw and ctx.needs_input_grad[0]
             oh, ow = (g.ph, g.pw) if same else (0, 0)
-            dw = _shift_wgrad(_embed(gy, g.Hp, g.Wp, oh, ow, 1), _embed(x, g.Hp, g.Wp, pad[0], pad[1], g.planes), g.P,
-                              [sh - oh * g.Wp - ow for sh in g.shifts()])
+            dw = _shift_wgrad(_embed(gy, g.Hp, g.Wp, oh, ow, 1), xp, g.P, [sh - oh * g.Wp - ow for sh in g.shifts()])
             gw = _deliver_filter_grad(w, dw, (KH * KW * Cin, 1, Cin))
         if ctx.needs_input_grad[0]:
             walks = input_gradient_walks(H, W, walk.out_h, walk.out_w, KH, KW, stride, pad[0], pad[1], dil)
@@ -497,7 +501,7 @@ class _WalkConv(torch.autograd.Function):
                 first += len(g.taps)
         if has_bias and ctx.needs_input_grad[2]:
             gb = gy.float().sum(dim=(0, 2, 3))
-        return gx, gw, gb, None, None, None, None
+        return gx, gw, gb, None, None, None, None, None
 
 
 def _deliver_weight_grad(w: torch.Tensor, dw_ohwi: torch.Tensor):
@@ -765,7 +769,7 @@ def conv2d(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         stats[path] += 1
         # walks outside the ranges of a tensor map (paddings above 127, taps more than 255 apart) keep the padded copy
         if path == "shift" and _walks_ok(x, weight, s, p, d):
-            y = _WalkConv.apply(x, weight, bias, s, p, d, fuse_relu)
+            y = _WalkConv.apply(x, weight, bias, s, p, d, fuse_relu, torch.is_grad_enabled())
         elif path == "pointwise":
             y = _PointwiseConv.apply(x, weight, bias, s, fuse_relu)
         elif path == "shift":

@@ -219,3 +219,22 @@ def test_patch_rows_of_four_channels(n, hw, k, stride, pad, dil):
     got = C._im2col(x.contiguous(memory_format=CL).permute(0, 2, 3, 1).contiguous().permute(0, 3, 1, 2), *k, stride, pad, dil, ho, wo, kpad)
     want = tF.unfold(x.float(), k, dil, pad, stride).view(n, 4, k[0] * k[1], ho * wo).permute(0, 3, 2, 1).reshape(n * ho * wo, -1)
     assert torch.equal(got[:, :want.shape[1]].float(), want) and not bool(got[:, want.shape[1]:].any())
+
+
+@pytest.mark.parametrize("k,stride,pad,relu", [(3, 1, 1, False), (3, 2, 1, True), (2, 1, 0, False)])
+def test_the_input_may_change_in_place_before_the_backward_pass(k, stride, pad, relu):
+    from ferrotorch_b200.ops import conv as C
+
+    x, w, b = _case(64, 64, k, 2, (9, 10), seed=k)
+    grads = []
+    for change in (False, True):
+        wn, h = w.clone().requires_grad_(), x.clone(memory_format=torch.preserve_format)
+        leaf = torch.zeros((), device="cuda", dtype=torch.bfloat16, requires_grad=True)
+        h = h + leaf                                    # an activation that records gradients
+        y = C.conv2d(h, wn, b, stride, pad, relu=relu)
+        if change:
+            h.mul_(-3).add_(1)
+        y.float().pow(2).sum().backward()
+        grads.append((y.detach(), wn.grad, leaf.grad))
+    for got, want in zip(grads[1], grads[0]):
+        assert torch.equal(got, want)
