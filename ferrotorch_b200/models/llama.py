@@ -264,8 +264,7 @@ class LlamaForCausalLM(nn.Module):
             attn = layer.self_attn
             Hq, Hkv, D, T = attn.n_heads, attn.n_kv_heads, attn.head_dim, batch.n_rows
             qkv = attn.qkv_proj(h).view(1, T, Hq + 2 * Hkv, D)
-            cache.append_rotated(li, qkv[0], attn.rope, batch, Hq)
-            a = cache.attend(li, qkv[0, :, :Hq], batch)
+            a = cache.attend(li, cache.append_rotated(li, qkv[0], attn.rope, batch, Hq), batch)
             h, x = layer.post_attention_layernorm(x, attn.o_proj(a.view(1, T, Hq * D)))
             delta = layer.mlp(h)
         h, _ = m.norm(x, delta)

@@ -16,6 +16,14 @@ from ..ops import functional as F
 from ..ops import reference as ref
 
 
+def runs_plainly(module: nn.Module, cls: type) -> bool:
+    """Whether calling ``module`` is ``cls.forward`` and nothing else, so that a kernel may stand for the call: no subclass, no ``forward``
+    set on the instance, no compiled call, no hook on it or on all modules."""
+    return (type(module) is cls and "forward" not in module.__dict__ and module._compiled_call_impl is None
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                     or nn.modules.module._has_any_global_hook()))
+
+
 class Linear(nn.Linear):
     """``y = x W^T + b`` on the tcgen05 GEMM (bf16 CUDA inputs); any other input uses torch."""
 
@@ -140,8 +148,7 @@ class SwiGLU(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         up = self.gate_up_proj
-        if type(up) is Linear and up.bias is None and F.serves() and not (up._forward_hooks or up._forward_pre_hooks
-                                                                            or nn.modules.module._has_any_global_hook()):
+        if F.serves() and runs_plainly(up, Linear) and up.bias is None:
             return self.down_proj(F.linear_swiglu(x, up.weight, self.activation, self.activation_param))
         return self.down_proj(F.swiglu(up(x), self.activation, self.activation_param))
 

@@ -17,6 +17,7 @@ import torch
 from .. import _native
 from ..ops import functional as F
 from ..ops import reference as ref
+from .layers import RotaryPositionEmbedding, runs_plainly
 
 _i, _ll, _f, _vp = _native._i, _native._ll, _native._f, _native._vp
 _native.register_protos({
@@ -440,27 +441,26 @@ class PagedKVCache:
             self.num_blocks, F._dev(k_new), F._stream())
         _native.check(rc, "ft_kv_append")
 
-    def append_rotated(self, layer: int, packed: torch.Tensor, rope, batch: RaggedBatch, n_heads: int) -> None:
+    def append_rotated(self, layer: int, packed: torch.Tensor, rope, batch: RaggedBatch, n_heads: int) -> torch.Tensor:
         """``packed [T, Hq + 2 Hkv, D]``: the q and k heads rotated by the positions of a batch, the keys and values written to their pages
-        (:meth:`append`).  On a device the keys of ``packed`` may be left as they were."""
+        (:meth:`append`).  Returns the rotated q heads.  On a device ``packed`` may be rotated in place, its keys may be left as they were."""
         T, H, D = packed.shape
         Hkv, Dk, Dv = self.shapes[layer]
-        if (packed.is_cuda and F.native_enabled() and packed.dtype == torch.bfloat16 == self.dtype and rope is not None and not rope.interleaved
-                and rope.head_dim == D and not (rope._forward_hooks or rope._forward_pre_hooks)
+        if (packed.is_cuda and F.native_enabled() and packed.dtype == torch.bfloat16 == self.dtype and rope is not None
+                and runs_plainly(rope, RotaryPositionEmbedding) and not rope.interleaved and rope.head_dim == D
                 and D == Dk == Dv and D % 16 == 0 and H == n_heads + 2 * Hkv and not self.values_in_keys[layer] and packed.stride(2) == 1
-                and packed.stride(1) == D and packed.stride(0) % 8 == 0 and packed.data_ptr() % 16 == 0 and not torch.is_grad_enabled()):
+                and packed.stride(1) == D and packed.stride(0) % 8 == 0 and packed.data_ptr() % 16 == 0 and not torch.is_grad_enabled()
+                and not F._transformed()):
             cos, sin = rope._tables(packed.device)
             rc = _native.kernels().ft_rope_append(
                 packed.data_ptr(), cos.data_ptr(), sin.data_ptr(), batch.positions.data_ptr(), batch.slots.data_ptr(), self.sync_table().data_ptr(),
                 self.k[layer].data_ptr(), self.v[layer].data_ptr(), T, n_heads, Hkv, D, packed.stride(0), self.block_size, self.max_blocks,
                 self.num_blocks, F._dev(packed), F._stream())
             _native.check(rc, "ft_rope_append")
-            return
-        if rope is not None:
-            rotated = rope(packed[None], positions=batch.positions, n_rot_heads=n_heads + Hkv)[0]
-            if rotated.data_ptr() != packed.data_ptr():
-                packed.copy_(rotated)
-        self.append(layer, packed[:, n_heads:n_heads + Hkv], packed[:, n_heads + Hkv:], batch.positions, batch.slots)
+            return packed[:, :n_heads]
+        rotated = packed if rope is None else rope(packed[None], positions=batch.positions, n_rot_heads=n_heads + Hkv)[0]
+        self.append(layer, rotated[:, n_heads:n_heads + Hkv], rotated[:, n_heads + Hkv:], batch.positions, batch.slots)
+        return rotated[:, :n_heads]
 
     def _check_pool(self, layer: int, pool, window, chunk, slopes) -> None:
         if pool and (not window or chunk or slopes is not None or (layer, pool) not in self.pooled):

@@ -208,3 +208,64 @@ def test_paged_decode_reads_nothing_past_the_context(bs, D, Dv, splits, window):
         want = torch.einsum("ht,thd->hd", p, v)
         # P and the result are rounded to bf16
         assert bool(((out[b].float() - want).abs() <= 2.0 ** -7 * (1 + want.abs())).all()), "sequence of %d" % n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("change", ["subclass", "forward", "hook", "global hook"])
+def test_rotations_and_projections_that_are_not_plain_are_called(change):
+    from torch import nn
+
+    from ferrotorch_b200.nn.layers import Linear, RotaryPositionEmbedding, SwiGLU
+    from ferrotorch_b200.nn.paged import RaggedBatch
+    from ferrotorch_b200.ops import functional as F
+
+    def altered(cls, factor, *args):
+        """A module of cls whose result is ``factor`` times what it would be."""
+        def scaled(m, x, **kwargs):
+            return cls.forward(m, x, **kwargs) * factor
+
+        handle = None
+        if change == "subclass":
+            m = type("Scaled", (cls,), {"forward": scaled})(*args)
+        else:
+            m = cls(*args)
+            if change == "forward":
+                m.forward = lambda x, **kwargs: scaled(m, x, **kwargs)
+            elif change == "hook":
+                m.register_forward_hook(lambda mod, args, out: out * factor)
+            else:
+                handle = nn.modules.module.register_module_forward_hook(lambda mod, args, out: out * factor if mod is m else None)
+        return m, handle
+
+    torch.manual_seed(0)
+    D, Hq, Hkv, T = 64, 4, 2, 5
+    packed = torch.randn(T, Hq + 2 * Hkv, D, device="cuda").to(torch.bfloat16)
+    rope, handle = altered(RotaryPositionEmbedding, 2, D, 64)
+    try:
+        cache = PagedKVCache(1, Hkv, D, num_blocks=8, max_seqs=2, max_seq_len=64, block_size=16)
+        PagedAttentionManager(cache).add_sequence(T)
+        batch = RaggedBatch([(0, list(range(T)), 0, [T - 1])], "cuda")
+        with torch.no_grad():
+            want = RotaryPositionEmbedding(D, 64)(packed.clone()[None], positions=batch.positions, n_rot_heads=Hq + Hkv)[0] * 2
+            q = cache.append_rotated(0, packed.clone(), rope, batch, Hq)
+        k, v = cache.gather(0, 0, T)
+        assert torch.equal(q, want[:, :Hq]) and torch.equal(k, want[:, Hq:Hq + Hkv]) and torch.equal(v, want[:, Hq + Hkv:])
+    finally:
+        handle and handle.remove()
+
+    mlp = SwiGLU(512, 1024).to("cuda", torch.bfloat16)
+    x = torch.randn(3, 512, device="cuda").to(torch.bfloat16)
+    up, handle = altered(Linear, 2, 512, 2048, False)
+    up = up.to("cuda", torch.bfloat16)
+    up.weight = mlp.gate_up_proj.weight
+    try:
+        with torch.no_grad():
+            want = mlp.down_proj(F.swiglu(F.linear(x, up.weight) * 2))
+            mlp.gate_up_proj = up
+            assert torch.equal(F.serving(mlp)(x), want)
+    finally:
+        handle and handle.remove()
+    # a bias keeps the projection as well
+    mlp = SwiGLU(512, 1024, bias=True).to("cuda", torch.bfloat16)
+    with torch.no_grad():
+        assert torch.equal(F.serving(mlp)(x), mlp(x))

@@ -356,3 +356,45 @@ def test_http_front_reports_a_failed_serving_loop(served):
     finally:
         app.shutdown()
     assert isinstance(app.loop_error, RuntimeError)
+
+
+def test_a_rotation_of_its_own_rotates_and_leaves_the_projection_as_it_was():
+    from ferrotorch_b200.nn.layers import RotaryPositionEmbedding
+    from ferrotorch_b200.nn.paged import PagedAttentionManager, RaggedBatch
+
+    class Doubled(RotaryPositionEmbedding):
+        def forward(self, x, *, positions=None, n_rot_heads=None, **kwargs):
+            return torch.cat([2 * x[..., :n_rot_heads, :], x[..., n_rot_heads:, :]], -2)
+
+    cache = PagedKVCache(1, 2, 16, num_blocks=4, max_seqs=1, max_seq_len=32, block_size=8, device="cpu", dtype=torch.float32)
+    PagedAttentionManager(cache).add_sequence(3)
+    packed = torch.randn(3, 8, 16)
+    seen = packed.clone()
+    with torch.no_grad():
+        q = cache.append_rotated(0, packed, Doubled(16, 32), RaggedBatch([(0, [1, 2, 3], 0, [2])], "cpu"), 4)
+    k, v = cache.gather(0, 0, 3)
+    assert torch.equal(q, 2 * seen[:, :4]) and torch.equal(k, 2 * seen[:, 4:6]) and torch.equal(v, seen[:, 6:]) and torch.equal(packed, seen)
+
+
+def test_what_counts_as_a_plain_call():
+    from torch import nn
+
+    from ferrotorch_b200.nn.layers import Linear, runs_plainly
+
+    class Other(Linear):
+        pass
+
+    assert runs_plainly(Linear(8, 8), Linear) and not runs_plainly(Other(8, 8), Linear) and not runs_plainly(nn.Linear(8, 8), Linear)
+    for change in ("forward", "hook", "pre_hook", "backward_hook", "compiled", "global"):
+        m, handle = Linear(8, 8), None
+        if change == "forward":
+            m.forward = lambda x: x
+        elif change == "compiled":
+            m._compiled_call_impl = m.forward
+        else:
+            handle = {"hook": m.register_forward_hook, "pre_hook": m.register_forward_pre_hook, "backward_hook": m.register_full_backward_hook,
+                      "global": nn.modules.module.register_module_forward_hook}[change](lambda *a: None)
+        assert not runs_plainly(m, Linear), change
+        if handle is not None:
+            handle.remove()
+            assert runs_plainly(m, Linear)
