@@ -125,6 +125,22 @@ __device__ __forceinline__ void act32(uint32_t (&r)[32], int flags) {
   for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(apply_act(__uint_as_float(r[j]), flags));
 }
 
+// 32 gated results, the kind decided once as above.  Lanes whose row does not exist compute nothing: their zeros would send every division
+// of a warp down its slow path (257 x 16384 x 2048 of MODE 5: 70 us, 35 without them and with the kind decided outside the loops).
+__device__ __forceinline__ void glu32(uint32_t (&g)[32], const uint32_t (&up)[32], int kind, bool there) {
+  if (!there) return;
+  if (kind == 1) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) g[j] = __float_as_uint(glu(__uint_as_float(g[j]), __uint_as_float(up[j]), 1));
+  } else if (kind == 2) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) g[j] = __float_as_uint(glu(__uint_as_float(g[j]), __uint_as_float(up[j]), 2));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) g[j] = __float_as_uint(glu(__uint_as_float(g[j]), __uint_as_float(up[j]), 3));
+  }
+}
+
 // Epilogue that writes straight to global memory, one accumulator row per lane.  Used where the
 // output needs a read-modify-write in fp32 before rounding (bf16 accumulate) or an activation
 // after the accumulation.  `t_row` addresses this warp's 32 TMEM lanes at the tile's first
@@ -501,7 +517,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 // 34.9 ms with padded copies, 31.7 now.
 // MODE 5 is a gated product without a pass of its own for the gate: B is [2 N, K], gate rows, then up rows; the two CTAs bring the gate and
 // the up rows of BN / 2 features, so that both accumulate side by side, and act(gate) * up leaves the epilogue (p.taps: the activation).
-// A prefill of four layers of 4096 / 14336: 12997 us with a pass over the rounded product behind it, 12608 now.
+// 1500 x 28672 x 4096: 262 us with a pass over the rounded product behind it, 243 here; where it does not pay: _gates_in_gemm in functional.py.
 template <int BN>
 struct PairCfg {
   static constexpr int BNH = BN / 2;
@@ -785,13 +801,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             uint32_t up[32];
             tmem_ld_32x32(t_row + BNH + c * step_cols, up);
             tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) r0[j] = __float_as_uint(glu(__uint_as_float(r0[j]), __uint_as_float(up[j]), p.taps));
+            glu32(r0, up, p.taps, m0 + lane < p.M);
             tmem_ld_32x32(t_row + c * step_cols + 32, r1);
             tmem_ld_32x32(t_row + BNH + c * step_cols + 32, up);
             tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) r1[j] = __float_as_uint(glu(__uint_as_float(r1[j]), __uint_as_float(up[j]), p.taps));
+            glu32(r1, up, p.taps, m0 + lane < p.M);
           } else if (!out_f32) {
             tmem_ld_32x32(t_row + c * step_cols + 32, r1);
           } else {

@@ -643,15 +643,26 @@ def swiglu(gu: torch.Tensor, activation: str = "silu", param: float | None = Non
     return _apply(_SwiGLUFn, gu, act)
 
 
+def _gates_in_gemm(rows: int, F2: int) -> bool:
+    """Whether a gated product of more than 128 rows is faster as one kernel (CTA pairs with 256 x 256 tiles of gate and up rows) than as a
+    plain product and the activation behind it (us, two kernels / one).  Where the tiles are fewer than the 74 CTA pairs, the plain
+    product has 128-wide ones: up to 37 they fit into one wave there (128 < rows <= 256, 2 x 4736 x 2048: 20 / 24), above they do not
+    (2 x 8192 x 2048: 31 / 26; 512 rows, 2 x 3584 x 3072: 41 / 29).  From one to two waves both have two, and the longer epilogue costs
+    what the pass did (400 rows, 2 x 5504 x 2048: 33 / 35; 2 x 8192 x 2048: 35 / 36).  Above, the pass goes for nothing as long as two
+    thirds of the tiles' rows exist (1024 rows, 2 x 14336 x 4096: 183 / 171; 640, 2 x 8192 x 3072: 65 / 63; 257, 2 x 11008 x 4096: 74 / 76)."""
+    blocks = (rows + 255) // 256
+    tiles = blocks * ((F2 + 255) // 256)
+    return 37 < tiles < 74 or tiles >= 148 and 3 * rows >= 2 * 256 * blocks
+
+
 def linear_swiglu(x: torch.Tensor, w: torch.Tensor, activation: str = "silu", param: float | None = None) -> torch.Tensor:
     """``act(x Wg^T) * (x Wu^T)`` for a fused ``[gate | up]`` weight ``w [2F, K]``; without gradients one kernel, which does not round the
-    projections in between: few rows on the clusters that share a contraction, more on CTA pairs where their 256 x 128 tiles fill half
-    of the GPU (with fewer the plain product has narrower tiles to choose from)."""
+    projections in between: up to 128 rows on the clusters that share a contraction, more on CTA pairs where that is faster."""
     K, F2 = x.shape[-1], w.shape[0]
     rows = x.numel() // K if K else 0
     if (_NATIVE and x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and not torch.is_grad_enabled() and activation in _ACT_ID
             and rows > 0 and F2 >= 1024 and K >= 512 and F2 % 16 == 0 and K % 8 == 0 and w.stride(1) == 1
-            and w.stride(0) % 8 == 0 and (rows <= 128 or ((rows + 255) // 256) * ((F2 + 255) // 256) >= 37)
+            and w.stride(0) % 8 == 0 and (rows <= 128 or _gates_in_gemm(rows, F2))
             and _GEMM_CTA_LIMIT == 0 and not _transformed()):
         x2 = x.reshape(rows, K)
         if x2.stride(1) == 1 and (rows == 1 or x2.stride(0) >= K) and x2.stride(0) % 8 == 0 and (x2.data_ptr() | w.data_ptr()) % 16 == 0:

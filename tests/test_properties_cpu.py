@@ -138,3 +138,16 @@ def test_roi_align_of_a_constant_map_is_that_constant_inside_the_map(c, h, w, k,
     for fn in (D.roi_align, D.roi_align_torch):
         out = fn(feat, rois, 3, 1.0, 2, True)
         assert torch.allclose(out, val.view(1, c, 1, 1).expand_as(out), atol=1e-5)
+
+
+def test_gated_products_take_the_faster_kernel_of_what_was_measured():
+    from ferrotorch_b200.ops import functional as F
+
+    # rows, features, contraction, us as two kernels, us as one (weights from HBM, launches back to back)
+    for rows, features, _k, two, one in [
+            (129, 512, 2048, 15.3, 22.0), (214, 4096, 2048, 20.1, 23.5), (256, 4736, 2048, 21.3, 23.7), (129, 5504, 2048, 30.1, 23.9),
+            (214, 8192, 2048, 31.3, 26.1), (257, 3584, 3072, 39.2, 28.8), (512, 4096, 2048, 31.5, 24.5), (257, 4736, 2048, 22.2, 24.4),
+            (257, 5504, 2048, 31.8, 34.5), (320, 8192, 3072, 45.5, 46.7), (257, 11008, 4096, 73.9, 76.2), (1024, 4096, 2048, 34.9, 34.6),
+            (640, 8192, 3072, 64.9, 62.8), (1024, 14336, 4096, 183.1, 171.2), (1500, 5504, 2048, 61.6, 56.1)]:
+        if abs(two - one) > 0.02 * one:
+            assert F._gates_in_gemm(rows, 2 * features) == (one < two), (rows, features)
