@@ -84,12 +84,23 @@ _GEMM_CTA_LIMIT = 0
 
 
 def _streams(M: int, N: int, K: int) -> bool:
-    """Whether a product has too few 256-wide tiles for the pair kernel, so that clusters which share a contraction are faster (us, pair /
-    stream kernel; 214 rows: 4096 x 14336 98 / 39, 2048 x 8192 40 / 30, 3072 x 2048 23 / 15, 6144 x 4096 25 / 29, 2048 x 1408 10 / 13;
-    524 rows: 4096 x 14336 141 / 86, 6144 x 4096 45 / 34, 2048 x 2048 18 / 20, 16384 x 2048 39 / 63; 1024 rows: equal or slower)."""
-    if N < 1024 or K < 512:
+    """Whether clusters that share a contraction (``gemm_stream.cu``) are faster than the undivided sums of the CTA pairs, for 128 < M rows.
+    A CTA pair's time grows with the contraction alone until its 128- or 256-wide tiles need a second wave, the clusters' with rows as well
+    (us, pairs / clusters, weights from HBM, 129 to 768 rows of 25 weights measured):
+
+    * up to 256 rows the pairs have one wave below 8192 columns.  A contraction of 2048 pays up to 192 rows (4096 x 2048, 192 rows 15.4 / 14.5,
+      224: 15.4 / 16.5), from 3072 on always (3072 x 3072, 256 rows 20.0 / 18.4), above 4096 columns up to 160 rows (6144 x 4096, 160 rows
+      26.3 / 24.9, 192: 26.1 / 26.6, 256: 26.3 / 33.1);
+    * up to 512 rows the pairs have one wave for 4096 columns (400 rows 25.7 / 30.4 for a contraction of 4096; 14336: 77.4 / 56.0) and two above
+      (6144 x 4096, 400 rows 45.1 / 36.7); the clusters have one round up to 2048 (2048 x 4096, 400 rows 24.6 / 19.0);
+    * up to 640 rows the pairs have two waves above 3072 columns (4096 x 4096, 640 rows 44.6 / 36.5), below they win unless the contraction
+      is long (2048 x 4096 24.7 / 29.1, 2048 x 8192 43.8 / 37.9) or the columns are few (1024 x 4096 24.4 / 18.3);
+    * contractions below 2048 are slower at all sizes (2048 x 1024, 192 rows 8.5 / 11.4)."""
+    if not 1024 <= N <= 6144 or M > 640:
         return False
-    return M <= 128 or M <= 256 and N <= 4096 and K >= 2048 or M <= 640 and N <= 6144 and K >= 4096
+    if M <= 256:
+        return K >= (3072 if M > 192 else 2048) if N <= 4096 else K >= 4096 and M <= 160
+    return K >= 8192 or K >= 4096 and (N > 4096 or (N > 3072 or N <= 1024 if M > 512 else N <= 2048))
 
 
 def set_gemm_cta_limit(n: int) -> int:
@@ -244,7 +255,7 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = Non
         # decode-sized batch against a large weight: the weight-stationary kernel
         return gemm_small_m(a, b, bias=bias, out=out, activation=activation)
     flags = _ACT_FLAGS[activation]
-    if (split and 128 < M and _streams(M, N, K) and not accumulate and out.dtype == torch.bfloat16 and la[0] == 0
+    if (split and M > 128 and _streams(M, N, K) and not accumulate and out.dtype == torch.bfloat16 and la[0] == 0
             and lb[0] == 0 and bn == 0 and max_ctas == 0 and _GEMM_CTA_LIMIT == 0):
         return _gemm_stream(a, b, out, bias, flags)
     if out.dtype == torch.float32:

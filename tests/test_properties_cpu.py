@@ -151,3 +151,17 @@ def test_gated_products_take_the_faster_kernel_of_what_was_measured():
             (640, 8192, 3072, 64.9, 62.8), (1024, 14336, 4096, 183.1, 171.2), (1500, 5504, 2048, 61.6, 56.1)]:
         if abs(two - one) > 0.02 * one:
             assert F._gates_in_gemm(rows, 2 * features) == (one < two), (rows, features)
+
+
+def test_divided_sums_are_taken_where_they_were_measured_to_be_faster():
+    from ferrotorch_b200.ops import functional as F
+
+    # rows, columns, contraction, us of the CTA pairs, us of the clusters
+    for m, n, k, pairs, clusters in [
+            (129, 4096, 2048, 15.4, 13.5), (224, 4096, 2048, 15.4, 16.5), (256, 3072, 3072, 20.0, 18.4), (129, 6144, 4096, 26.1, 24.0),
+            (192, 6144, 4096, 26.1, 26.6), (224, 6144, 4096, 26.6, 30.6), (256, 6144, 6144, 36.5, 39.4), (256, 2048, 2048, 15.1, 15.5),
+            (288, 4096, 4096, 25.7, 26.3), (512, 4096, 4096, 26.2, 35.0), (400, 4096, 14336, 77.4, 56.0), (400, 6144, 4096, 45.1, 36.7),
+            (400, 2048, 4096, 24.6, 19.0), (524, 4096, 4096, 44.5, 31.8), (640, 2048, 4096, 24.7, 29.1), (640, 2048, 8192, 43.8, 37.9),
+            (640, 1024, 4096, 24.4, 18.3), (640, 6144, 4096, 46.4, 39.8), (192, 2048, 1024, 8.5, 11.4), (400, 3072, 2048, 15.6, 23.0),
+            (640, 16384, 2048, 39.8, 76.2), (768, 3072, 2048, 16.1, 20.4)]:
+        assert F._streams(m, n, k) == (clusters < pairs), (m, n, k)
