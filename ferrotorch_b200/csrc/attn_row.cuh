@@ -116,7 +116,7 @@ struct PooledKeys {
   __device__ __forceinline__ long long row(int b, const int* bt, int block_size, int max_blocks, int num_blocks) const {
     const int page = min((b * pool + pool - 1) / block_size, max_blocks - 1);
     const int at = min(max(b - page * block_size / pool, 0), per_page - 1);
-    return static_cast<long long>(min(max(__ldg(bt + page), 0), num_blocks - 1)) * per_page + at;
+    return static_cast<long long>(min(max(bt[page], 0), num_blocks - 1)) * per_page + at;
   }
 };
 static inline PooledKeys pooled_keys(const void* k, const void* v, int pool, int block_size) {

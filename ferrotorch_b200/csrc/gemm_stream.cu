@@ -247,7 +247,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           if (j < left)
-            bias[j] = (p.flags & GEMM_BIAS_F32) ? __ldg(static_cast<const float*>(p.bias) + n + j)
+            bias[j] = (p.flags & GEMM_BIAS_F32) ? static_cast<const float*>(p.bias)[n + j]
                                                 : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n + j]);
       }
       ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), acc_phase, abort_word, FT_ERR_TIMEOUT_EPILOGUE));

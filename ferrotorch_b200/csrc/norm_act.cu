@@ -55,7 +55,7 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // One block per row, grid-stride over rows. H % 8 == 0.
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* delta,
-                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                   const __nv_bfloat16* w, __nv_bfloat16* __restrict__ y,
                    __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int rows, int H,
                    float eps) {
   grid_dependency_launch();
@@ -254,8 +254,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 // half of a head and the 16 bytes that pair with them in the second half; interleaved layout:
 // 32 contiguous bytes.  cos/sin come as two float4 each.  Needs D % 16 == 0 and 16-byte
 // aligned rows (checked by the launcher).
-__global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cos_t,
-                                const float* __restrict__ sin_t, const int* pos, int T,
+__global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* cos_t,
+                                const float* sin_t, const int* pos, int T,
                                 int n_rot_heads, int D, long long ld, int seq_len, int pos_offset,
                                 int interleaved, float sign) {
   grid_dependency_launch();
@@ -310,7 +310,7 @@ __global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __re
 // Rotation (pair (d, d + D/2)) of the q and k heads of packed rows x [T, ld] (Hq query, Hkv key, Hkv value heads of D), the keys and values
 // going to their cache pages: q in place, k rotated into the cache (the row's k stays as it is), v copied.  One launch and one read of
 // k and v instead of a rotation in place and an append behind it; a thread owns eight pairs, or eight elements of v.
-__global__ void rope_append_kernel(__nv_bfloat16* x, const float* __restrict__ cos_t, const float* __restrict__ sin_t, const int* pos,
+__global__ void rope_append_kernel(__nv_bfloat16* x, const float* cos_t, const float* sin_t, const int* pos,
                                    const int* slots, const int* block_table, uint4* k_cache, uint4* v_cache, int T, int Hq, int Hkv, int D,
                                    long long ld, int block_size, int max_blocks, int num_blocks) {
   grid_dependency_launch();

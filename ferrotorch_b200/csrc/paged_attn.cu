@@ -278,7 +278,7 @@ paged_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
 }
 
 __global__ void paged_decode_combine_kernel(const float* part_o, const float* part_ml, __nv_bfloat16* __restrict__ out, int Hq, int D, long long ldo, int n_splits,
-                                            const float* __restrict__ sink, HeadGate gate, float out_scale) {
+                                            const float* sink, HeadGate gate, float out_scale) {
   grid_dependency_launch();
   grid_dependency_wait();
   const int hq = blockIdx.x, b = blockIdx.y;
@@ -354,12 +354,12 @@ struct PtCfg {  // HD: width of the K tile (64 or 128)
 template <int HD, int G, int SLOTS>
 __global__ void __launch_bounds__(PT_THREADS, SLOTS == 3 ? 2 : 1)
 paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, int box,
-                       const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
+                       const __nv_bfloat16* k_cache, const __nv_bfloat16* v_cache,
                        const __nv_bfloat16* q, const int* block_table,
                        const int* row_slot, const int* ctx_len, __nv_bfloat16* __restrict__ out,
                        float* __restrict__ part_o, float* __restrict__ part_ml, int Hq, int Hkv, int D, int Dv, int g_real,
                        long long ldq, long long ldo, int block_size, int max_blocks, int num_blocks, float scale_log2,
-                       int n_splits, KeyRange range, PooledKeys pooled, const float* __restrict__ slopes, const float* __restrict__ sink,
+                       int n_splits, KeyRange range, PooledKeys pooled, const float* slopes, const float* sink,
                        HeadGate gate, float out_scale, int* status) {
   using Cfg = PtCfg<HD, SLOTS>;
   extern __shared__ uint8_t smem_raw[];

@@ -246,7 +246,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       auto load_scales = [&](int cb, uint32_t (&s)[Q4_CK]) {
 #pragma unroll
         for (int j = 0; j < Q4_CK; ++j)
-          s[j] = cb < cb1 && cb * Q4_CK + j < k_blocks ? __ldg(reinterpret_cast<const uint32_t*>(srow + (cb * Q4_CK + j) * 4)) : 0u;
+          s[j] = cb < cb1 && cb * Q4_CK + j < k_blocks ? *reinterpret_cast<const uint32_t*>(srow + (cb * Q4_CK + j) * 4) : 0u;
       };
       uint32_t next[Q4_CK];
       load_scales(cb0, next);

@@ -510,3 +510,30 @@ def test_linear_swiglu_in_one_kernel(M, F_, K, act, monkeypatch):
     xg = x.clone().requires_grad_()
     F.linear_swiglu(xg, w, act).sum().backward()
     assert xg.grad is not None and _native.device_status(0) == 0
+
+
+def test_operands_made_by_the_kernel_just_before_are_seen():
+    # a norm weight and an fp32 bias that come straight out of the kernel which an overlapped launch follows, in buffers that
+    # hold other values from the step before
+    torch.manual_seed(0)
+    H = 2048
+    w, h = _rand(H, H) * 0.05, _rand(64, H)
+    nw, bias = torch.empty(1, H, device=DEV, dtype=torch.bfloat16), torch.empty(64, H, device=DEV)
+    xs = [_rand(1, H) for _ in range(40)]
+
+    def step(x, wait):
+        F.gemm_small_m(x, w, out=nw)
+        wait()
+        y = F.rmsnorm(h, nw[0], 1e-5)
+        F._small_m_f32(h, w, bias, False, None)
+        wait()
+        z = F.gemm_small_m(h, w, bias=bias[7])
+        wait()
+        return y, z
+
+    with torch.no_grad():
+        want = [step(x, torch.cuda.synchronize) for x in xs]
+        got = [step(x, lambda: None) for x in xs]
+    for a, b in zip(got, want):
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    assert _native.device_status(0) == 0
