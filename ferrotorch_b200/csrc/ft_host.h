@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #define FT_API extern "C" __attribute__((visibility("default")))
 
 namespace ft {
@@ -86,5 +88,30 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t
       return ft::FT_E_BAD_ARG;                   \
     }                                            \
   } while (0)
+
+// Clusters of 1, 2, 4 and 8 CTAs of a kernel that a device holds at a time (148, 74, 33 and 15 where a CTA fills an SM).  `known` is the
+// caller's, one per device; threads may ask at the same time, the entries are asked for before the first of them is published.
+template <typename... P>
+int resident_clusters(std::atomic<int> (&known)[64][4], void (*kernel)(P...), int threads, int smem, int device, int (&n)[4]) {
+  FT_REQUIRE(device >= 0 && device < 64, "device %d is out of range", device);
+  bool all = true;
+  for (int lg = 0; lg < 4; ++lg) all &= (n[lg] = known[device][lg].load(std::memory_order_acquire)) > 0;
+  if (all) return FT_E_OK;
+  FT_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = threads; cfg.dynamicSmemBytes = smem; cfg.attrs = &attr; cfg.numAttrs = 1;
+  for (int lg = 0; lg < 4; ++lg) {
+    attr.val.clusterDim.x = 1 << lg;
+    cfg.gridDim = sm_count(device) >> lg << lg;
+    FT_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n[lg], kernel, &cfg));
+    if (n[lg] < 1) n[lg] = 1;
+  }
+  for (int lg = 0; lg < 4; ++lg) known[device][lg].store(n[lg], std::memory_order_release);
+  return FT_E_OK;
+}
+
 
 }  // namespace ft

@@ -313,7 +313,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 }
 
 static int launch_stream(const void* X, const void* W, StreamParams p, int K, long long ldx, long long ldw, int device, cudaStream_t stream) {
-  static int max_clusters[64][4] = {};    // clusters of 1, 2, 4, 8 CTAs that are resident at a time (148, 74, 33, 15)
+  static std::atomic<int> known_clusters[64][4];
+  int max_clusters[4];
+  if (int rc = resident_clusters(known_clusters, gemm_stream_kernel, ST_THREADS, ST_SMEM, device, max_clusters)) return rc;
   p.m_tiles = (p.M + ST_MAX_ROWS - 1) / ST_MAX_ROWS;
   p.bn = ((p.M + p.m_tiles - 1) / p.m_tiles + 15) / 16 * 16;
   p.m_tiles = (p.M + p.bn - 1) / p.bn;
@@ -325,21 +327,11 @@ static int launch_stream(const void* X, const void* W, StreamParams p, int K, lo
   p.status = device_status_word(device);
   cudaLaunchAttribute attr[2] = {};
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.blockDim = ST_THREADS; cfg.dynamicSmemBytes = ST_SMEM; cfg.stream = stream; cfg.attrs = attr; cfg.numAttrs = 1;
-  if (!max_clusters[device][0]) {
-    FT_CUDA_CHECK(cudaFuncSetAttribute(gemm_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM));
-    for (int lg = 3; lg >= 0; --lg) {
-      attr[0].val.clusterDim.x = 1 << lg;
-      cfg.gridDim = sm_count(device) >> lg << lg;
-      int n = 0;
-      FT_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, gemm_stream_kernel, &cfg));
-      max_clusters[device][lg] = n > 0 ? n : 1;
-    }
-  }
+  cfg.blockDim = ST_THREADS; cfg.dynamicSmemBytes = ST_SMEM; cfg.stream = stream; cfg.attrs = attr; cfg.numAttrs = 2;
   // CTAs per tile, as measured with clusters of 1 / 2 / 4 / 8 (us, one row): two where there are tiles enough for that (128256 x 4096:
   // 163 / 156 / 169 / 245; 28672 x 4096: 46 / 42 / 43 / 57; 16384 x 2048: 17 / 16 / 17 / 26), else four (6144 x 4096: 24 / 16 / 14 / 15;
   // 4096 x 14336: 67 / 38 / 24 / 28; 3072 x 3072: 17 / 11 / 9 / 9), and eight for a few tiles with a long contraction (2048 x 8192:
@@ -348,8 +340,7 @@ static int launch_stream(const void* X, const void* W, StreamParams p, int K, lo
   while ((1 << lg) > p.k_blocks) --lg;
   p.cluster = 1 << lg;
   attr[0].val.clusterDim.x = p.cluster;
-  cfg.gridDim = (p.tiles < max_clusters[device][lg] ? p.tiles : max_clusters[device][lg]) * p.cluster;
-  cfg.numAttrs = 2;
+  cfg.gridDim = (p.tiles < max_clusters[lg] ? p.tiles : max_clusters[lg]) * p.cluster;
   CUtensorMap tmW, tmX;
   int rc = make_tmap_2d(&tmW, W, 2, K, p.glu ? 2ull * p.N : p.N, ldw * 2, ST_BK, p.n_tile, 3);
   if (rc) return rc;

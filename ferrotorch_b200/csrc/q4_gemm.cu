@@ -367,7 +367,9 @@ FT_API int ft_q4_0_gemm(const void* x, const void* nibbles, const void* scales, 
              "ft_q4_0_gemm: K must be a multiple of 64, N of 8");
   FT_REQUIRE((reinterpret_cast<uintptr_t>(nibbles) & 15) == 0 && (reinterpret_cast<uintptr_t>(scales) & 3) == 0,
              "ft_q4_0_gemm: nibble plane must be 16-byte aligned");
-  static int max_clusters[64][4] = {};    // clusters of 1, 2, 4, 8 CTAs that are resident at a time
+  static std::atomic<int> known_clusters[64][4];
+  int max_clusters[4];
+  if (int rc = resident_clusters(known_clusters, q4_gemm_kernel, Q4_THREADS, Q4_SMEM, device, max_clusters)) return rc;
   Q4Params p{};
   p.C = y; p.bias = static_cast<const __nv_bfloat16*>(bias); p.scales = static_cast<const uint8_t*>(scales);
   p.M = M; p.N = N; p.K = K; p.out_f32 = out_f32; p.ldc = ldy;
@@ -385,34 +387,23 @@ FT_API int ft_q4_0_gemm(const void* x, const void* nibbles, const void* scales, 
   p.status = device_status_word(device);
   cudaLaunchAttribute attr[2] = {};
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.blockDim = Q4_THREADS; cfg.dynamicSmemBytes = Q4_SMEM; cfg.stream = stream; cfg.attrs = attr; cfg.numAttrs = 1;
-  if (!max_clusters[device][0]) {
-    FT_CUDA_CHECK(cudaFuncSetAttribute(q4_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Q4_SMEM));
-    for (int lg = 3; lg >= 0; --lg) {
-      attr[0].val.clusterDim.x = 1 << lg;
-      cfg.gridDim = sm_count(device) >> lg << lg;
-      int n = 0;
-      FT_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, q4_gemm_kernel, &cfg));
-      max_clusters[device][lg] = n > 0 ? n : 1;
-    }
-  }
+  cfg.blockDim = Q4_THREADS; cfg.dynamicSmemBytes = Q4_SMEM; cfg.stream = stream; cfg.attrs = attr; cfg.numAttrs = 2;
   // Bound by expansion, so the SMs have to be equally busy: the cluster size with the fewest compressed blocks in a row (rounds of
   // tiles times a CTA's part of a contraction; a part below two blocks gains nothing).  Ties go to the smaller cluster.
   int lg = 0;
   long long best = 0;
   for (int i = 0; i <= 3 && (1 << i) <= p.c_blocks; ++i) {
-    const int rounds = (p.tiles + max_clusters[device][i] - 1) / max_clusters[device][i], part = (p.c_blocks + (1 << i) - 1) >> i;
+    const int rounds = (p.tiles + max_clusters[i] - 1) / max_clusters[i], part = (p.c_blocks + (1 << i) - 1) >> i;
     const long long cost = static_cast<long long>(rounds) * (part > 2 ? part : 2);
     if (i == 0 || cost < best) { best = cost; lg = i; }
   }
   p.cluster = 1 << lg;
   attr[0].val.clusterDim.x = p.cluster;
-  cfg.gridDim = (p.tiles < max_clusters[device][lg] ? p.tiles : max_clusters[device][lg]) * p.cluster;
-  cfg.numAttrs = 2;
+  cfg.gridDim = (p.tiles < max_clusters[lg] ? p.tiles : max_clusters[lg]) * p.cluster;
   CUtensorMap tmW, tmX;
   int rc = make_tmap_2d(&tmW, nibbles, 1, K / 2, N, K / 2, 128, Q4_BM, 3);
   if (rc) return rc;

@@ -537,3 +537,34 @@ def test_operands_made_by_the_kernel_just_before_are_seen():
     for a, b in zip(got, want):
         assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
     assert _native.device_status(0) == 0
+
+
+_FIRST_CALLS = """
+import threading, torch
+from ferrotorch_b200.ops import functional as F
+from ferrotorch_b200.ops.quant import Q4Linear, quantize_q4_0_planes
+torch.manual_seed(0)
+w = torch.randn(2048, 1024, device="cuda")
+layer, wb, x = Q4Linear(*quantize_q4_0_planes(w)), w.to(torch.bfloat16), torch.randn(16, 1024, device="cuda").to(torch.bfloat16)
+start, out = threading.Barrier(8), [None] * 8
+torch.cuda.synchronize()
+def work(i):
+    start.wait()
+    out[i] = (F.gemm_small_m(x, wb), layer(x)) if i % 2 else (layer(x), F.gemm_small_m(x, wb))[::-1]
+ts = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+[t.start() for t in ts], [t.join() for t in ts]
+torch.cuda.synchronize()
+want = F.gemm_small_m(x, wb), layer(x)
+assert all(o is not None and torch.equal(o[0], want[0]) and torch.equal(o[1], want[1]) for o in out)
+"""
+
+
+def test_first_calls_from_several_threads():
+    # each asks how many clusters the device holds; none may see a table that another one has half filled
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", _FIRST_CALLS], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
