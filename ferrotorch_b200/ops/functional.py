@@ -55,8 +55,8 @@ def gemm_small_m(x: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None 
     if residual is not None and ksplit == 1:
         raise ValueError("gemm_small_m: a residual needs the split path (ksplit != 1)")
     rc = lib.ft_gemm_small_m(x.data_ptr(), w.data_ptr(), out.data_ptr(), bias_ptr,
-                             residual.data_ptr() if residual is not None else None, None, M, N, K, x.stride(0), w.stride(0),
-                             out.stride(0), residual.stride(0) if residual is not None else 0, flags, ksplit,
+                             residual.data_ptr() if residual is not None else None, None, M, N, K,
+                             x.stride(0) if M > 1 else max(x.stride(0), K), w.stride(0) if N > 1 else max(w.stride(0), K), out.stride(0), residual.stride(0) if residual is not None else 0, flags, ksplit,
                              _dev(x), _stream())
     _native.check(rc, "ft_gemm_small_m")
     stats["gemm_small_m"] += 1
@@ -673,10 +673,10 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor, activation: str = "silu", pa
     rows = x.numel() // K if K else 0
     if (_NATIVE and x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and not torch.is_grad_enabled() and activation in _ACT_ID
             and rows > 0 and F2 >= 1024 and K >= 512 and F2 % 16 == 0 and K % 8 == 0 and w.stride(1) == 1
-            and w.stride(0) % 8 == 0 and (rows <= 128 or _gates_in_gemm(rows, F2))
+            and w.stride(0) >= K and w.stride(0) % 8 == 0 and (rows <= 128 or _gates_in_gemm(rows, F2))
             and _GEMM_CTA_LIMIT == 0 and not _transformed()):
         x2 = x.reshape(rows, K)
-        if x2.stride(1) == 1 and (rows == 1 or x2.stride(0) >= K) and x2.stride(0) % 8 == 0 and (x2.data_ptr() | w.data_ptr()) % 16 == 0:
+        if x2.stride(1) == 1 and x2.stride(0) >= K and x2.stride(0) % 8 == 0 and (x2.data_ptr() | w.data_ptr()) % 16 == 0:
             out = torch.empty((*x.shape[:-1], F2 // 2), device=x.device, dtype=x.dtype)
             lib = _native.kernels()
             rc = (lib.ft_gemm_stream_glu if rows <= 128 else lib.ft_gemm_glu)(

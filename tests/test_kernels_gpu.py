@@ -512,6 +512,22 @@ def test_linear_swiglu_in_one_kernel(M, F_, K, act, monkeypatch):
     assert xg.grad is not None and _native.device_status(0) == 0
 
 
+@pytest.mark.parametrize("rows", [1, 5, 300])
+def test_gated_products_of_operands_in_any_order(rows):
+    # rows that lie on one another, further apart, closer than a row is long, or column by column
+    torch.manual_seed(rows)
+    K, F2 = 512, 2 * 5504
+    w, x = _rand(F2, K) * 0.05, _rand(rows, K)
+    spaced = torch.zeros(F2, K + 24, device=DEV, dtype=torch.bfloat16)[:, 8:K + 8].copy_(w)
+    weights = [w, spaced, w.t().contiguous().t(), w[:1].expand(F2, K), torch.as_strided(w, (F2, K), (8, 1))]
+    inputs = [x, x[:1].expand(rows, K), torch.as_strided(w, (rows, K), (0, 1)), torch.as_strided(w, (rows, K), (8, 1)), x.t().contiguous().t()]
+    with torch.no_grad():
+        for a, b in [(x, t) for t in weights] + [(t, w) for t in inputs]:
+            got, want = F.linear_swiglu(a, b), F.linear_swiglu(a.clone(memory_format=torch.contiguous_format), b.clone(memory_format=torch.contiguous_format))
+            assert got.shape == want.shape and float((got.double() - want.double()).norm()) <= 2.0 ** -7 * float(want.double().norm())
+    assert _native.device_status(0) == 0
+
+
 def test_operands_made_by_the_kernel_just_before_are_seen():
     # a norm weight and an fp32 bias that come straight out of the kernel which an overlapped launch follows, in buffers that
     # hold other values from the step before
