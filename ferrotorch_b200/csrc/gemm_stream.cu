@@ -387,27 +387,22 @@ FT_API int ft_gemm_stream_glu(const void* X, const void* W, void* C, int M, int 
   return launch_stream(X, W, p, K, ldx, ldw, device, stream);
 }
 
-// The same for a small batch M <= 128 (decode).  workspace and ksplit are not needed any more; a residual with ksplit 1 stays refused.
-FT_API int ft_gemm_small_m(const void* X, const void* W, void* C, const void* bias, const void* residual,
-                           float* workspace, int M, int N, int K, long long ldx, long long ldw, long long ldc,
-                           long long ldr, int flags, int ksplit, int device, cudaStream_t stream) {
+// The same for a small batch M <= 128 (decode).
+FT_API int ft_gemm_small_m(const void* X, const void* W, void* C, const void* bias, const void* residual, int M, int N, int K,
+                           long long ldx, long long ldw, long long ldc, long long ldr, int flags, int device, cudaStream_t stream) {
   using namespace ft;
-  (void)workspace;
   FT_REQUIRE(M > 0 && M <= 128 && N > 0 && K > 0, "ft_gemm_small_m: M=%d must be in 1..128 (N=%d K=%d)", M, N, K);
-  FT_REQUIRE(ksplit != 1 || !residual, "ft_gemm_small_m: the residual is added by the split path only");
   return ft_gemm_stream(X, W, C, bias, residual, M, N, K, ldx, ldw, ldc, ldr, flags, device, stream);
 }
 
 // C[M, N] (fp32) (+)= X[M, K] W[N, K]^T for a small batch M <= 128; with dyt_out also the next layer's dynamic tanh of the new values,
 // dyt_out[M, N] = (tanh(alpha C) w + b) * dyt_scale as bf16 (being element by element, that norm needs no pass of its own over the
-// residual stream).  workspace and ksplit as in ft_gemm_small_m.
+// residual stream).
 FT_API int ft_gemm_small_m_f32(const void* X, const void* W, float* C, int accumulate, const float* alpha, const float* dyt_w,
-                               const float* dyt_b, void* dyt_out, float dyt_scale, float* workspace, int M, int N, int K,
-                               long long ldx, long long ldw, long long ldc, long long ldd, int ksplit, int device,
-                               cudaStream_t stream) {
+                               const float* dyt_b, void* dyt_out, float dyt_scale, int M, int N, int K, long long ldx,
+                               long long ldw, long long ldc, long long ldd, int device, cudaStream_t stream) {
   if (int _rc = ft::ensure_device(device)) return _rc;
   using namespace ft;
-  (void)workspace; (void)ksplit;
   FT_REQUIRE(X && W && C, "ft_gemm_small_m_f32: null operand");
   FT_REQUIRE(M > 0 && M <= 128 && N > 0 && K > ST_BK, "ft_gemm_small_m_f32: M=%d must be in 1..128, K=%d above %d (N=%d)", M, K, ST_BK, N);
   FT_REQUIRE(ldx % 8 == 0 && ldw % 8 == 0, "ft_gemm_small_m_f32: strides must be multiples of 8");

@@ -190,7 +190,7 @@ class LlamaEngine:
         """Row-parallel linear + reduce-scatter + residual add: this rank's rows ``[rows, H]``."""
         if not isinstance(w, tuple):
             if self.W == 1 and a.shape[0] <= 128:
-                return F.gemm_small_m(a, w, residual=residual)    # residual added by its split-K finalize pass
+                return F.gemm_small_m(a, w, residual=residual)    # residual added where the parts of a sum meet
             return self.tp.gemm_rs(slot, a, w, residual=residual)
         y = q4_0_linear(a, w[0], w[1])
         if self.W == 1:

@@ -31,7 +31,7 @@ _native.register_protos({
     "ft_gemm_stream": (_native._i, [_native._vp] * 5 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 2 + [_native._vp]),
     "ft_gemm_stream_glu": (_native._i, [_native._vp] * 3 + [_native._i] * 3 + [_native._ll] * 3 + [_native._i] * 2 + [_native._vp]),
     "ft_gemm_glu": (_native._i, [_native._vp] * 3 + [_native._i] * 3 + [_native._ll] * 3 + [_native._i] * 2 + [_native._vp]),
-    "ft_gemm_small_m": (_native._i, [_native._vp] * 6 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 3 + [_native._vp]),
+    "ft_gemm_small_m": (_native._i, [_native._vp] * 5 + [_native._i] * 3 + [_native._ll] * 4 + [_native._i] * 2 + [_native._vp]),
 })
 
 
@@ -40,7 +40,7 @@ def gemm_small_m(x: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None 
                  activation: str | None = None, ksplit: int = 0) -> torch.Tensor:
     """``x @ w.T (+ bias) (+ residual)`` for a small batch ``x [M <= 128, K]`` against ``w [N, K]``
     (both bf16, row-major): the decode-time GEMM.  The weight is the 128-row operand of the MMA, the contraction of a tile is
-    shared by a cluster of CTAs (``ksplit`` is a hint that is not needed any more)."""
+    shared by a cluster of CTAs.  ``ksplit`` has no effect, except that 1 still refuses a residual, as it did when it chose between kernels."""
     M, K = x.shape
     N = w.shape[0]
     if out is None:
@@ -53,11 +53,11 @@ def gemm_small_m(x: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None 
         bias_ptr = bias.data_ptr()
     lib = _native.kernels()
     if residual is not None and ksplit == 1:
-        raise ValueError("gemm_small_m: a residual needs the split path (ksplit != 1)")
+        raise ValueError("gemm_small_m: no residual with ksplit=1")
+    ldx, ldw = (t.stride(0) if t.shape[0] > 1 else max(t.stride(0), K) for t in (x, w))
     rc = lib.ft_gemm_small_m(x.data_ptr(), w.data_ptr(), out.data_ptr(), bias_ptr,
-                             residual.data_ptr() if residual is not None else None, None, M, N, K,
-                             x.stride(0) if M > 1 else max(x.stride(0), K), w.stride(0) if N > 1 else max(w.stride(0), K), out.stride(0), residual.stride(0) if residual is not None else 0, flags, ksplit,
-                             _dev(x), _stream())
+                             residual.data_ptr() if residual is not None else None, M, N, K, ldx, ldw,
+                             out.stride(0), residual.stride(0) if residual is not None else 0, flags, _dev(x), _stream())
     _native.check(rc, "ft_gemm_small_m")
     stats["gemm_small_m"] += 1
     return out
@@ -422,8 +422,8 @@ _native.register_protos({
                    [_native._f, _native._i, _native._vp]),
     "ft_qkv_finish": (_native._i, [_native._vp, _native._ll] + [_native._vp] * 8 + [_native._ll] + [_native._i] * 11 + [_native._f] * 3 +
                       [_native._i] * 7 + [_native._vp]),
-    "ft_gemm_small_m_f32": (_native._i, [_native._vp] * 3 + [_native._i] + [_native._vp] * 4 + [_native._f, _native._vp] + [_native._i] * 3 +
-                            [_native._ll] * 4 + [_native._i] * 2 + [_native._vp]),
+    "ft_gemm_small_m_f32": (_native._i, [_native._vp] * 3 + [_native._i] + [_native._vp] * 4 + [_native._f] + [_native._i] * 3 +
+                            [_native._ll] * 4 + [_native._i] + [_native._vp]),
 })
 
 
@@ -523,8 +523,8 @@ def _small_m_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate
     h = torch.empty((M, N), device=a.device, dtype=torch.bfloat16) if norm is not None else None
     alpha, nw, nb, scale = norm if norm is not None else (None, None, None, 1.0)
     rc = lib.ft_gemm_small_m_f32(a.data_ptr(), w.data_ptr(), out.data_ptr(), int(accumulate),
-                                 *(t.data_ptr() if t is not None else None for t in (alpha, nw, nb, h)), float(scale), None,
-                                 M, N, K, a.stride(0), w.stride(0), out.stride(0), N, 0, _dev(a), _stream())
+                                 *(t.data_ptr() if t is not None else None for t in (alpha, nw, nb, h)), float(scale),
+                                 M, N, K, a.stride(0), w.stride(0), out.stride(0), N, _dev(a), _stream())
     _native.check(rc, "ft_gemm_small_m_f32")
     stats["gemm_small_m"] += 1
     return h

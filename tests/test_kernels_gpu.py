@@ -92,7 +92,7 @@ def test_gemm_pair_kernel_long_run(a_mn, b_mn):
 @pytest.mark.parametrize("M,N,K,ksplit", [(64, 4096, 4096, 0), (64, 4096, 14336, 0), (64, 28672, 4096, 0), (17, 6144, 4096, 0),
                                           (128, 4096, 4096, 0), (100, 1032, 520, 1), (64, 4096, 4096, 1), (1, 2048, 1024, 4)])
 def test_gemm_small_m(M, N, K, ksplit):
-    # decode-sized batches: weight as the 128-row operand, transposed epilogue or split-K + finalize
+    # decode-sized batches: weight as the 128-row operand, its contraction shared by a cluster (ksplit has no effect but to refuse a residual)
     torch.manual_seed(M + N + K)
     x, w = _rand(M, K), _rand(N, K) * 0.05
     bias = _rand(N)
@@ -108,7 +108,7 @@ def test_gemm_small_m(M, N, K, ksplit):
         res = _rand(M, N)
         _assert_close(F.gemm_small_m(x, w, residual=res, ksplit=ksplit), want + res.float(), rtol=1e-2,
                       atol=0.02 * math.sqrt(K) * 0.05 + 0.02, what="small-m residual")
-        # pieces are summed in a fixed order: a second call gives the same bits
+        # parts are added in a fixed order: a second call gives the same bits
         assert torch.equal(F.gemm_small_m(x, w, ksplit=ksplit), y)
     else:
         _assert_close(F.gemm_small_m(x, w, activation="silu", ksplit=1), torch.nn.functional.silu(want), rtol=1e-2,
