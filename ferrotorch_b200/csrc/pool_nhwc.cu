@@ -130,9 +130,14 @@ static int make_geom(PoolGeom& g, int N, int H, int W, int C, int KH, int KW, in
 
 using namespace ft;
 
-// y [N, Ho, Wo, C] bf16 and arg [N, Ho, Wo, C] u8 (winning tap) from x [N, H, W, C] bf16; C % 8 == 0.
+// Whether `total` vectors and a stride of the grid beyond them can be counted in 32 bits: the divisions were most of the kernels' work (a
+// ResNet-50 step of 256 images: 29.03 ms with 64 bits, 28.93 with 32).
+static bool narrow_index(long long total, int blocks) { return total + static_cast<long long>(blocks) * 256 < (1ll << 31); }
+
+// y [N, Ho, Wo, C] bf16 and arg [N, Ho, Wo, C] u8 (winning tap) from x [N, H, W, C] bf16; C % 8 == 0.  wide: indices in 64 bits whatever
+// the size (tests).
 FT_API int ft_maxpool2d_fwd_nhwc(const void* x, void* y, void* arg, int N, int H, int W, int C, int KH, int KW, int stride,
-                                 int pad_h, int pad_w, int device, cudaStream_t stream) {
+                                 int pad_h, int pad_w, int wide, int device, cudaStream_t stream) {
   if (int _rc = ft::ensure_device(device)) return _rc;
   FT_REQUIRE(x && y && arg && C % 8 == 0, "ft_maxpool2d_fwd_nhwc: null pointer or C not a multiple of 8");
   FT_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 && (reinterpret_cast<uintptr_t>(arg) & 7) == 0,
@@ -142,10 +147,8 @@ FT_API int ft_maxpool2d_fwd_nhwc(const void* x, void* y, void* arg, int N, int H
   const long long total = static_cast<long long>(N) * g.Ho * g.Wo * (C / 8);
   long long grid = (total + 255) / 256;
   const long long cap = static_cast<long long>(sm_count(device)) * 16;
-  // indices in 32 bits where the vectors and a stride beyond can be counted so: the divisions were most of the kernel's work (a ResNet-50 step of
-  // 256 images: 29.03 ms, 28.93 now)
   const int blocks = static_cast<int>(grid < cap ? grid : cap);
-  if (total + static_cast<long long>(blocks) * 256 < (1ll << 31))
+  if (!wide && narrow_index(total, blocks))
     maxpool_fwd_nhwc_kernel<unsigned><<<blocks, 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), static_cast<uint8_t*>(arg), g);
   else
@@ -156,9 +159,9 @@ FT_API int ft_maxpool2d_fwd_nhwc(const void* x, void* y, void* arg, int N, int H
   return FT_E_OK;
 }
 
-// gx [N, H, W, C] bf16 from gy and arg of the forward call.
+// gx [N, H, W, C] bf16 from gy and arg of the forward call; wide as there.
 FT_API int ft_maxpool2d_bwd_nhwc(const void* gy, const void* arg, void* gx, int N, int H, int W, int C, int KH, int KW,
-                                 int stride, int pad_h, int pad_w, int device, cudaStream_t stream) {
+                                 int stride, int pad_h, int pad_w, int wide, int device, cudaStream_t stream) {
   if (int _rc = ft::ensure_device(device)) return _rc;
   FT_REQUIRE(gy && arg && gx && C % 8 == 0, "ft_maxpool2d_bwd_nhwc: null pointer or C not a multiple of 8");
   FT_REQUIRE(((reinterpret_cast<uintptr_t>(gy) | reinterpret_cast<uintptr_t>(gx)) & 15) == 0 && (reinterpret_cast<uintptr_t>(arg) & 7) == 0,
@@ -169,7 +172,7 @@ FT_API int ft_maxpool2d_bwd_nhwc(const void* gy, const void* arg, void* gx, int 
   long long grid = (total + 255) / 256;
   const long long cap = static_cast<long long>(sm_count(device)) * 16;
   const int blocks = static_cast<int>(grid < cap ? grid : cap);
-  if (total + static_cast<long long>(blocks) * 256 < (1ll << 31))
+  if (!wide && narrow_index(total, blocks))
     maxpool_bwd_nhwc_kernel<unsigned><<<blocks, 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(gy), static_cast<const uint8_t*>(arg), static_cast<__nv_bfloat16*>(gx), g);
   else

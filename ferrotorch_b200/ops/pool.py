@@ -21,8 +21,8 @@ from .conv import _pair
 
 _i, _vp = _native._i, _native._vp
 _native.register_protos({
-    "ft_maxpool2d_fwd_nhwc": (_i, [_vp] * 3 + [_i] * 10 + [_vp]),
-    "ft_maxpool2d_bwd_nhwc": (_i, [_vp] * 3 + [_i] * 10 + [_vp]),
+    "ft_maxpool2d_fwd_nhwc": (_i, [_vp] * 3 + [_i] * 11 + [_vp]),
+    "ft_maxpool2d_bwd_nhwc": (_i, [_vp] * 3 + [_i] * 11 + [_vp]),
     "ft_maxpool2d_host": (_i, [_vp] * 5 + [_i] * 9),
 })
 
@@ -56,7 +56,7 @@ class _MaxPoolNhwc(torch.autograd.Function):
         y = torch.empty((N, C, Ho, Wo), device=x.device, dtype=x.dtype, memory_format=CL)
         arg = torch.empty((N, Ho, Wo, C), device=x.device, dtype=torch.uint8)
         rc = _native.kernels().ft_maxpool2d_fwd_nhwc(x.data_ptr(), y.data_ptr(), arg.data_ptr(), N, H, W, C, k[0], k[1], s,
-                                                     p[0], p[1], F._dev(x), F._stream())
+                                                     p[0], p[1], 0, F._dev(x), F._stream())
         _native.check(rc, "ft_maxpool2d_fwd_nhwc")
         ctx.save_for_backward(arg)
         ctx.geom = (N, C, H, W, k, s, p)
@@ -69,7 +69,7 @@ class _MaxPoolNhwc(torch.autograd.Function):
         gy = gy.contiguous(memory_format=CL)
         gx = torch.empty((N, C, H, W), device=gy.device, dtype=gy.dtype, memory_format=CL)
         rc = _native.kernels().ft_maxpool2d_bwd_nhwc(gy.data_ptr(), arg.data_ptr(), gx.data_ptr(), N, H, W, C, k[0], k[1], s,
-                                                     p[0], p[1], F._dev(gy), F._stream())
+                                                     p[0], p[1], 0, F._dev(gy), F._stream())
         _native.check(rc, "ft_maxpool2d_bwd_nhwc")
         return gx, None, None, None
 

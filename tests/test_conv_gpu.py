@@ -172,7 +172,7 @@ def test_folded_resnet_matches_eval_model():
     (64, 64, 3, 1, (1, 1), 1, 1, (1, 1)), (64, 128, 3, 2, (1, 1), 1, 1, (5, 7)), (128, 64, 1, 2, (0, 0), 1, 2, (9, 8)),
     (64, 64, 3, 2, (1, 1), 1, 3, (97, 97)), (192, 320, 3, 1, (1, 1), 1, 2, (16, 8)), (64, 256, 2, 2, (0, 0), 1, 2, (8, 10)),
     (64, 64, (5, 3), 1, (2, 0), 1, 2, (11, 6)), (64, 64, 3, 1, (4, 4), 4, 1, (20, 20)), (64, 64, 3, 2, (0, 0), 1, 2, (8, 8)),
-    (64, 64, 3, 1, (130, 130), 130, 1, (5, 4)),                       # outside a tensor map's range: the padded copy
+    (64, 64, 3, 1, (130, 130), 130, 1, (5, 4)), (64, 64, 3, 2, (130, 2), 1, 1, (7, 6)),     # outside a tensor map's range: the padded copy
 ])
 @pytest.mark.parametrize("channels_last_filter", [False, True])
 def test_walks_against_torch(cin, cout, k, stride, pad, dil, n, hw, channels_last_filter):

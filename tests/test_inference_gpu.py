@@ -269,3 +269,34 @@ def test_rotations_and_projections_that_are_not_plain_are_called(change):
     mlp = SwiGLU(512, 1024, bias=True).to("cuda", torch.bfloat16)
     with torch.no_grad():
         assert torch.equal(F.serving(mlp)(x), mlp(x))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bs,D", [(16, 128), (20, 128), (64, 64), (16, 96)])
+@pytest.mark.parametrize("Hkv,G", [(8, 1), (4, 2), (4, 4), (4, 8)])
+def test_paged_decode_of_more_ctas_than_sms(bs, D, Hkv, G):
+    # a loaded server: one CTA for each sequence and key head, two to an SM (a ring of three tiles that wraps many times) up to groups of
+    # four heads; boxes, and pages of 20 tokens that are copied; what the pages hold behind the context is not finite
+    torch.manual_seed(bs + D + G)
+    lens = [1, 128, 129, 700, 1900, 256, 383, 1031] * 5
+    B = len(lens)
+    assert B * Hkv > torch.cuda.get_device_properties(0).multi_processor_count
+    cache = PagedKVCache(1, Hkv, D, num_blocks=sum((n + bs - 1) // bs for n in lens) + 2, max_seqs=B, max_seq_len=1920, block_size=bs)
+    cache.k[0].fill_(float("nan")), cache.v[0].fill_(float("nan"))
+    mgr = PagedAttentionManager(cache)
+    for b, n in enumerate(lens):
+        assert mgr.add_sequence(n) == b
+    T = sum(lens)
+    k, v = (torch.randn(T, Hkv, D, device="cuda").to(torch.bfloat16) for _ in range(2))
+    pos = torch.cat([torch.arange(n, dtype=torch.int32) for n in lens]).cuda()
+    cache.append(0, k, v, pos, torch.repeat_interleave(torch.arange(B, dtype=torch.int32), torch.tensor(lens)).cuda())
+    q = torch.randn(B, Hkv * G, D, device="cuda").to(torch.bfloat16)
+    out = cache.decode(0, q, torch.tensor(lens, device="cuda", dtype=torch.int32), n_splits=1)
+    at = 0
+    for b, n in enumerate(lens):
+        kb, vb = (t[at:at + n].float().repeat_interleave(G, 1) for t in (k, v))
+        at += n
+        want = torch.einsum("ht,thd->hd", torch.softmax(torch.einsum("hd,thd->ht", q[b].float(), kb) * D ** -0.5, -1), vb)
+        # P and the result are rounded to bf16
+        assert bool(((out[b].float() - want).abs() <= 2.0 ** -7 * (1 + want.abs())).all()), "sequence of %d" % n
+    assert _native.device_status(0) == 0
