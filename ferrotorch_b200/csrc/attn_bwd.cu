@@ -110,14 +110,25 @@ attn_delta_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* 
 #pragma unroll
   for (int k = 0; k < ROWS; ++k) {
     const uint32_t a[4] = {ov[k].x, ov[k].y, ov[k].z, ov[k].w}, c[4] = {dv[k].x, dv[k].y, dv[k].z, dv[k].w};
-    float s = 0.f;
+    float t[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float2 x = unpack_bf16x2(a[j]), y = unpack_bf16x2(c[j]);
-      s += x.x * y.x + x.y * y.y;
+      t[j] = 0.f;
+      t[j] += x.x * y.x + x.y * y.y;
     }
+    // Added in the order of attn_delta_kernel, so that gradients keep their bits: pairs 32 apart, then 16, 8, 4, 2 and 1 (pairs of two
+    // elements, four neighbours to a lane).  The first two steps hand half of a lane's sums to its partner.
+    const bool upper = l & (LANES / 2), odd = l & (LANES / 4);
+    float k0 = upper ? t[2] : t[0], k1 = upper ? t[3] : t[1];
+    k0 += __shfl_xor_sync(0xffffffffu, upper ? t[0] : t[2], LANES / 2);
+    k1 += __shfl_xor_sync(0xffffffffu, upper ? t[1] : t[3], LANES / 2);
+    float s = odd ? k1 : k0;
+    s += __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, LANES / 4);
 #pragma unroll
-    for (int m = LANES / 2; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    for (int m = LANES / 8; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    s += __shfl_xor_sync(0xffffffffu, s, LANES / 2);
+    s += __shfl_xor_sync(0xffffffffu, s, LANES / 4);
     const int i = i0 + k * GROUPS;
     if (l == 0 && i < Sq) {
       const long long idx = (static_cast<long long>(b) * Hq + h) * Sq + i;
