@@ -90,9 +90,8 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
   }
 }
 
-// The same with 16-byte loads: D / 8 lanes a row, four rows of a head in flight per lane, so that it runs at memory bandwidth (1 x 8192
-// tokens, 32 heads of 128, attention and its backward: 2908 us with four bytes a lane and one row a warp, 2862 now; of it 134 MB, 20 us, are
-// read here).
+// The same with 16-byte loads: D / 8 lanes a row, four rows of a head in flight per lane (8192 tokens, 32 heads of 128: 74 us with four bytes
+// a lane and one row a warp, 33 now; 134 MB are read, 20 us of HBM).
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout, const float* __restrict__ lse,
@@ -945,7 +944,8 @@ FT_API int ft_flash_attn_bwd(const void* q, const void* k, const void* v, const 
     const int threads = 256;
     const long long blocks = (rows * 32 + threads - 1) / threads;
     const __nv_bfloat16 *ob = static_cast<const __nv_bfloat16*>(o), *db = static_cast<const __nv_bfloat16*>(dout);
-    const bool vectors = ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 15) == 0 && Hq < 65536 && B < 65536;
+    // few rows are over before four of them per lane have paid (us, narrow / wide loads: 4896 rows of 128 2.7 / 2.8, 8192: 3.7 / 3.0)
+    const bool vectors = rows >= 6144 && ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 15) == 0 && Hq < 65536 && B < 65536;
     const long long lddo_ = static_cast<long long>(Hq) * D;
     if (vectors && D == 128)
       attn_delta_vec_kernel<128><<<dim3((Sq + 63) / 64, Hq, B), 256, 0, stream>>>(ob, db, lse, delta_scratch, delta_scratch + rows, Sq, Hq, ldo, lddo_);

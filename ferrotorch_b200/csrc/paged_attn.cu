@@ -332,7 +332,8 @@ constexpr int PT_VD = 128;     // rows of O^T
 
 // SLOTS tiles in the ring: six, or three so that two CTAs share an SM and the start of a CTA, its end, and the chain scores - maximum - P -
 // O of a tile run under the other one's loads.  With no more CTAs than SMs the long ring is better (148 CTAs of 8000 keys: 125 us against
-// 153; 512 of 1800: 129 against 105), and groups above four heads need its registers.
+// 153), above at once the short one (us, six / three tiles: 152 CTAs of 1800 keys 68 / 40, 296: 70 / 51, 304: 102 / 81, 512: 137 / 90; of 300
+// keys 20 / 12, 23 / 14, 31 / 23, 43 / 26); groups above four heads need the long one's registers.
 template <int HD, int SLOTS_>
 struct PtCfg {  // HD: width of the K tile (64 or 128)
   static constexpr int K_BYTES = PT_TILE * HD * 2;

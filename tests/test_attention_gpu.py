@@ -135,7 +135,7 @@ def test_flash_bwd_packed_qkv_grad_layout():
 @pytest.mark.parametrize("D,offset", [(128, 0), (128, 4), (64, 0), (64, 4)])
 @pytest.mark.parametrize("Sq", [1, 63, 130])
 def test_flash_bwd_with_an_output_at_any_place(D, offset, Sq):
-    # the row sums of O * dO read 16 bytes at a time where both allow it; an output eight bytes into its buffer takes the narrow loads
+    # an output eight bytes into its buffer cannot be read 16 bytes at a time by the row sums of O * dO
     from ferrotorch_b200.ops.attention import attention_block_backward
 
     torch.manual_seed(D + Sq)
@@ -157,12 +157,13 @@ def test_flash_bwd_with_an_output_at_any_place(D, offset, Sq):
 
 
 @pytest.mark.parametrize("D", [64, 128])
-def test_row_sums_keep_their_bits_whatever_the_loads(D):
-    # wide loads add in the order of the narrow ones: the two-pass kernels give the same gradients for an output at an odd place
+@pytest.mark.parametrize("B,Sq,H", [(2, 1031, 3), (1, 6145, 1), (3, 257, 8)])
+def test_row_sums_keep_their_bits_whatever_the_loads(D, B, Sq, H):
+    # wide loads (from 6144 rows on) add in the order of the narrow ones: the two-pass kernels give the same gradients for an output at an
+    # odd place, which takes the narrow loads
     from ferrotorch_b200.ops.attention import attention_block_backward, deterministic
 
     torch.manual_seed(D)
-    B, Sq, H = 2, 333, 3
     q, k, v, do = _rand(B, Sq, H, D), _rand(B, Sq, H, D), _rand(B, Sq, H, D), _rand(B, Sq, H, D)
     out, lse = F.flash_attn_fwd(q, k, v, True)
     moved = torch.empty(out.numel() + 4, device=DEV, dtype=out.dtype)[4:].view(out.shape).copy_(out)
