@@ -5,7 +5,7 @@ import pytest
 import torch
 
 hypothesis = pytest.importorskip("hypothesis")
-from hypothesis import given, settings  # noqa: E402
+from hypothesis import example, given, settings  # noqa: E402
 from hypothesis import strategies as st  # noqa: E402
 
 FAST = settings(max_examples=40, deadline=None)
@@ -36,6 +36,7 @@ def test_nms_keeps_an_independent_dominating_set(n, thr, seed):
 
 
 @FAST
+@example(1, 7, 16454)               # the top code beside a scale that lost 3.7e-4 of itself to fp16
 @given(st.integers(1, 6), st.integers(1, 8), st.integers(0, 2 ** 31 - 1))
 def test_q4_0_round_trip_error_and_fixed_point(rows, blocks, seed):
     # |x - dq(q(x))| <= |d| / 2 except at the clamped top code (<= |d|); quantising the result again changes nothing
@@ -46,7 +47,8 @@ def test_q4_0_round_trip_error_and_fixed_point(rows, blocks, seed):
     nib, sc = quantize_q4_0_planes(x)
     y = dequant_q4_0_planes(nib, sc)
     d = sc.float().abs().repeat_interleave(32, dim=1)
-    assert ((x - y).abs() <= d * 1.001 + 1e-6).all()
+    # |x| <= 8 |d| before d is rounded to fp16 (by 2^-11 of it at most): at the top code |x| - 7 |d| <= |d| (1 + 8 * 2^-11)
+    assert ((x - y).abs() <= d * (1 + 2.0 ** -8) + 1e-6).all()
     inner = (x - y).abs() <= d * 0.5 * 1.01 + 1e-3 * d + 1e-6          # fp16 scale rounding leaves a little slack
     assert inner.float().mean() > 0.9
     nib2, sc2 = quantize_q4_0_planes(y)
